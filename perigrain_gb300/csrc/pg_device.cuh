@@ -16,6 +16,8 @@
 //     doubles as the cell-start table. Cell coordinates are clamped to the grid, so a node that
 //     moves outside the box still lands in an edge cell and every pair within R_c is still found.
 #pragma once
+#include <vector_types.h>
+
 #include <cstdint>
 
 #include "../../include/perigrain.h"
@@ -185,6 +187,13 @@ struct Dev {
   double* bxin;
   uint32_t* alive;
   uint32_t* break_step;
+  // FP64 path: the edge list, one entry per bond: its end nodes, their slots of the slab (second slot
+  // NONE when the other node's row does not hold the bond) and its reference length; in the order of
+  // the first slot. addend: each slot's force addend of this step (two components, 3D the third in
+  // addend_z), zero for padding.
+  uint32_t n_edges;
+  uint2 *edge_ij, *edge_slot;
+  double *edge_xin, *addend, *addend_z;
   // grains / instances
   GrainDev* grain;
   unsigned long long* bbox;  // [G][2*dim] ordered keys: min..., max... (the step parity's buffer)

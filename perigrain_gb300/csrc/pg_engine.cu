@@ -13,6 +13,7 @@
 #include <string>
 #include <vector>
 
+#include "pg_bonds.h"
 #include "pg_device.cuh"
 #include "pg_handle.h"
 #include "pg_order.h"
@@ -184,6 +185,87 @@ static int mixed_setup(pg_handle* h, const pg_setup_desc* s) {
     k_mixed_images<<<(N + 255) / 256, 256>>>(P);
     CU(cudaGetLastError());
   }
+  return PG_OK;
+}
+
+// Edge list of the FP64 path (Dev::edge_ij). Slot s = (i -> j, the m-th entry of row i naming j) is
+// paired with the m-th entry of row j naming i when there is one (the two compute the same bond); a
+// pair is listed once, at the lower node's slot, an unpaired slot by itself.
+// k_edge_pairs: each slot's partner (NONE: unpaired) to pair[s], EDGE_SKIP where the slot is not listed
+// (padding, or the partner's entry covers it),
+// and the chunk's number of entries to count[c]. One warp per 32-node chunk, lane = node.
+constexpr uint32_t EDGE_SKIP = NONE - 1u;
+__global__ void k_edge_pairs(const Dev P, uint32_t* pair, uint32_t* count) {
+  const uint32_t c = blockIdx.x, lane = threadIdx.x, i = c * 32 + lane;
+  const uint32_t deg = i < P.N ? P.node_deg[i] : 0u;
+  const uint32_t row = P.chunk_slot[c] + lane, cd = P.chunk_deg[c];
+  uint32_t n = 0;
+  for (uint32_t k = 0; k < cd; ++k) {
+    const uint32_t s = row + 32u * k;
+    uint32_t other = EDGE_SKIP;
+    if (k < deg) {
+      const uint32_t j = P.bcol[s];
+      uint32_t m = 0;
+      for (uint32_t q = 0; q < k; ++q) m += P.bcol[row + 32u * q] == j ? 1u : 0u;
+      const uint32_t rj = P.chunk_slot[j >> 5] + (j & 31), dj = P.node_deg[j];
+      other = NONE;
+      for (uint32_t q = 0; q < dj && j != i; ++q)
+        if (P.bcol[rj + 32u * q] == i && m-- == 0) {
+          other = i < j ? rj + 32u * q : EDGE_SKIP;
+          break;
+        }
+    }
+    pair[s] = other;
+    n += other != EDGE_SKIP ? 1u : 0u;
+  }
+  n = __reduce_add_sync(0xffffffffu, n);
+  if (lane == 0) count[c] = n;
+}
+// The chunk's entries, in slot order from first[c].
+__global__ void k_edge_fill(const Dev P, const uint32_t* pair, const uint32_t* first, uint2* ij, uint2* slot,
+                            double* xin) {
+  const uint32_t c = blockIdx.x, lane = threadIdx.x, i = c * 32 + lane;
+  const uint32_t row = P.chunk_slot[c] + lane, cd = P.chunk_deg[c];
+  uint32_t at = first[c];
+  for (uint32_t k = 0; k < cd; ++k) {
+    const uint32_t s = row + 32u * k, other = pair[s];
+    const uint32_t b = __ballot_sync(0xffffffffu, other != EDGE_SKIP);
+    if (other != EDGE_SKIP) {
+      const uint32_t o = at + __popc(b & ((1u << lane) - 1u));
+      ij[o] = make_uint2(i, P.bcol[s]);
+      slot[o] = make_uint2(s, other);
+      xin[o] = P.bxin[s];
+    }
+    at += __popc(b);
+  }
+}
+
+static int edges_setup(pg_handle* h) {
+  Dev& P = h->P;
+  const uint32_t NC = P.n_chunks, slots = h->chunk_slot[NC];
+  P.n_edges = 0;
+  CU(h->dalloc(&P.addend, (size_t)slots * 2));
+  if (h->dim == 3) CU(h->dalloc(&P.addend_z, slots));
+  if (!slots) return PG_OK;
+  DevPool tmp;
+  uint32_t *pair = (uint32_t*)P.addend, *count = nullptr, *first = nullptr, *tile = nullptr, *done = nullptr;
+  CU(tmp.alloc(&count, NC));
+  CU(tmp.alloc(&first, NC + 1));
+  CU(tmp.alloc(&tile, bond_scan_tiles(NC)));
+  CU(tmp.alloc(&done, 1));
+  CU(cudaMemset(done, 0, 4));
+  k_edge_pairs<<<NC, 32>>>(P, pair, count);
+  CU(cudaGetLastError());
+  CU(scan_u32_dev(count, NC, first, tile, done, 0));
+  CU(cudaMemcpy(&P.n_edges, first + NC, 4, cudaMemcpyDeviceToHost));
+  CU(h->dalloc(&P.edge_ij, P.n_edges));
+  CU(h->dalloc(&P.edge_slot, P.n_edges));
+  CU(h->dalloc(&P.edge_xin, P.n_edges));
+  k_edge_fill<<<NC, 32>>>(P, pair, first, P.edge_ij, P.edge_slot, P.edge_xin);
+  CU(cudaGetLastError());
+  CU(cudaMemset(P.addend, 0, (size_t)slots * 16));
+  if (h->dim == 3) CU(cudaMemset(P.addend_z, 0, (size_t)slots * 8));
+  CU(cudaDeviceSynchronize());
   return PG_OK;
 }
 
@@ -714,6 +796,11 @@ static int create_impl(const pg_setup_desc* s, const pg_config* cfg_in, pg_handl
     CU(e);
   }
   tr.mark("bond layout");
+  if (h->precision == PG_FP64) {
+    rc = edges_setup(h.get());
+    if (rc) return rc;
+    tr.mark("edge list");
+  }
 
   // ---- grains ----
   std::vector<GrainDev> grains(G);

@@ -1,6 +1,6 @@
 // Correctly rounded FP64 arithmetic computed on the integer and FP32 pipes: division and square
-// root (used by the FP64 force kernel and the packing ascent), multiplication (the FP64 force
-// kernel's squared bond length), addition, subtraction, FP32 -> FP64 conversion and an ordered
+// root (used by the FP64 bond and force kernels and the packing ascent), multiplication (the bond
+// kernel's squared length), addition, subtraction, FP32 -> FP64 conversion and an ordered
 // compare against a non-negative threshold.
 //
 // GB300 executes FP64 arithmetic at about 1/64 of its FP32 rate, and an IEEE FP64 division or
@@ -11,16 +11,16 @@
 // infinite or NaN operands, a result outside the normal range) is passed to the FP64 hardware
 // operation, so the functions are drop-in replacements bit for bit.
 //
-// Division (schoolbook long division with a reciprocal estimate, Knuth TAOCP vol. 2 section 4.3.1,
-// in the form of division by a precomputed reciprocal of Granlund and Montgomery 1994). With
-// ma, mb the 53-bit significands and k in {53, 54} chosen so that Q = floor(ma 2^k / mb) lies in
-// [2^53, 2^54), Q is developed in three digits of 20, 20 and k - 40 bits. A 31-bit estimate
-// y ~ 2^83 / mb (an FP32 reciprocal of the divisor's top 24 bits, relative error below 2^-21)
-// gives each digit as floor(R y / 2^(83 - s)) from the running remainder R; the remainder update
-// R <- R 2^s - q mb is exact in 64-bit two's complement arithmetic because its true value stays
-// below 2 mb < 2^54 in magnitude. After the last digit the remainder lies in (-mb/64, 1.02 mb), so
-// one correction step makes 0 <= R < mb. Q's lowest bit is the guard bit of the 53-bit result and
-// R != 0 is the sticky bit, which settles round-to-nearest-even.
+// Division (by a precomputed reciprocal: Granlund and Montgomery, "Division by invariant integers
+// using multiplication", PLDI 1994). With ma, m the 53-bit significands and k in {53, 54} chosen so
+// that Q = floor(ma 2^k / m) lies in [2^53, 2^54): the reciprocal y ~ 2^115 / m starts as the FP32
+// reciprocal of the divisor's top 24 bits (y0 ~ 2^82 / m) and takes two Newton steps from the exact
+// integer remainders 2^82 - m y0 (below 2^63 in magnitude) and 2^99 - m y1 (below 2^60), which
+// leave a relative error below 2^-60; the high half of (ma 2^11) y is ma 2^62 / m to within nine
+// units, so its top 54 bits are within one of Q. The remainder ma 2^k - Q m, exact in 64-bit
+// two's complement arithmetic, settles that unit; Q's lowest bit is the guard bit of the 53-bit
+// result and a nonzero remainder is the sticky bit, which settles round-to-nearest-even. (Three
+// digits of 20, 20 and 13 bits from a 31-bit reciprocal took about 20 instructions more a quotient.)
 //
 // Square root (two-stage integer square root with Newton refinement and remainder correction,
 // Zimmermann, "Karatsuba square root", INRIA RR-3805, 1999, in a fixed two-level form). With
@@ -34,11 +34,11 @@
 // 0 <= M - S^2 <= 2S, and the remainder gives the sticky bit as for the quotient.
 //
 // Addition, subtraction and multiplication (add_rn, sub_rn, mul_rn) and the FP32 -> FP64
-// conversion (widen_f32) are provided the same way. Measured in the FP64 force kernel's bond loop
+// conversion (widen_f32) are provided the same way. Measured in the FP64 bond loop
 // (bond vector e = (dj - dp) + (xj - xp)) and in the mixed path's position update, the integer
 // sum was slower than the FP64 instruction it replaced (about 40 integer instructions with
 // branches against one FP64 add); the nearly branch-free product pays off for the squares of the
-// bond length, which is where the FP64 force kernel uses it.
+// bond length, which is where k_bonds uses it.
 //
 // Host and device share the code, so the routines are tested bit for bit against the host's
 // IEEE operations as well as against the GPU's.
@@ -81,14 +81,6 @@ PG_HD double from_bits(uint64_t b) {
   double x;
   std::memcpy(&x, &b, 8);
   return x;
-#endif
-}
-// High 32 bits of a 32 x 32 bit product.
-PG_HD uint32_t umulhi32(uint32_t a, uint32_t b) {
-#ifdef __CUDA_ARCH__
-  return __umulhi(a, b);
-#else
-  return (uint32_t)(((uint64_t)a * b) >> 32);
 #endif
 }
 // FP32 reciprocal and reciprocal square root estimates (relative error about 2^-23). The host
@@ -151,18 +143,15 @@ PG_HD double hw_sqrt(double x) {
 #endif
 }
 
-// floor(r * y / 2^(32 + sh)) for |r| < 2^62 and 0 < y < 2^31.
-PG_HD int64_t mul_shift(int64_t r, int32_t y, int sh) {
-  const int32_t rh = (int32_t)(r >> 32);
-  const uint32_t rl = (uint32_t)(uint64_t)r;
-  const int64_t p = (int64_t)rh * (int64_t)y + (int64_t)umulhi32(rl, (uint32_t)y);
-  return p >> sh;
-}
+// Division, square root and multiplication come twice: X_rn is the drop-in, which takes the hardware
+// operation outside the integer range; X_bits has no such branch and clears *ok there instead, so a
+// chain of them runs straight through and is redone once in hardware when any flag fell. (The +-1
+// corrections stay branches: as selects they took k_pack_maximin from 23.6 to 29.9 ms.)
 
 // A divisor prepared once for several quotients.
 struct Divisor {
   uint64_t m;  // significand with the hidden bit
-  int32_t y;   // ~ 2^83 / m, relative error below 2^-21
+  uint64_t y;  // ~ 2^115 / m, relative error below 2^-60
   int32_t e;   // biased exponent; 0 routes every quotient to the hardware
   uint64_t s;  // sign bit
   double b;    // the divisor itself, for the hardware route
@@ -176,12 +165,51 @@ PG_HD Divisor make_divisor(double b) {
   d.m = (bb & kFrac) | kHidden;
   const int32_t e = (int32_t)((bb >> 52) & 0x7ff);
   d.e = e == 0x7ff ? 0 : e;
-  // top 24 bits of the significand, exact in FP32: x in [2^23, 2^24), y ~ 2^54 / x
+  // top 24 bits of the significand, exact in FP32: x in [2^23, 2^24), y0 ~ 2^53 / x = 2^82 / m
   const float x = (float)(uint32_t)(d.m >> 29);
-  float r = rcp_est(x) * 18014398509481984.0f;  // 2^54
-  r = r < 2147483520.0f ? r : 2147483520.0f;    // largest FP32 below 2^31
-  d.y = (int32_t)r;
+  const int32_t y0 = (int32_t)(rcp_est(x) * 9007199254740992.0f);  // 2^53; at most 2^30 (1 + 2^-20)
+  // Newton: y1 = y0 (1 + e0 / 2^82), |e0| = |2^82 - m y0| < 2^63, kept to 47 bits
+  const int64_t e0 = (int64_t)(0 - d.m * (uint64_t)(uint32_t)y0);
+  const int64_t y1 = (int64_t)((uint64_t)(uint32_t)y0 << 33) + (((int64_t)y0 * (int64_t)(int32_t)(e0 >> 32)) >> 17);
+  const uint64_t y1s = (uint64_t)y1 >> 16;  // ~ 2^99 / m
+  // and once more: |e1| = |2^99 - m y1s| < 2^60
+  const int64_t e1 = (int64_t)(0 - d.m * y1s);
+  d.y = (y1s << 16) + (uint64_t)(((int64_t)(int32_t)(y1s >> 17) * (int64_t)(int32_t)(e1 >> 30)) >> 36);
   return d;
+}
+
+// Significand quotient of ma / d.m rounded to nearest even, hidden bit included (2^53 when the
+// rounding carries out); lt = 1 when ma < d.m.
+PG_HD uint64_t div_core(uint64_t ma, const Divisor& d, int32_t lt) {
+  // Q = floor(ma 2^k / m), k = 53 + lt, to within one unit
+  uint64_t Q = umulhi64(ma << 11, d.y) >> (9 - lt);
+  uint64_t r = (ma << (53 + lt)) - Q * d.m;
+  // 0 <= r < m
+  if ((int64_t)r < 0) {
+    Q -= 1;
+    r += d.m;
+  } else if (r >= d.m) {
+    Q += 1;
+    r -= d.m;
+  }
+  // Q in [2^53, 2^54): 53-bit significand, guard bit, and the remainder as the sticky bit
+  uint64_t M = Q >> 1;
+  M += (Q & 1ull) & ((r != 0 ? 1ull : 0ull) | (M & 1ull));
+  return M;
+}
+
+// The quotient a / d.b for normal a, d.b and result, and for a zero a over a normal d.b.
+PG_HD uint64_t div_bits(uint64_t ab, const Divisor& d, bool* ok) {
+  const int32_t ea = (int32_t)((uint32_t)(ab >> 52) & 0x7ffu);
+  const uint64_t ma = (ab & kFrac) | kHidden;
+  const uint64_t sign = (ab ^ d.s) & kSign;
+  const int32_t lt = ma < d.m ? 1 : 0;  // significand quotient below 1: develop one more bit
+  const int32_t be = ea - d.e + 1023 - lt;
+  const bool zero = (ab << 1) == 0;
+  *ok = d.e != 0 && (zero || ((uint32_t)(ea - 1) < 0x7feu && (uint32_t)(be - 1) < 2045u));
+  const uint64_t M = div_core(ma, d, lt);
+  // a carry out of the significand (M == 2^53) moves into the exponent field
+  return zero ? sign : (sign | (((uint64_t)(uint32_t)be << 52) + M - kHidden));
 }
 
 // IEEE round-to-nearest-even quotient a / d.b.
@@ -189,48 +217,20 @@ PG_HD double div_rn(double a, const Divisor& d) {
   const uint64_t ab = bits(a);
   const int32_t ea = (int32_t)((ab >> 52) & 0x7ff);
   const uint64_t ma = (ab & kFrac) | kHidden;
-  const int32_t lt = ma < d.m ? 1 : 0;  // significand quotient below 1: develop one more bit
+  const int32_t lt = ma < d.m ? 1 : 0;
   const int32_t be = ea - d.e + 1023 - lt;
   if (ea == 0 || ea == 0x7ff || d.e == 0 || be < 1 || be > 2045) {
     // a zero over a normal divisor is a zero with the product of the signs
     if ((ab << 1) == 0 && d.e != 0) return from_bits((ab ^ d.s) & kSign);
     return hw_div(a, d.b);
   }
-  const uint64_t mb = d.m;
-  const int32_t s3 = 13 + lt;  // k - 40
-  // digit 1: q ~ ma / mb 2^20
-  int64_t q = mul_shift((int64_t)ma, d.y, 31);
-  uint64_t r = (ma << 20) - (uint64_t)q * mb;
-  // digit 2
-  int64_t t = mul_shift((int64_t)r, d.y, 31);
-  r = (r << 20) - (uint64_t)t * mb;
-  q = (int64_t)(((uint64_t)q << 20) + (uint64_t)t);
-  // digit 3
-  t = mul_shift((int64_t)r, d.y, 51 - s3);
-  r = (r << s3) - (uint64_t)t * mb;
-  uint64_t Q = ((uint64_t)q << s3) + (uint64_t)t;
-  // 0 <= r < mb
-  if ((int64_t)r < 0) {
-    Q -= 1;
-    r += mb;
-  } else if (r >= mb) {
-    Q += 1;
-    r -= mb;
-  }
-  // Q in [2^53, 2^54): 53-bit significand, guard bit, and the remainder as the sticky bit
-  uint64_t M = Q >> 1;
-  M += (Q & 1ull) & ((r != 0 ? 1ull : 0ull) | (M & 1ull));
-  // a carry out of the significand (M == 2^53) moves into the exponent field
-  return from_bits(((ab ^ d.s) & kSign) | (((uint64_t)be << 52) + M - kHidden));
+  return from_bits(((ab ^ d.s) & kSign) | (((uint64_t)be << 52) + div_core(ma, d, lt) - kHidden));
 }
 
 PG_HD double div_rn(double a, double b) { return div_rn(a, make_divisor(b)); }
 
-// IEEE round-to-nearest-even square root.
-PG_HD double sqrt_rn(double x) {
-  const uint64_t xb = bits(x);
-  const int32_t ex = (int32_t)((xb >> 52) & 0x7ff);
-  if (ex == 0 || ex == 0x7ff || (xb & kSign)) return hw_sqrt(x);
+// Square root of the positive normal number with bits xb and biased exponent ex.
+PG_HD uint64_t sqrt_core(uint64_t xb, int32_t ex) {
   const uint64_t m = (xb & kFrac) | kHidden;
   // x = m 2^(ex - 1075); k = 54, or 55 when ex - 1075 is odd, makes the exponent of M = m 2^k even
   const int32_t odd = (ex & 1) ^ 1;
@@ -274,7 +274,22 @@ PG_HD double sqrt_rn(double x) {
   }
   uint64_t Mt = S >> 1;
   Mt += (S & 1ull) & ((R != 0 ? 1ull : 0ull) | (Mt & 1ull));
-  return from_bits(((uint64_t)be << 52) + Mt - kHidden);
+  return ((uint64_t)be << 52) + Mt - kHidden;
+}
+
+// The square root of a positive normal number.
+PG_HD uint64_t sqrt_bits(uint64_t xb, bool* ok) {
+  const int32_t ex = (int32_t)((uint32_t)(xb >> 52) & 0xfffu);  // the sign bit with the exponent
+  *ok = (uint32_t)(ex - 1) < 0x7feu;
+  return sqrt_core(xb, ex & 0x7ff);
+}
+
+// IEEE round-to-nearest-even square root.
+PG_HD double sqrt_rn(double x) {
+  const uint64_t xb = bits(x);
+  const int32_t ex = (int32_t)((xb >> 52) & 0x7ff);
+  if (ex == 0 || ex == 0x7ff || (xb & kSign)) return hw_sqrt(x);
+  return from_bits(sqrt_core(xb, ex));
 }
 
 // Core of the IEEE round-to-nearest-even sum of two doubles given by their bits (b's sign already
@@ -341,28 +356,30 @@ PG_HD double sub_rn(double a, double b) {
   return ok ? from_bits(r) : hw_sub(a, b);
 }
 
-// IEEE round-to-nearest-even a * b: the 106-bit product of the significands from a 64 x 64 bit
-// multiplication, its top 53 bits rounded with the next bit and the rest as the sticky bit. A
-// zero times a finite number is the signed zero; other zero, subnormal, infinite or NaN operands
-// and results outside the normal range take the hardware operation.
-PG_HD double mul_rn(double a, double b) {
-  const uint64_t ab = bits(a), bb = bits(b);
-  const int32_t ea = (int32_t)((ab >> 52) & 0x7ff), eb = (int32_t)((bb >> 52) & 0x7ff);
+// The product a * b of normal numbers with a normal result, and of a zero and a finite number: the
+// 106-bit product of the significands from a 64 x 64 bit multiplication, its top 53 bits rounded with
+// the next bit and the rest as the sticky bit.
+PG_HD uint64_t mul_bits(uint64_t ab, uint64_t bb, bool* ok) {
+  const int32_t ea = (int32_t)((uint32_t)(ab >> 52) & 0x7ffu), eb = (int32_t)((uint32_t)(bb >> 52) & 0x7ffu);
   const uint64_t sign = (ab ^ bb) & kSign;
-  const uint64_t ma = (ab & kFrac) | kHidden, mb = (bb & kFrac) | kHidden;
-  const uint64_t lo = ma * mb, hi = umulhi64(ma, mb);  // product in [2^104, 2^106)
-  const int32_t top = (int32_t)(hi >> 41);               // 1 when the product is >= 2^105
-  const int32_t e = ea + eb - 1023 + top;
-  if (ea == 0 || ea == 0x7ff || eb == 0 || eb == 0x7ff || e < 1 || e > 2045) {
-    if ((((ab << 1) == 0) && eb != 0x7ff) || (((bb << 1) == 0) && ea != 0x7ff)) return from_bits(sign);
-    return hw_mul(a, b);
-  }
-  const int32_t sh = 52 + top;
-  uint64_t q = (hi << (64 - sh)) | (lo >> sh);
-  const uint64_t g = (lo >> (sh - 1)) & 1ull;
-  const uint64_t st = (lo & ((1ull << (sh - 1)) - 1ull)) != 0 ? 1ull : 0ull;
-  q += g & (st | (q & 1ull));
-  return from_bits(sign | (((uint64_t)e << 52) + q - kHidden));
+  const uint64_t ma = ((ab & kFrac) | kHidden) << 10, mb = ((bb & kFrac) | kHidden) << 10;
+  const uint64_t lo = ma * mb;
+  uint64_t hi = umulhi64(ma, mb);                // product in [2^124, 2^126)
+  const uint32_t top = (uint32_t)(hi >> 61);      // 1 when the product is >= 2^125
+  hi = (hi << (1u - top)) | (lo != 0 ? 1ull : 0ull);  // all below the guard bit
+  const int32_t e = ea + eb - 1023 + (int32_t)top;
+  const uint64_t q = (hi + 0xffull + ((hi >> 9) & 1ull)) >> 9;  // round to nearest, ties to even
+  const bool zero = (ab << 1) == 0 || (bb << 1) == 0;
+  *ok = zero ? (ea != 0x7ff && eb != 0x7ff)
+             : ((uint32_t)(ea - 1) < 0x7feu && (uint32_t)(eb - 1) < 0x7feu && (uint32_t)(e - 1) < 2045u);
+  return zero ? sign : (sign | (((uint64_t)(uint32_t)e << 52) + q - kHidden));
+}
+
+// IEEE round-to-nearest-even a * b.
+PG_HD double mul_rn(double a, double b) {
+  bool ok;
+  const uint64_t r = mul_bits(bits(a), bits(b), &ok);
+  return ok ? from_bits(r) : hw_mul(a, b);
 }
 
 // Exact FP32 -> FP64 conversion from the bits; subnormal, infinite and NaN inputs take the

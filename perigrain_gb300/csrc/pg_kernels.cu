@@ -1,12 +1,12 @@
 // GB300 (sm_103a) kernels of the PeriDEM time step, FP64 parity path.
 //
-// One step (reference src/particle/timeloop.h:608-879) is six launches on one stream:
+// One step (reference src/particle/timeloop.h:608-879) is these launches on one stream:
 //   k_predict      position update (timeloop.h:661-669) + grid key + per-grain bounding box
 //   k_scan_reduce  \ exclusive scan of the per-bucket counts = cell-start table
 //   k_scan_final   /
 //   k_scatter      nodes -> bucket order (counting sort, one digit spanning all buckets)
-//   k_force        bond force + break (particle2.h:102-232), self/inter-grain contact
-//                  (contact.h:668-812), wall (contact.h:900-964, :314-431, :16-41),
+//   k_bonds        bond force addends + break (particle2.h:102-232), one bond per thread
+//   k_force        sum of the bond forces, self/inter-grain contact (contact.h:668-812), wall (contact.h:900-964, :314-431, :16-41),
 //                  external force and torque (timeloop.h:774-824), velocity update
 //                  (timeloop.h:834-863) -- fused, one node per thread
 //   k_finalize     ordered wall-reaction sums, pair log, wall move (timeloop.h:866-878)
@@ -126,6 +126,142 @@ __global__ void __launch_bounds__(256) k_predict(const Dev P) {
   }
 }
 
+// Addend of one bond of a node, the reference's operations in its order, for any operands: the
+// stretch in *str.
+template <int D>
+__device__ __noinline__ void bond_addend_any(const double* e, double xin, double cnot, double vol, double* g,
+                                             double* str) {
+  double n2 = e[0] * e[0];
+  for (int c = 1; c < D; ++c) n2 = n2 + e[c] * e[c];
+  const double en = sqrt(n2);
+  *str = (en - xin) / xin;
+  const double sc = (cnot * *str) * vol;
+  for (int c = 0; c < D; ++c) g[c] = sc * (e[c] / en);
+}
+
+// Addend of a bond stored for the force kernel, and read back.
+template <int D>
+__device__ __forceinline__ void st_addend(const Dev& P, uint32_t s, const double (&g)[D]) {
+  reinterpret_cast<double2*>(P.addend)[s] = make_double2(g[0], g[1]);
+  if constexpr (D == 3) P.addend_z[s] = g[2];
+}
+template <int D>
+__device__ __forceinline__ void ld_addend(const Dev& P, uint32_t s, double (&g)[D]) {
+  const double2 q = reinterpret_cast<const double2*>(P.addend)[s];
+  g[0] = q.x;
+  g[1] = q.y;
+  if constexpr (D == 3) g[2] = P.addend_z[s];
+}
+
+// Bond forces and bond breaking (particle2.h:102-150, :191-232), one thread per bond of the edge
+// list (Dev::edge_ij): the two directions of a bond differ in the sign of the bond vector and in
+// the neighbour's volume only, so its length, stretch and unit vector are formed once and the
+// addends of both nodes written to their slots of the bond slab, where the force kernel sums each
+// node's in bond order. Squares, square root and divisions run on the integer pipe, bit-identical
+// to the IEEE operations (pg_ieee64.cuh); a bond with an operand or a result outside their range is
+// redone in hardware.
+//
+// Bound by the FP64 pipe (one warp instruction per 16 cycles and SM) beside the integer ALU: 15
+// FP64 instructions per bond in 2D, 21 in 3D, against twice 14 and twice 20 when each node
+// computed its own bonds. Collision ensemble (10.0M directed bonds): k_bonds 158 us + k_force 61 us
+// against 364 us fused; 3D spheres (10.8M): 245 + 116 against 804 us; two disks (65k): 4.8 + 8.0
+// against 56 us, the work spread over 1,019 warps instead of 79. More of it on the integer pipe
+// (the extension en - xin, the scale and force products, the sum of the squares) was slower: the
+// ensemble step 250 us as it stands, 263 with the extension moved, 323 with all of them moved.
+template <int D>
+__global__ void __launch_bounds__(256) k_bonds(const Dev P) {
+  pdl_enter();
+  const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool in_list = b < P.n_edges;
+  const uint32_t be = in_list ? b : P.n_edges - 1u;
+  const uint2 ij = P.edge_ij[be], sl = P.edge_slot[be];
+  const double xin = P.edge_xin[be];
+  const GrainDev& gr = P.grain[P.node_grain[ij.x]];
+  const bool mov = gr.flags & GF_MOVABLE;
+  const bool two = sl.y != NONE;
+  const uint32_t wi = P.alive[sl.x >> 5], wj = two ? P.alive[sl.y >> 5] : 0u;
+  const bool ai = mov && ((wi >> (sl.x & 31)) & 1u), aj = mov && ((wj >> (sl.y & 31)) & 1u);
+  const bool use = in_list && (ai || aj);
+  double di[D], dj[D], xi[D], xj[D];
+  ldv<D>(P.disp, ij.x, di);
+  ldv<D>(P.disp, ij.y, dj);
+  ldv<D>(P.xpos, ij.x, xi);
+  ldv<D>(P.xpos, ij.y, xj);
+  const double vi = P.vol[ij.x], vj = P.vol[ij.y], cnot = gr.cnot;
+  double e[D];
+  uint64_t eb[D];
+  for (int c = 0; c < D; ++c) {
+    e[c] = (dj[c] - di[c]) + (xj[c] - xi[c]);
+    eb[c] = ieee64::bits(e[c]);
+  }
+  bool ok, all;
+  double n2d = ieee64::from_bits(ieee64::mul_bits(eb[0], eb[0], &all));
+  for (int c = 1; c < D; ++c) {
+    n2d = n2d + ieee64::from_bits(ieee64::mul_bits(eb[c], eb[c], &ok));
+    all &= ok;
+  }
+  const uint64_t n2 = ieee64::bits(n2d);
+  const uint64_t en = ieee64::sqrt_bits(n2, &ok);
+  all &= ok;
+  const uint64_t ext = ieee64::bits(ieee64::from_bits(en) - xin);
+  uint64_t str = ieee64::div_bits(ext, ieee64::make_divisor(xin), &ok);
+  all &= ok;
+  double gi[D], gj[D];
+  for (int c = 0; c < D; ++c) {
+    gi[c] = 0.0;
+    gj[c] = 0.0;
+  }
+  // an unstretched bond (str = +-0 and |e[c] / en| <= 1) adds +-0, which leaves a sum's bits
+  // unchanged (it starts at +0 and never becomes -0 under round-to-nearest)
+  if (__any_sync(0xffffffffu, use && (str << 1) != 0)) {
+    const double cs = cnot * ieee64::from_bits(str);
+    const double si = cs * vj, sj = cs * vi;
+    const ieee64::Divisor den = ieee64::make_divisor(ieee64::from_bits(en));
+    for (int c = 0; c < D; ++c) {
+      const uint64_t u = ieee64::div_bits(eb[c], den, &ok);
+      all &= ok;
+      const double ud = ieee64::from_bits(u);
+      gi[c] = si * ud;
+      gj[c] = sj * -ud;
+    }
+  }
+  if (!in_list) return;
+  if (use && !all) {
+    double ea[D], ga[D], sa;
+    for (int c = 0; c < D; ++c) ea[c] = -e[c];
+    bond_addend_any<D>(ea, xin, cnot, vi, ga, &sa);
+    for (int c = 0; c < D; ++c) {
+      gj[c] = ga[c];
+      ea[c] = e[c];
+    }
+    bond_addend_any<D>(ea, xin, cnot, vj, ga, &sa);
+    for (int c = 0; c < D; ++c) gi[c] = ga[c];
+    str = ieee64::bits(sa);
+  }
+  for (int c = 0; c < D; ++c) {
+    gi[c] = ai ? gi[c] : 0.0;
+    gj[c] = aj ? gj[c] : 0.0;
+  }
+  st_addend<D>(P, sl.x, gi);
+  if (two) st_addend<D>(P, sl.y, gj);
+  if (use && P.enable_fracture && (gr.flags & GF_BREAKABLE) && (gr.flags & GF_BREAK_BONDS)) {
+    // the break test str > snot on the integer pipe when snot is +0 or more and not NaN
+    const uint64_t snot_bits = ieee64::bits(gr.snot);
+    const double s = ieee64::from_bits(str);
+    if (ieee64::gt_nonneg_ok(snot_bits) ? ieee64::gt_nonneg(s, snot_bits) : s > gr.snot) {
+      const uint32_t t = *P.step;
+      if (ai) {
+        atomicAnd(&P.alive[sl.x >> 5], ~(1u << (sl.x & 31)));
+        P.break_step[sl.x] = t;
+      }
+      if (aj) {
+        atomicAnd(&P.alive[sl.y >> 5], ~(1u << (sl.y & 31)));
+        P.break_step[sl.y] = t;
+      }
+    }
+  }
+}
+
 template <int D, bool REC, bool GC>
 __global__ void __launch_bounds__(128) k_force(const Dev P) {
   pdl_enter();
@@ -138,63 +274,24 @@ __global__ void __launch_bounds__(128) k_force(const Dev P) {
   const uint32_t g = act ? P.node_grain[d] : 0;
   const GrainDev gr = P.grain[g];
   const bool mov = act && (gr.flags & GF_MOVABLE);
-  const bool brk = P.enable_fracture && (gr.flags & GF_BREAKABLE) && (gr.flags & GF_BREAK_BONDS);
+  const uint32_t slot0 = P.chunk_slot[chunk] + lane;
+  const uint32_t w0 = P.chunk_word[chunk];
 
   double f[D];
   for (int c = 0; c < D; ++c) f[c] = 0.0;
   double vp[D];
   if (act) ldv<D>(P.vel_in, d, vp);
 
-  // ---- bond force and bond breaking (particle2.h:102-150, :191-232) ----
-  const uint32_t cdeg = P.chunk_deg[chunk];
-  const uint32_t slot0 = P.chunk_slot[chunk] + lane;
-  const uint32_t w0 = P.chunk_word[chunk];
+  // ---- bond forces: the node's addends (k_bonds) in bond order ----
   {
-    // the break test str > snot on the integer pipe when snot is +0 or more and not NaN
-    const uint64_t snot_bits = ieee64::bits(gr.snot);
-    const bool snot_int = ieee64::gt_nonneg_ok(snot_bits);
-    double dp[D], xp[D];
-    if (mov) {
-      ldv<D>(P.disp, d, dp);
-      ldv<D>(P.xpos, d, xp);
-    }
+    const uint32_t cdeg = P.chunk_deg[chunk];
+#pragma unroll 4
     for (uint32_t k = 0; k < cdeg; ++k) {
-      const uint32_t word = P.alive[w0 + k];
-      bool bit = (word >> lane) & 1u;
-      if (mov && bit) {
-        const uint32_t s = slot0 + 32u * k;
-        const uint32_t j = P.bcol[s];
-        const double xin = P.bxin[s];
-        double dj[D], xj[D];
-        ldv<D>(P.disp, j, dj);
-        ldv<D>(P.xpos, j, xj);
-        double e[D];
-        for (int c = 0; c < D; ++c) e[c] = (dj[c] - dp[c]) + (xj[c] - xp[c]);
-        // the squares on the integer pipe too (the sums stay FP64 instructions: the integer sum
-        // measured slower, and so did moving the scale and force products as well)
-        double n2 = ieee64::mul_rn(e[0], e[0]);
-        for (int c = 1; c < D; ++c) n2 = n2 + ieee64::mul_rn(e[c], e[c]);
-        // sqrt and the divisions on the integer pipe, bit-identical to the IEEE operations
-        const double en = ieee64::sqrt_rn(n2);
-        const double str = ieee64::div_rn(en - xin, xin);
-        const double sc = (gr.cnot * str) * P.vol[j];
-        // an unstretched bond (sc = +-0 with 0 < en < inf, so |e[c] / en| <= 1) adds +-0, which
-        // leaves f's bits unchanged (f starts at +0 and never becomes -0 under round-to-nearest)
-        const uint64_t enb = ieee64::bits(en);
-        if ((ieee64::bits(sc) << 1) != 0 || enb - 1 >= 0x7fefffffffffffffull) {
-          const ieee64::Divisor den = ieee64::make_divisor(en);
-          for (int c = 0; c < D; ++c) f[c] = f[c] + sc * ieee64::div_rn(e[c], den);
-        }
-        if (brk && (snot_int ? ieee64::gt_nonneg(str, snot_bits) : str > gr.snot)) {
-          bit = false;
-          P.break_step[s] = t;
-        }
-      }
-      const uint32_t nw = __ballot_sync(0xffffffffu, bit);
-      if (lane == 0 && nw != word) P.alive[w0 + k] = nw;
+      double q[D];
+      ld_addend<D>(P, slot0 + 32u * k, q);
+      for (int c = 0; c < D; ++c) f[c] = f[c] + q[c];
     }
   }
-  __syncwarp();
 
   unsigned long long my_pairs = 0, my_hash = 0, my_close = 0;
   uint32_t rent[REC ? MAX_CAND : 1];  // recorded contact entries of this node (REC only)
@@ -561,6 +658,10 @@ static void launch_step_t(const Dev& P, const LaunchCfg& L, cudaStream_t s, uint
     *launches += 1;
   }
   if (e0) cudaEventRecord(e0, s);
+  if (P.n_edges) {
+    launch_k(k_bonds<D>, cdiv(P.n_edges, 256), 256, 0, s, pdl, P);
+    *launches += 1;
+  }
   const dim3 grid(cdiv(nthr_nodes, L.force_block)), block(L.force_block);
   if (P.grain_contact) {
     if (rec) launch_k(k_force<D, true, true>, grid, block, 0, s, pdl, P);
