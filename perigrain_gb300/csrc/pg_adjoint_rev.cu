@@ -26,6 +26,7 @@
 #include "pg_adjoint.h"
 #include "pg_common.cuh"
 #include "pg_device.cuh"
+#include "pg_hilo.cuh"
 
 namespace pg {
 
@@ -155,41 +156,6 @@ __device__ __forceinline__ bool force_bar(const Dev& P, const AdjStep& A, uint32
   return true;
 }
 
-// bond reference positions (hi/lo FP32, relative to the instance origin) from the mixed engine's
-// bond record, and the displacement hi/lo pairs of a recorded step (same layout as the record's
-// displacement part)
-template <int D>
-__device__ __forceinline__ void ld_xref(const float* __restrict__ bref, uint32_t N, uint32_t i, float (&xh)[D],
-                                        float (&xl)[D]) {
-  if constexpr (D == 2) {
-    const float4 b = __ldg(reinterpret_cast<const float4*>(bref) + 2ull * i + 1);
-    xh[0] = b.x;
-    xh[1] = b.y;
-    xl[0] = b.z;
-    xl[1] = b.w;
-  } else {
-    for (int c = 0; c < D; ++c) {
-      xh[c] = __ldg(bref + (size_t)(2 * D + c) * N + i);
-      xl[c] = __ldg(bref + (size_t)(3 * D + c) * N + i);
-    }
-  }
-}
-template <int D>
-__device__ __forceinline__ void ld_dhl(const float* __restrict__ df, uint32_t N, uint32_t i, float (&dh)[D],
-                                       float (&dl)[D]) {
-  if constexpr (D == 2) {
-    const float4 a = __ldg(reinterpret_cast<const float4*>(df) + i);
-    dh[0] = a.x;
-    dh[1] = a.y;
-    dl[0] = a.z;
-    dl[1] = a.w;
-  } else {
-    for (int c = 0; c < D; ++c) {
-      dh[c] = __ldg(df + (size_t)c * N + i);
-      dl[c] = __ldg(df + (size_t)(D + c) * N + i);
-    }
-  }
-}
 template <int D>
 __device__ __forceinline__ void ldfv(const float* a, uint32_t i, float (&v)[D]) {
   if constexpr (D == 2) {
@@ -215,7 +181,7 @@ __device__ __forceinline__ void stfv(float* a, uint32_t i, const float (&v)[D]) 
 // Bond part of the reverse step: f_p = sum_j cnot vol_j s(eta) e(eta), eta = X_j - X_p; H =
 // d(s e)/d(eta) is symmetric, so Xb_p = cnot sum_j H (vol_p Fb_j - vol_j Fb_p), and
 // dF_p/dcnot = f_p / cnot. Writes the node's bond share of Xb (xbb) and of the cnot cotangent
-// (pcb). F32: the mixed engine's form -- xi from the bond record's hi/lo reference positions,
+// (pcb). F32: the mixed engine's form -- xi from the hi/lo reference positions,
 // the displacement difference from the tape's hi/lo pairs, the cancellation-free stretch
 // s = (2 xi.et + et.et) / (|xi| (|xi + et| + |xi|)), force cotangents from the FP32 array fbf.
 template <int D, bool F32>
@@ -238,8 +204,8 @@ __global__ void __launch_bounds__(32 * SUB) k_adj_bonds(const Dev P, const AdjSt
     const uint32_t w0 = P.chunk_word[chunk];
     if constexpr (F32) {
       float dh[D], dl[D], xh[D], xl[D], Fb[D], xb[D], pc = 0.f;
-      ld_dhl<D>(A.df, P.N, d, dh, dl);
-      ld_xref<D>(P.bref, P.N, d, xh, xl);
+      ld_hl<D>(A.df, P.np, d, dh, dl);
+      ld_hl<D>(P.xref, P.np, d, xh, xl);
       ldfv<D>(A.fbf, d, Fb);
       for (int c = 0; c < D; ++c) xb[c] = 0.f;
       const float volp = P.vol_f[d];
@@ -248,8 +214,8 @@ __global__ void __launch_bounds__(32 * SUB) k_adj_bonds(const Dev P, const AdjSt
         if (!bond_used(A.end_alive, A.break_step, w0 + k, lane, s, t)) continue;
         const uint32_t j = P.bcol[s];
         float jdh[D], jdl[D], jxh[D], jxl[D], Fj[D];
-        ld_dhl<D>(A.df, P.N, j, jdh, jdl);
-        ld_xref<D>(P.bref, P.N, j, jxh, jxl);
+        ld_hl<D>(A.df, P.np, j, jdh, jdl);
+        ld_hl<D>(P.xref, P.np, j, jxh, jxl);
         ldfv<D>(A.fbf, j, Fj);
         const float volj = P.vol_f[j];
         float xi[D], et[D], y[D];

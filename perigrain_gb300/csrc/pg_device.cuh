@@ -240,13 +240,13 @@ struct Dev {
   uint32_t rec_cap;
   double *rec_x, *rec_v, *rec_w;
   uint32_t* rec_t;
-  float* rec_df;  // mixed precision: the step's displacement as FP32 hi/lo pairs (layout of bref's disp part)
-  // mixed precision (PG_MIXED): FP32 hi/lo pairs (x = hi + lo to ~2^-47 |x|). `bref` interleaves,
-  // per node, the pair of the FP64 displacement and the pair of the bond reference position
-  // (relative to the instance's fixed origin) -- 4*SF floats, one 32-byte sector in 2D -- so a bond
-  // gathers its neighbour's data from one sector. FP32 acceleration, force, external force and
-  // volume.
-  float* bref;
+  float* rec_df;  // mixed precision: the step's displacement as FP32 hi/lo pairs (layout of dref)
+  // mixed precision (PG_MIXED): FP32 hi/lo pairs (x = hi + lo to ~2^-47 |x|, layout in pg_hilo.cuh)
+  // of the FP64 displacement (dref) and of the bond reference position relative to the instance's
+  // fixed origin (xref), np = nodes padded to whole chunks; FP32 acceleration, force, external force
+  // and volume.
+  uint32_t np;
+  float *dref, *xref;
   float *acc_f, *force_f, *extf_f, *vol_f;
   float dt_f, hdt2_f, half_dt_f;
 };

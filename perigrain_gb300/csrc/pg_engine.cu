@@ -16,6 +16,7 @@
 #include "pg_bonds.h"
 #include "pg_device.cuh"
 #include "pg_handle.h"
+#include "pg_hilo.cuh"
 #include "pg_order.h"
 #include "pg_sqrt_threshold.h"
 #include "pg_kernels.h"
@@ -111,68 +112,60 @@ int build_graphs(pg_handle* h) {
   return PG_OK;
 }
 
-// hi/lo FP32 image of FP64 vectors (hi = (float)x, lo = (float)(x - hi)), layout of ld_hl():
-// 2D [hx, hy, lx, ly]; 3D [hx, hy, hz, 0, lx, ly, lz, 0]
-static void pack_hl(const double* x, uint32_t N, uint32_t D, const std::vector<double>* origin_of_node,
-                    std::vector<float>* out) {
-  const uint32_t SF = (D == 2) ? 2 : 4;
-  out->assign((size_t)N * 2 * SF, 0.f);
-  for (uint32_t i = 0; i < N; ++i)
-    for (uint32_t c = 0; c < D; ++c) {
-      double v = x[(size_t)i * D + c] - (origin_of_node ? (*origin_of_node)[(size_t)i * 3 + c] : 0.0);
-      float hi = (float)v;
-      float lo = (float)(v - (double)hi);
-      (*out)[(size_t)i * 2 * SF + c] = hi;
-      (*out)[(size_t)i * 2 * SF + SF + c] = lo;
-    }
-}
-
-static void pack_f(const double* x, uint32_t N, uint32_t D, std::vector<float>* out) {
-  const uint32_t SF = (D == 2) ? 2 : 4;
-  out->assign((size_t)N * SF, 0.f);
-  for (uint32_t i = 0; i < N; ++i)
-    for (uint32_t c = 0; c < D; ++c) (*out)[(size_t)i * SF + c] = (float)x[(size_t)i * D + c];
-}
-
-// FP32 images of the uploaded FP64 state for the mixed path (the host packing of pack_hl/pack_f,
-// same conversions): bref = [disp hi, disp lo, (pos - xorigin) hi, lo] per node (2D record, 3D
-// planes), acc, extforce and vol in FP32.
-__global__ void k_mixed_images(const Dev P) {
+// FP32 images of the uploaded FP64 state for the mixed path: hi/lo pairs (hi = (float)x, lo =
+// (float)(x - hi)) of the displacement and of pos - xorigin, and acc, extforce and vol in FP32;
+// `what` picks them.
+enum { IMG_DISP = 1, IMG_ACC = 2, IMG_CONST = 4 };
+template <int D>
+__global__ void k_mixed_images(const Dev P, int what) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= P.N) return;
-  const uint32_t D = P.dim, S = (D == 2) ? 2 : 4, SF = S, N = P.N;
-  const InstDev& in = P.inst[P.grain[P.node_grain[i]].inst];
-  for (uint32_t c = 0; c < D; ++c) {
-    const double dv = P.disp[(size_t)i * S + c];
-    const float dh = (float)dv, dl = (float)(dv - (double)dh);
-    const double xv = P.pos[(size_t)i * S + c] - in.xorigin[c];
-    const float xh = (float)xv, xl = (float)(xv - (double)xh);
-    const float q4[4] = {dh, dl, xh, xl};
-    for (uint32_t q = 0; q < 4; ++q) {
-      if (D == 2) {
-        P.bref[(size_t)i * 8 + q * 2 + c] = q4[q];
-      } else {
-        P.bref[(size_t)(q * D + c) * N + i] = q4[q];
-      }
+  constexpr uint32_t S = (D == 2) ? 2 : 4;
+  float h[D], l[D];
+  if (what & IMG_DISP) {
+    for (int c = 0; c < D; ++c) {
+      const double v = P.disp[(size_t)i * S + c];
+      h[c] = (float)v;
+      l[c] = (float)(v - (double)h[c]);
     }
-    P.acc_f[(size_t)i * SF + c] = (float)P.acc[(size_t)i * S + c];
-    P.extf_f[(size_t)i * SF + c] = (float)P.extf[(size_t)i * S + c];
+    st_hl<D>(P.dref, P.np, i, h, l);
   }
-  P.vol_f[i] = (float)P.vol[i];
+  if (what & IMG_ACC)
+    for (int c = 0; c < D; ++c) P.acc_f[(size_t)i * S + c] = (float)P.acc[(size_t)i * S + c];
+  if (what & IMG_CONST) {
+    const InstDev& in = P.inst[P.grain[P.node_grain[i]].inst];
+    for (int c = 0; c < D; ++c) {
+      const double v = P.pos[(size_t)i * S + c] - in.xorigin[c];
+      h[c] = (float)v;
+      l[c] = (float)(v - (double)h[c]);
+      P.extf_f[(size_t)i * S + c] = (float)P.extf[(size_t)i * S + c];
+    }
+    st_hl<D>(P.xref, P.np, i, h, l);
+    P.vol_f[i] = (float)P.vol[i];
+  }
+}
+static cudaError_t mixed_images(const Dev& P, int what, cudaStream_t st) {
+  if (!P.N) return cudaSuccess;
+  if (P.dim == 2) k_mixed_images<2><<<(P.N + 255) / 256, 256, 0, st>>>(P, what);
+  else k_mixed_images<3><<<(P.N + 255) / 256, 256, 0, st>>>(P, what);
+  return cudaGetLastError();
 }
 
 static int mixed_setup(pg_handle* h, const pg_setup_desc* s) {
   Dev& P = h->P;
   const uint32_t N = P.N, D = h->dim, SF = (D == 2) ? 2 : 4;
-  // bref and vol_f padded to whole warp chunks: the mixed force kernel's lanes past the last node
-  // gather their own (padding) index for bonds they never use
-  const size_t NP = (size_t)P.n_chunks * 32;
-  CU(h->dalloc(&P.bref, (NP - N) * 8 + (size_t)N * 4 * D));
+  // dref, xref and vol_f padded to whole warp chunks: the mixed force kernel's lanes past the last
+  // node gather their own (padding) index for bonds they never use
+  const size_t NP = (size_t)P.n_chunks * 32, HL = (D == 2) ? HL_FLOATS<2> : HL_FLOATS<3>;
+  P.np = (uint32_t)NP;
+  CU(h->dalloc(&P.dref, NP * HL));
+  CU(h->dalloc(&P.xref, NP * HL));
   CU(h->dalloc(&P.acc_f, (size_t)N * SF));
   CU(h->dalloc(&P.force_f, (size_t)N * SF));
   CU(h->dalloc(&P.extf_f, (size_t)N * SF));
   CU(h->dalloc(&P.vol_f, NP));
-  CU(cudaMemset(P.bref, 0, ((NP - N) * 8 + (size_t)N * 4 * D) * 4));
+  CU(cudaMemset(P.dref, 0, NP * HL * 4));
+  CU(cudaMemset(P.xref, 0, NP * HL * 4));
   CU(cudaMemset(P.vol_f, 0, NP * 4));
   P.dt_f = (float)P.dt;
   P.hdt2_f = (float)P.hdt2;
@@ -181,10 +174,7 @@ static int mixed_setup(pg_handle* h, const pg_setup_desc* s) {
   CU(cudaMemset(P.acc_f, 0, (size_t)N * SF * 4));
   CU(cudaMemset(P.extf_f, 0, (size_t)N * SF * 4));
   CU(cudaMemset(P.force_f, 0, (size_t)N * SF * 4));
-  if (N) {
-    k_mixed_images<<<(N + 255) / 256, 256>>>(P);
-    CU(cudaGetLastError());
-  }
+  CU(mixed_images(P, IMG_DISP | IMG_ACC | IMG_CONST, 0));
   return PG_OK;
 }
 
@@ -1196,28 +1186,8 @@ int pg_set_field(pg_handle* h, int field, const double* in) {
   rc = request_list_rebuild(h);
   if (rc) return rc;
   if (h->precision == PG_MIXED && (field == PG_FIELD_DISP || field == PG_FIELD_ACC)) {
-    std::vector<float> tf;
-    if (field == PG_FIELD_DISP) {
-      const uint32_t SF = (D == 2) ? 2 : 4;
-      pack_hl(in, N, D, nullptr, &tf);
-      std::vector<float> ref((size_t)N * 4 * D);
-      CU(cudaMemcpy(ref.data(), h->P.bref, ref.size() * 4, cudaMemcpyDeviceToHost));
-      for (uint32_t i = 0; i < N; ++i)
-        for (uint32_t c = 0; c < D; ++c) {
-          const float hv = tf[(size_t)i * 2 * SF + c], lv = tf[(size_t)i * 2 * SF + SF + c];
-          if (D == 2) {
-            ref[(size_t)i * 8 + c] = hv;
-            ref[(size_t)i * 8 + 2 + c] = lv;
-          } else {
-            ref[(size_t)c * N + i] = hv;
-            ref[(size_t)(D + c) * N + i] = lv;
-          }
-        }
-      CU(cudaMemcpy(h->P.bref, ref.data(), ref.size() * 4, cudaMemcpyHostToDevice));
-    } else {
-      pack_f(in, N, D, &tf);
-      CU(cudaMemcpy(h->P.acc_f, tf.data(), tf.size() * 4, cudaMemcpyHostToDevice));
-    }
+    CU(mixed_images(h->P, field == PG_FIELD_DISP ? IMG_DISP : IMG_ACC, h->stream));
+    CU(cudaStreamSynchronize(h->stream));
   }
   return PG_OK;
 }

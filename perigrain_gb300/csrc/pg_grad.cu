@@ -14,12 +14,18 @@
 
 #include "pg_adjoint.h"
 #include "pg_handle.h"
+#include "pg_hilo.cuh"
 #include "pg_kernels.h"
 #include "pg_kernels_mixed.h"
 
 using namespace pg;
 
 static int fail(int code, const std::string& msg) { return pg_fail(code, msg); }
+
+// floats of one step's displacement pairs on the tape
+static size_t df_floats(const pg_handle* h) {
+  return (size_t)h->P.np * (h->dim == 2 ? HL_FLOATS<2> : HL_FLOATS<3>);
+}
 
 static GradState* grad_state(pg_handle* h) {
   if (!h->grad) h->grad.reset(new GradState);
@@ -49,7 +55,7 @@ static int ensure_regions(pg_handle* h) {
   if (h->precision == PG_MIXED) {
     const size_t SF = (D == 2) ? 2 : 4;
     add(P.acc_f, N * SF * 4);
-    add(P.bref, N * 4 * D * 4);
+    add(P.dref, (size_t)P.np * (D == 2 ? HL_FLOATS<2> : HL_FLOATS<3>) * 4);
   }
   CU(cudaEventCreate(&G->e0));
   CU(cudaEventCreate(&G->e1));
@@ -187,7 +193,7 @@ static int ensure_tape(pg_handle* h, uint32_t C, bool masks, uint64_t ent_cap) {
     CU(G->tape.alloc(&G->V, (size_t)C * N * S));
     CU(G->tape.alloc(&G->W, (size_t)C * I * NS));
     CU(G->tape.alloc(&G->tstep, C));
-    if (h->precision == PG_MIXED) CU(G->tape.alloc(&G->DF, (size_t)C * N * (h->dim == 2 ? 4 : 6)));
+    if (h->precision == PG_MIXED) CU(G->tape.alloc(&G->DF, (size_t)C * df_floats(h)));
     G->tape_steps = C;
   }
   if (masks && !G->off) {
@@ -227,7 +233,7 @@ static int enqueue_recompute(pg_handle* h, int parity, uint32_t len, uint32_t fi
     } else if (h->overlap) {
       // the recording steps with each finalize beside the next position update, as in the
       // forward graphs (bit-identical to the serial order)
-      float* DF = G->DF ? G->DF + (size_t)i * N * (h->dim == 2 ? 4 : 6) : nullptr;
+      float* DF = G->DF ? G->DF + (size_t)i * df_floats(h) : nullptr;
       const Dev P = rec_dev(h, parity, G->off + (size_t)i * N, G->cnt + (size_t)i * N, G->wall + (size_t)i * N,
                             G->ent, G->ent_n, G->ent_cap, X, V, W, G->tstep + i, DF);
       if (i == 0) launch_mixed_predict(P, h->stream, true, launches);
@@ -246,7 +252,7 @@ static int enqueue_recompute(pg_handle* h, int parity, uint32_t len, uint32_t fi
       }
     } else {
       // the recording force kernel writes the tape itself
-      float* DF = G->DF ? G->DF + (size_t)i * N * (h->dim == 2 ? 4 : 6) : nullptr;
+      float* DF = G->DF ? G->DF + (size_t)i * df_floats(h) : nullptr;
       enqueue_rec_step(h, parity, G->off + (size_t)i * N, G->cnt + (size_t)i * N, G->wall + (size_t)i * N, G->ent,
                        G->ent_n, G->ent_cap, launches, X, V, W, G->tstep + i, DF);
     }
@@ -293,7 +299,7 @@ static void enqueue_reverse(pg_handle* h, int cur, uint32_t len, uint32_t first_
     A.xbb = G->xbb;
     A.pcb = G->pcb;
     const bool f32 = h->precision == PG_MIXED && !G->frozen;
-    A.df = f32 ? G->DF + (size_t)ii * N * (h->dim == 2 ? 4 : 6) : nullptr;
+    A.df = f32 ? G->DF + (size_t)ii * df_floats(h) : nullptr;
     A.fbf = f32 ? G->fbf : nullptr;
     launch_adjoint_step(h->P, A, h->stream, launches);
     cur ^= 1;

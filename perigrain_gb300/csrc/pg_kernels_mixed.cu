@@ -18,6 +18,7 @@
 
 #include "pg_common.cuh"
 #include "pg_device.cuh"
+#include "pg_hilo.cuh"
 #include "pg_kernels_mixed.h"
 
 namespace pg {
@@ -86,78 +87,6 @@ __device__ __forceinline__ void split_hl(double x, float* hi, float* lo) {
   *lo = __uint_as_float(sgn | ((unsigned int)(ed - 896) << 23) | frac);
 }
 
-template <int D>
-__device__ __forceinline__ void ld_hl(const float* a, uint32_t i, float (&h)[D], float (&l)[D]) {
-  if constexpr (D == 2) {
-    float4 t = reinterpret_cast<const float4*>(a)[i];
-    h[0] = t.x;
-    h[1] = t.y;
-    l[0] = t.z;
-    l[1] = t.w;
-  } else {
-    const float4* p = reinterpret_cast<const float4*>(a) + 2ull * i;
-    float4 t0 = p[0], t1 = p[1];
-    h[0] = t0.x;
-    h[1] = t0.y;
-    h[2] = t0.z;
-    l[0] = t1.x;
-    l[1] = t1.y;
-    l[2] = t1.z;
-  }
-}
-// bref layout. 2D: one 32-byte record per node, [disp hi.xy, disp lo.xy, xpos hi.xy, xpos lo.xy]
-// (a neighbour gather touches one sector). 3D: 4*3 planes of N floats -- disp hi, disp lo, xpos
-// hi, xpos lo (a padded 3D record would span two sectors; planes keep a warp's gather of the k-th
-// neighbours of 32 consecutive nodes on consecutive entries).
-template <int D>
-__device__ __forceinline__ void ld_ref(const float* __restrict__ bref, uint32_t N, uint32_t i, float (&dh)[D],
-                                       float (&dl)[D], float (&xh)[D], float (&xl)[D]) {
-  if constexpr (D == 2) {
-    const float4* p = reinterpret_cast<const float4*>(bref) + 2ull * i;
-    const float4 a = __ldg(p), b = __ldg(p + 1);
-    dh[0] = a.x;
-    dh[1] = a.y;
-    dl[0] = a.z;
-    dl[1] = a.w;
-    xh[0] = b.x;
-    xh[1] = b.y;
-    xl[0] = b.z;
-    xl[1] = b.w;
-  } else {
-    for (int c = 0; c < D; ++c) {
-      dh[c] = __ldg(bref + (size_t)c * N + i);
-      dl[c] = __ldg(bref + (size_t)(D + c) * N + i);
-      xh[c] = __ldg(bref + (size_t)(2 * D + c) * N + i);
-      xl[c] = __ldg(bref + (size_t)(3 * D + c) * N + i);
-    }
-  }
-}
-template <int D>
-__device__ __forceinline__ void st_ref_disp(float* bref, uint32_t N, uint32_t i, const double (&x)[D]) {
-  float h[D], l[D];
-  for (int c = 0; c < D; ++c) split_hl(x[c], &h[c], &l[c]);
-  if constexpr (D == 2) {
-    reinterpret_cast<float4*>(bref)[2ull * i] = make_float4(h[0], h[1], l[0], l[1]);
-  } else {
-    for (int c = 0; c < D; ++c) {
-      bref[(size_t)c * N + i] = h[c];
-      bref[(size_t)(D + c) * N + i] = l[c];
-    }
-  }
-}
-
-template <int D>
-__device__ __forceinline__ void st_hl(float* a, uint32_t i, const double (&x)[D]) {
-  float h[D], l[D];
-  for (int c = 0; c < D; ++c) split_hl(x[c], &h[c], &l[c]);
-  if constexpr (D == 2) {
-    reinterpret_cast<float4*>(a)[i] = make_float4(h[0], h[1], l[0], l[1]);
-  } else {
-    float4* p = reinterpret_cast<float4*>(a) + 2ull * i;
-    p[0] = make_float4(h[0], h[1], h[2], 0.f);
-    p[1] = make_float4(l[0], l[1], l[2], 0.f);
-  }
-}
 template <int D>
 __device__ __forceinline__ void ldvf(const float* a, uint32_t i, float (&v)[D]) {
   if constexpr (D == 2) {
@@ -229,7 +158,9 @@ __global__ void __launch_bounds__(256) k_predict_mx(const Dev P) {
     }
     if (wrote) {
       stv<D>(P.disp, d, dp);
-      st_ref_disp<D>(P.bref, P.N, d, dp);
+      float dh[D], dl[D];
+      for (int c = 0; c < D; ++c) split_hl(dp[c], &dh[c], &dl[c]);
+      st_hl<D>(P.dref, P.np, d, dh, dl);
     }
     for (int c = 0; c < D; ++c) cu[c] = ps[c] + dp[c];
     stv<D>(P.cur, d, cu);
@@ -368,7 +299,7 @@ __global__ void __launch_bounds__(128) k_force_mx(const Dev P) {
   }
 
   const bool brk = P.enable_fracture && (gr.flags & GF_BREAKABLE) && (gr.flags & GF_BREAK_BONDS);
-  const float cnot = gr.cnot_f, snot = gr.snot_f;
+  const float cnot = gr.cnot_f, snot = brk ? gr.snot_f : INFINITY;  // never exceeded without the break test
   const uint32_t cdeg = P.chunk_deg[chunk];
   const uint32_t slot0 = P.chunk_slot[chunk] + lane;
   const uint32_t w0 = P.chunk_word[chunk];
@@ -376,22 +307,16 @@ __global__ void __launch_bounds__(128) k_force_mx(const Dev P) {
     // bond forces and bond breaking (particle2.h:102-232): two bonds per iteration, both
     // neighbour gathers issued before either is used
     float dh[D], dl[D], xh[D], xl[D];
-    if (mov) ld_ref<D>(P.bref, P.N, d, dh, dl, xh, xl);
+    if (mov) {
+      ld_hl<D>(P.dref, P.np, d, dh, dl);
+      ld_hl<D>(P.xref, P.np, d, xh, xl);
+    }
     if constexpr (REC) {
-      if (mov && P.rec_df) {
-        if constexpr (D == 2) {
-          reinterpret_cast<float4*>(P.rec_df)[d] = make_float4(dh[0], dh[1], dl[0], dl[1]);
-        } else {
-          for (int c = 0; c < D; ++c) {
-            P.rec_df[(size_t)c * P.N + d] = dh[c];
-            P.rec_df[(size_t)(D + c) * P.N + d] = dl[c];
-          }
-        }
-      }
+      if (mov && P.rec_df) st_hl<D>(P.rec_df, P.np, d, dh, dl);
     }
     // the alive words and neighbour indices of the next pair are loaded one iteration ahead, so
     // only the neighbour gathers wait on memory in each iteration. A lane past the last node (d >= N
-    // in the last chunk) gathers its own index for bonds it never uses: bref and vol_f are allocated
+    // in the last chunk) gathers its own index for bonds it never uses: dref, xref and vol_f are allocated
     // in whole chunks (zero padding), so those reads stay inside the arrays.
     uint32_t wa_n = 0u, wb_n = 0u, ca_n = d, cb_n = d;
     if (cdeg > 0) {
@@ -422,17 +347,24 @@ __global__ void __launch_bounds__(128) k_force_mx(const Dev P) {
       const uint32_t ja = ua ? ca : d;
       const uint32_t jb = ub ? cb : d;
       float adh[D], adl[D], axh[D], axl[D], bdh[D], bdl[D], bxh[D], bxl[D];
-      ld_ref<D>(P.bref, P.N, ja, adh, adl, axh, axl);
-      ld_ref<D>(P.bref, P.N, jb, bdh, bdl, bxh, bxl);
+      ld_hl<D>(P.dref, P.np, ja, adh, adl);
+      ld_hl<D>(P.xref, P.np, ja, axh, axl);
+      ld_hl<D>(P.dref, P.np, jb, bdh, bdl);
+      ld_hl<D>(P.xref, P.np, jb, bxh, bxl);
       const float va = P.vol_f[ja], vb = P.vol_f[jb];
       float stra, strb;
       bond_term<D>(dh, dl, xh, xl, adh, adl, axh, axl, cnot * va, ua, f, &stra);
       bond_term<D>(dh, dl, xh, xl, bdh, bdl, bxh, bxl, cnot * vb, ub, f, &strb);
-      if (brk && ua && stra > snot) {
+      // the alive words change only where a bond of the warp breaks: one vote a pair instead of two
+      // ballots and two conditional stores (step times: collision ensemble 74.9 -> 72.5 us, settling
+      // 23.7 -> 22.3, 3D spheres 104.4 -> 99.0, two disks 16.8 -> 15.8)
+      const bool xa = ua && stra > snot, xb = ub && strb > snot;
+      if (!__any_sync(0xffffffffu, xa || xb)) continue;
+      if (xa) {
         ba = false;
         P.break_step[sa] = t;
       }
-      if (brk && ub && strb > snot) {
+      if (xb) {
         bb = false;
         P.break_step[sb] = t;
       }
