@@ -5,6 +5,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 
 #include "pg_device.cuh"
@@ -55,15 +56,26 @@ __device__ __forceinline__ void ldf(const float* a, uint32_t i, float (&v)[D]) {
   }
 }
 
+template <int D>
+__device__ __forceinline__ void stf(float* a, uint32_t i, const float (&v)[D]) {
+  if constexpr (D == 2) {
+    reinterpret_cast<float2*>(a)[i] = make_float2(v[0], v[1]);
+  } else {
+    reinterpret_cast<float4*>(a)[i] = make_float4(v[0], v[1], v[2], 0.f);
+  }
+}
+
 __device__ __forceinline__ void set_status(int32_t* st, int32_t code) { atomicCAS(st, 0, code); }
 
 // Programmatic dependent launch. Every kernel of a step starts with pdl_enter(), which waits until
 // the previous kernel in the stream has finished and its writes are visible; launched with
 // programmatic stream serialization, the kernel's blocks are scheduled while the previous kernel's
-// last blocks drain instead of after it. (No early launch_dependents: letting the next kernel's
-// blocks in while the current one still runs measured slower.) A no-op for a kernel launched
-// without the attribute.
+// last blocks drain instead of after it. pdl_release() lets the next kernel's blocks in once every
+// block of this one has started (they wait in their own pdl_enter): in the force kernels and the
+// grid build it took 1-2 % off every step (collision ensemble 69.4 -> 68.1 us, two disks FP64 24.0 ->
+// 23.4). No-ops for kernels launched without the attribute.
 __device__ __forceinline__ void pdl_enter() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // Launch k<<<g, b, smem, s>>>(args...), with programmatic stream serialization when `pdl`.
 template <class... KArgs, class... Args>
@@ -175,15 +187,10 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* warp_s
   return base + x - v;
 }
 
-// With candidate lists the grid is rebuilt only on rebuild steps; the grid kernels return at once
-// on the other steps.
-__device__ __forceinline__ bool grid_idle(const Dev& P) { return P.cand_q && !*P.rebuild; }
-
 static __global__ void __launch_bounds__(SCAN_THREADS) k_scan_reduce(const Dev P) {
   pdl_enter();
   __shared__ uint32_t ws[32];
   __shared__ bool last;
-  if (grid_idle(P)) return;
   const uint32_t tile = blockIdx.x;
   const uint32_t base = tile * SCAN_TILE + threadIdx.x * SCAN_PER;
   uint32_t s = 0;
@@ -228,7 +235,6 @@ static __global__ void __launch_bounds__(SCAN_THREADS) k_scan_reduce(const Dev P
 static __global__ void __launch_bounds__(SCAN_THREADS) k_scan_final(const Dev P) {
   pdl_enter();
   __shared__ uint32_t ws[32];
-  if (grid_idle(P)) return;
   const uint32_t tile = blockIdx.x;
   const uint32_t base = tile * SCAN_TILE + threadIdx.x * SCAN_PER;
   uint32_t v[SCAN_PER];
@@ -274,27 +280,10 @@ static __global__ void __launch_bounds__(SCAN_THREADS) k_scan_final(const Dev P)
   if (tile == gridDim.x - 1 && threadIdx.x == blockDim.x - 1) P.cell_start[P.table_total] = P.N;
 }
 
-// Node d's entry of the cell-sorted order (and, with candidate lists, its position image and key).
-__device__ __forceinline__ void scatter_node(const Dev& P, uint32_t d) {
-  const uint32_t at = P.cell_start[P.cell_key[d]] + P.cell_rank[d];
-  P.sorted[at] = d;
-  if (P.sorted_key) {
-    const uint32_t g = P.node_grain[d];
-    const uint32_t sub = P.node_sub[d];
-    P.sorted_key[at] = ((unsigned long long)g << 32) | sub;
-    if (P.dim == 2) {
-      reinterpret_cast<float2*>(P.sorted_pos)[at] = reinterpret_cast<const float2*>(P.curf)[d];
-    } else {
-      reinterpret_cast<float4*>(P.sorted_pos)[at] = reinterpret_cast<const float4*>(P.curf)[d];
-    }
-  }
-}
-
 static __global__ void __launch_bounds__(256) k_scatter(const Dev P) {
   pdl_enter();
-  if (grid_idle(P)) return;
   const uint32_t d = blockIdx.x * blockDim.x + threadIdx.x;
-  if (d < P.N) scatter_node(P, d);
+  if (d < P.N) P.sorted[P.cell_start[P.cell_key[d]] + P.cell_rank[d]] = d;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -322,6 +311,39 @@ __device__ __forceinline__ void grain_box(const Dev& P, uint32_t g, double (&mn)
   for (int c = 0; c < D; ++c) {
     mn[c] = ordered_to_dbl(P.bbox[(size_t)g * 2 * D + c]);
     mx[c] = ordered_to_dbl(P.bbox[(size_t)g * 2 * D + D + c]);
+  }
+}
+
+// Per-grain bounding box (contact.h:1024-1062) grown by the positions x of a warp's nodes (all 32
+// lanes call; `act`: the lane has a node, of grain g); min/max are exact, so atomics are
+// deterministic.
+template <int D>
+__device__ __forceinline__ void grow_box(unsigned long long* bbox, uint32_t g, bool act, const double (&x)[D]) {
+  const uint32_t full = 0xffffffffu;
+  const uint32_t lane = threadIdx.x & 31;
+  unsigned long long kmin[D], kmax[D];
+  for (int c = 0; c < D; ++c) {
+    kmin[c] = act ? dbl_to_ordered(x[c]) : ~0ull;
+    kmax[c] = act ? kmin[c] : 0ull;
+  }
+  const uint32_t g0 = __shfl_sync(full, g, 0);
+  if (!__shfl_sync(full, act ? 1 : 0, 0)) return;  // a warp past the last node
+  if (__ballot_sync(full, !act || g == g0) == full) {
+    for (int c = 0; c < D; ++c) {
+      kmin[c] = warp_min_u64(kmin[c]);
+      kmax[c] = warp_max_u64(kmax[c]);
+    }
+    if (lane == 0) {
+      for (int c = 0; c < D; ++c) {
+        atomicMin(&bbox[(size_t)g0 * 2 * D + c], kmin[c]);
+        atomicMax(&bbox[(size_t)g0 * 2 * D + D + c], kmax[c]);
+      }
+    }
+  } else if (act) {
+    for (int c = 0; c < D; ++c) {
+      atomicMin(&bbox[(size_t)g * 2 * D + c], kmin[c]);
+      atomicMax(&bbox[(size_t)g * 2 * D + D + c], kmax[c]);
+    }
   }
 }
 
@@ -429,7 +451,8 @@ __device__ __forceinline__ void finalize_instances(const Dev& P) {
       hi[c] = ordered_to_dbl(mx[c]);
       ok = ok && isfinite(lo[c]) && isfinite(hi[c]);
     }
-    if (ok) fit_grid(*in, D, lo, hi);
+    // with candidate lists the grid is fitted when it is built (refit_instance)
+    if (ok && !P.cand_q) fit_grid(*in, D, lo, hi);
   }
 }
 
@@ -554,7 +577,6 @@ static __global__ void __launch_bounds__(FINAL_THREADS) k_finalize(const Dev P) 
 
 
 inline uint32_t cdiv(uint32_t a, uint32_t b) { return (a + b - 1) / b; }
-__device__ __forceinline__ uint32_t cdiv_dev(uint32_t a, uint32_t b) { return (a + b - 1) / b; }
 
 // ---------------------------------------------------------------------------------------------
 // Contact candidate lists (Verlet lists with a skin): on rebuild steps the grid is recounted and
@@ -563,21 +585,72 @@ __device__ __forceinline__ uint32_t cdiv_dev(uint32_t a, uint32_t b) { return (a
 // last build while no node has moved more than skin/2 since (predict raises `rebuild` at 0.45 skin),
 // so every pair the grid search would evaluate is in the list, in the same order.
 // ---------------------------------------------------------------------------------------------
-// grid keys of a rebuild step (the grid-search path computes them in the predict kernels)
+// Rebuild steps: the grid of instance k fitted to this step's grain boxes by one warp.
 template <int D>
-static __global__ void __launch_bounds__(256) k_keys(const Dev P) {
-  pdl_enter();
-  if (!*P.rebuild) return;
-  const uint32_t d = blockIdx.x * blockDim.x + threadIdx.x;
-  if (d >= P.N) return;
+__device__ __forceinline__ void refit_instance(const Dev& P, uint32_t k) {
+  constexpr int NS = 2 * D;
+  InstDev* in = &P.inst[k];
+  const uint32_t lane = threadIdx.x & 31;
+  unsigned long long mn[D], mx[D];
+  for (int c = 0; c < D; ++c) {
+    mn[c] = ~0ull;
+    mx[c] = 0ull;
+  }
+  const uint32_t gb = in->grain_begin, ge = in->grain_end;
+  for (uint32_t g = gb + lane; g < ge; g += 32)
+    for (int c = 0; c < D; ++c) {
+      const unsigned long long a = P.bbox[(size_t)g * NS + c], b = P.bbox[(size_t)g * NS + D + c];
+      mn[c] = a < mn[c] ? a : mn[c];
+      mx[c] = b > mx[c] ? b : mx[c];
+    }
+  double lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};
+  bool ok = ge > gb;
+  for (int c = 0; c < D; ++c) {
+    lo[c] = ordered_to_dbl(warp_min_u64(mn[c]));
+    hi[c] = ordered_to_dbl(warp_max_u64(mx[c]));
+    ok = ok && isfinite(lo[c]) && isfinite(hi[c]);
+  }
+  if (ok && lane == 0) fit_grid(*in, D, lo, hi);
+}
+
+// Candidate lists keep the nodes of a cell as a chain: cell_start[cell] = its first node (NONE:
+// empty), cell_rank[node] = the next. unlink_node empties the cell node d was chained in at the last
+// build; chain_node puts it into its cell of this step's grid. Where the images are offsets from
+// the grid's origin (rel_frame == 0), which the refit moved, node d's is formed anew.
+__device__ __forceinline__ void unlink_node(const Dev& P, uint32_t d) { P.cell_start[P.cell_key[d]] = NONE; }
+template <int D>
+__device__ __forceinline__ void chain_node(const Dev& P, uint32_t d) {
   const InstDev& in = P.inst[P.grain[P.node_grain[d]].inst];
   float rf[D];
-  ldf<D>(P.curf, d, rf);
+  if (in.rel_frame) {
+    ldf<D>(P.curf, d, rf);
+  } else {
+    double cu[D];
+    ldv<D>(P.cur, d, cu);
+    for (int c = 0; c < D; ++c) rf[c] = (float)(cu[c] - in.origin[c]);
+    stf<D>(P.curf, d, rf);
+  }
   int32_t ci[3] = {0, 0, 0};
   for (int c = 0; c < D; ++c) ci[c] = cell_coord(rf[c] + in.frame_off_f[c], in.inv_cell_f, in.dims[c]);
   const uint32_t key = in.table_off + ((uint32_t)ci[2] * in.dims[1] + (uint32_t)ci[1]) * in.dims[0] + (uint32_t)ci[0];
   P.cell_key[d] = key;
-  P.cell_rank[d] = atomicAdd(&P.cell_count[key], 1u);
+  P.cell_rank[d] = atomicExch(&P.cell_start[key], d);
+}
+// The build in separate launches, for devices without a cooperative one.
+template <int D>
+static __global__ void __launch_bounds__(256) k_refit(const Dev P) {
+  pdl_enter();
+  if (!*P.rebuild) return;
+  const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
+  if (tid < P.N) unlink_node(P, tid);
+  if ((tid >> 5) < P.I) refit_instance<D>(P, tid >> 5);
+}
+template <int D>
+static __global__ void __launch_bounds__(256) k_chain(const Dev P) {
+  pdl_enter();
+  if (!*P.rebuild) return;
+  const uint32_t d = blockIdx.x * blockDim.x + threadIdx.x;
+  if (d < P.N) chain_node<D>(P, d);
 }
 
 // Rebuild of node d's list: every node q of the 3x3 (3x3x3) cells within the FP32 radius pre_b that
@@ -613,37 +686,41 @@ __device__ __forceinline__ void cand_build_node(const Dev& P, uint32_t d) {
     for (int z = z0; z <= z1; ++z)
       for (int y = y0; y <= y1; ++y) {
         const uint32_t row = in.table_off + ((uint32_t)z * in.dims[1] + (uint32_t)y) * in.dims[0];
-        const uint32_t b0 = P.cell_start[row + x0], b1 = P.cell_start[row + x1 + 1];
-        for (uint32_t b = b0; b < b1; ++b) {
-          // the cell's entries are consecutive: index, position image and key without gathers
-          const uint32_t q = P.sorted[b];
-          float qf[D];
-          ldf<D>(P.sorted_pos, b, qf);
-          const unsigned long long qk = P.sorted_key[b];
-          if (q == d) continue;
-          float d2 = 0.f;
-          for (int c = 0; c < D; ++c) {
-            const float dd = qf[c] - pf[c];
-            d2 += dd * dd;
+        uint32_t first[3];  // the row's three chains, started together
+        for (int i = 0; i < 3; ++i) first[i] = x0 + i <= x1 ? P.cell_start[row + x0 + i] : NONE;
+        for (int i = 0; i < 3; ++i) {
+          uint32_t qn = first[i];
+          while (qn != NONE) {
+            const uint32_t q = qn;
+            qn = P.cell_rank[q];
+            float qf[D];
+            ldf<D>(P.curf, q, qf);
+            if (q == d) continue;
+            float d2 = 0.f;
+            for (int c = 0; c < D; ++c) {
+              const float dd = qf[c] - pf[c];
+              d2 += dd * dd;
+            }
+            if (d2 > thr2) continue;
+            const uint32_t gq = P.node_grain[q], sub = P.node_sub[q];
+            const bool same = gq == g;
+            if (same ? !selfc : !other) continue;
+            if (P.nl_bdry_only && sub == NONE) continue;
+            const unsigned long long key =
+                ((unsigned long long)(same ? 0u : 1u) << 63) | ((unsigned long long)gq << 32) | sub;
+            if (n >= P.cand_cap) {
+              set_status(P.status, PG_ECAPACITY);
+              continue;
+            }
+            int k = (int)n++;
+            while (k > 0 && keys[k - 1] > key) {
+              keys[k] = keys[k - 1];
+              idx[k] = idx[k - 1];
+              --k;
+            }
+            keys[k] = key;
+            idx[k] = q;
           }
-          if (d2 > thr2) continue;
-          const uint32_t gq = (uint32_t)(qk >> 32), sub = (uint32_t)qk;
-          const bool same = gq == g;
-          if (same ? !selfc : !other) continue;
-          if (P.nl_bdry_only && sub == NONE) continue;
-          const unsigned long long key = ((unsigned long long)(same ? 0u : 1u) << 63) | qk;
-          if (n >= P.cand_cap) {
-            set_status(P.status, PG_ECAPACITY);
-            continue;
-          }
-          int k = (int)n++;
-          while (k > 0 && keys[k - 1] > key) {
-            keys[k] = keys[k - 1];
-            idx[k] = idx[k - 1];
-            --k;
-          }
-          keys[k] = key;
-          idx[k] = q;
         }
       }
     const size_t base = (size_t)chunk * P.cand_cap * 32 + lane;
@@ -661,11 +738,16 @@ static __global__ void __launch_bounds__(128) k_cand_build(const Dev P) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// Cooperative grid build (candidate lists): keys and counts, scan of the counts, scatter and the
-// candidate-list rebuild in one launch of co-resident blocks separated by grid barriers, so a step
-// without a rebuild costs one idle launch here instead of five. The barrier waits are bounded: past GBAR_SPIN_LIMIT polls a
-// block records PG_ETIMEOUT and returns (the step's status then reports it).
+// Cooperative grid build (candidate lists): the end of the step before (fused runs) and, on rebuild
+// steps, the grid refit, the cells' node chains and the candidate lists, in one launch of co-resident
+// blocks separated by grid barriers, so a step without a rebuild costs one idle launch (2.5 us). Bound
+// by the latency of the dependent loads of each phase and by the barriers: chains need two barriers
+// where a counting sort (counts, tile sums, their scan, starts, scatter) needed six, which took the
+// collision ensemble's step from 68.1 to 64.0 us at a rebuild every ten steps or so. The barrier
+// waits are bounded: past GBAR_SPIN_LIMIT polls a block records PG_ETIMEOUT and returns (the step's
+// status then reports it).
 // ---------------------------------------------------------------------------------------------
+constexpr int COOP_THREADS = 256;
 constexpr uint32_t GBAR_SPIN_LIMIT = 1u << 22;  // polls of ~64 ns: about 0.3 s
 
 __device__ __forceinline__ bool grid_barrier(const Dev& P, uint32_t* ok_smem) {
@@ -701,126 +783,64 @@ __device__ __forceinline__ bool grid_barrier(const Dev& P, uint32_t* ok_smem) {
   return *ok_smem != 0;
 }
 
-// SCAN_PER consecutive cell counts from `base` (a multiple of SCAN_PER): four 16-byte loads when the
-// run lies inside the table, element by element at its end (zeros past it).
-__device__ __forceinline__ void load_counts(const Dev& P, uint32_t base, uint32_t (&v)[SCAN_PER]) {
-  if (base + SCAN_PER <= P.table_total) {
-    const uint4* q4 = reinterpret_cast<const uint4*>(P.cell_count + base);
-    for (int k = 0; k < SCAN_PER / 4; ++k) {
-      const uint4 q = q4[k];
-      v[4 * k] = q.x;
-      v[4 * k + 1] = q.y;
-      v[4 * k + 2] = q.z;
-      v[4 * k + 3] = q.w;
-    }
-  } else {
-    for (int k = 0; k < SCAN_PER; ++k) v[k] = base + k < P.table_total ? P.cell_count[base + k] : 0u;
+// End of the step before inside a fused run, over all threads of the grid: the wall move
+// (timeloop.h:866-878), the pair log, counters, and the boxes and rebuild flag of its parity cleared
+// for the position update of the next force kernel. The wall reactions of a step inside a run are
+// overwritten by the next step's and seen by nobody: k_finalize sums the last step's.
+template <int D>
+__device__ __forceinline__ void end_of_step(const Dev& P) {
+  constexpr uint32_t NS = 2 * D;
+  const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, nthr = gridDim.x * blockDim.x;
+  for (uint32_t i = tid; i < P.G * NS; i += nthr) P.bbox_n[i] = (i % NS) < (uint32_t)D ? ~0ull : 0ull;
+  for (uint32_t i = tid; i < P.I * NS; i += nthr) {
+    InstDev* in = &P.inst[i / NS];
+    in->wall[i % NS] = in->wall[i % NS] + in->wall_speed[i % NS] * P.dt;
   }
-}
-// Cell starts of the run at `base`, and its counts cleared for the next build.
-__device__ __forceinline__ void store_starts_clear_counts(const Dev& P, uint32_t base, const uint32_t (&st)[SCAN_PER]) {
-  if (base + SCAN_PER <= P.table_total) {
-    uint4* s4 = reinterpret_cast<uint4*>(P.cell_start + base);  // base is a multiple of 16 entries
-    uint4* z4 = reinterpret_cast<uint4*>(P.cell_count + base);
-    for (int k = 0; k < SCAN_PER / 4; ++k) {
-      s4[k] = make_uint4(st[4 * k], st[4 * k + 1], st[4 * k + 2], st[4 * k + 3]);
-      z4[k] = make_uint4(0u, 0u, 0u, 0u);
-    }
-  } else {
-    for (int k = 0; k < SCAN_PER; ++k)
-      if (base + k < P.table_total) {
-        P.cell_start[base + k] = st[k];
-        P.cell_count[base + k] = 0u;
-      }
+  if (tid != 0) return;
+  const uint32_t R = *P.wrec_count, t = *P.step;
+  if (R > 0 && (R > P.wrec_smem || R > P.wrec_cap)) set_status(P.status, PG_ECAPACITY);
+  if (P.record_pairs) {
+    const uint32_t slot = (t - 1) % P.log_cap;
+    P.log_count[slot] = P.pair_acc[0];
+    P.log_hash[slot] = P.pair_acc[1];
+    P.pair_acc[0] = 0;
+    P.pair_acc[1] = 0;
   }
+  *P.wrec_count = 0;
+  *P.step = t + 1;
+  *P.rebuild_n = 0;
 }
 
 template <int D>
-static __global__ void __launch_bounds__(SCAN_THREADS) k_grid_coop(const Dev P) {
+static __global__ void __launch_bounds__(COOP_THREADS) k_grid_coop(const Dev P) {
   pdl_enter();
-  __shared__ uint32_t ws[32];
+  pdl_release();
   __shared__ uint32_t ok;
-  __shared__ bool last;
-  if (!*P.rebuild) return;  // set by the predict kernel before this launch: the same for every block
+  if (P.turn_prev) end_of_step<D>(P);
+  if (!*P.rebuild) return;  // set by the position update before this launch: the same for every block
   // a barrier of an earlier launch timed out: the handle is halted (the host refuses further steps
   // once it sees PG_ETIMEOUT; launches already enqueued return here)
   if (((volatile uint32_t*)P.gbar)[2]) return;
-  const uint32_t nthr = gridDim.x * blockDim.x;
-  // 1. grid keys and per-cell ranks
-  for (uint32_t d = blockIdx.x * blockDim.x + threadIdx.x; d < P.N; d += nthr) {
-    const InstDev& in = P.inst[P.grain[P.node_grain[d]].inst];
-    float rf[D];
-    ldf<D>(P.curf, d, rf);
-    int32_t ci[3] = {0, 0, 0};
-    for (int c = 0; c < D; ++c) ci[c] = cell_coord(rf[c] + in.frame_off_f[c], in.inv_cell_f, in.dims[c]);
-    const uint32_t key = in.table_off + ((uint32_t)ci[2] * in.dims[1] + (uint32_t)ci[1]) * in.dims[0] + (uint32_t)ci[0];
-    P.cell_key[d] = key;
-    P.cell_rank[d] = atomicAdd(&P.cell_count[key], 1u);
-  }
+  const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, nthr = gridDim.x * blockDim.x;
+  // 0. the last build's chains emptied, grids fitted to this step's boxes (one warp per instance)
+  for (uint32_t d = tid; d < P.N; d += nthr) unlink_node(P, d);
+  for (uint32_t k = tid >> 5; k < P.I; k += nthr >> 5) refit_instance<D>(P, k);
   if (!grid_barrier(P, &ok)) return;
-  // 2. tile sums of the counts
-  const uint32_t ntiles = cdiv_dev(P.table_total, SCAN_TILE);
-  for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const uint32_t base = tile * SCAN_TILE + threadIdx.x * SCAN_PER;
-    uint32_t v[SCAN_PER], sum = 0;
-    load_counts(P, base, v);
-    for (int k = 0; k < SCAN_PER; ++k) sum += v[k];
-    uint32_t tot;
-    block_excl_scan(sum, ws, &tot);
-    if (threadIdx.x == 0) P.scan_tile_sum[tile] = tot;
-    __syncthreads();
-  }
+  // 1. chains
+  for (uint32_t d = tid; d < P.N; d += nthr) chain_node<D>(P, d);
   if (!grid_barrier(P, &ok)) return;
-  // 3. exclusive scan of the tile sums (block 0)
-  if (blockIdx.x == 0) {
-    uint32_t carry = 0;
-    for (uint32_t b0 = 0; b0 < ntiles; b0 += SCAN_THREADS) {
-      const uint32_t i = b0 + threadIdx.x;
-      const uint32_t v = i < ntiles ? ((volatile uint32_t*)P.scan_tile_sum)[i] : 0;
-      uint32_t t2;
-      const uint32_t ex = block_excl_scan(v, ws, &t2);
-      __syncthreads();
-      if (i < ntiles) P.scan_tile_sum[i] = carry + ex;
-      carry += t2;
-      __syncthreads();
-    }
-  }
-  (void)last;
-  if (!grid_barrier(P, &ok)) return;
-  // 4. cell starts, counts cleared for the next build
-  for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const uint32_t base = tile * SCAN_TILE + threadIdx.x * SCAN_PER;
-    uint32_t v[SCAN_PER], sum = 0;
-    load_counts(P, base, v);
-    for (int k = 0; k < SCAN_PER; ++k) sum += v[k];
-    uint32_t ex = block_excl_scan(sum, ws, nullptr) + ((volatile uint32_t*)P.scan_tile_sum)[tile];
-    uint32_t st[SCAN_PER];
-    for (int k = 0; k < SCAN_PER; ++k) {
-      st[k] = ex;
-      ex += v[k];
-    }
-    store_starts_clear_counts(P, base, st);
-    __syncthreads();
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) P.cell_start[P.table_total] = P.N;
-  if (!grid_barrier(P, &ok)) return;
-  // 5. scatter
-  for (uint32_t d = blockIdx.x * blockDim.x + threadIdx.x; d < P.N; d += nthr) scatter_node(P, d);
-  if (!grid_barrier(P, &ok)) return;
-  // 6. candidate lists
-  for (uint32_t d = blockIdx.x * blockDim.x + threadIdx.x; d < P.N; d += nthr) cand_build_node<D>(P, d);
+  // 2. candidate lists
+  for (uint32_t d = tid; d < P.N; d += nthr) cand_build_node<D>(P, d);
 }
 
-// Grid build shared by both precisions: exclusive scan of the bucket counts, then scatter; with
-// candidate lists also the grid keys (before) and the list rebuild (after), all of them returning
-// at once on steps that need no rebuild.
+// Grid build shared by both precisions: with candidate lists the cooperative launch above; for the
+// grid search the exclusive scan of the bucket counts, then the scatter.
 template <int D>
 inline void launch_grid_build(const Dev& P, cudaStream_t s, uint64_t* launches, bool pdl = false) {
-  const uint32_t ntiles = cdiv(P.table_total, SCAN_TILE);
   if (P.cand_q && P.coop_blocks) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(P.coop_blocks);
-    cfg.blockDim = dim3(SCAN_THREADS);
+    cfg.blockDim = dim3(COOP_THREADS);
     cfg.stream = s;
     cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeCooperative;
@@ -834,17 +854,17 @@ inline void launch_grid_build(const Dev& P, cudaStream_t s, uint64_t* launches, 
     return;
   }
   if (P.cand_q) {
-    launch_k(k_keys<D>, cdiv(P.N, 256), 256, 0, s, pdl, P);
-    *launches += 1;
+    launch_k(k_refit<D>, cdiv(std::max(P.N, P.I * 32), 256), 256, 0, s, pdl, P);
+    launch_k(k_chain<D>, cdiv(P.N, 256), 256, 0, s, pdl, P);
+    launch_k(k_cand_build<D>, cdiv(P.N, 128), 128, 0, s, pdl, P);
+    *launches += 3;
+    return;
   }
+  const uint32_t ntiles = cdiv(P.table_total, SCAN_TILE);
   launch_k(k_scan_reduce, ntiles, SCAN_THREADS, 0, s, pdl, P);
   launch_k(k_scan_final, ntiles, SCAN_THREADS, 0, s, pdl, P);
   launch_k(k_scatter, cdiv(P.N, 256), 256, 0, s, pdl, P);
   *launches += 3;
-  if (P.cand_q) {
-    launch_k(k_cand_build<D>, cdiv(P.N, 128), 128, 0, s, pdl, P);
-    *launches += 1;
-  }
 }
 
 }  // namespace pg

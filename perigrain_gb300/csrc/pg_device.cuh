@@ -171,11 +171,8 @@ struct Dev {
   uint8_t *clamped, *clamp_pending;
   // grid
   uint32_t *cell_key, *cell_rank, *cell_count, *cell_start, *sorted;
-  // with candidate lists, beside `sorted`: each entry's FP32 position image (curf layout) and
-  // candidate key (grain << 32 | rank in the reference's loop order, NONE for a node outside the
-  // nonlocal boundary when nl_bdry_only), so a list rebuild reads a cell's nodes contiguously
-  float* sorted_pos;
-  unsigned long long* sorted_key;
+  // (grid search: per-cell counts, the cell-sorted node list and cell starts; candidate lists: the
+  // cells' node chains, cell_start = first node of a cell, cell_rank = next node of the chain)
   uint32_t *scan_tile_sum;
   uint32_t *scan_done;
   uint32_t* gbar;      // [3] grid barrier of the cooperative grid build: arrivals, generation,
@@ -247,6 +244,15 @@ struct Dev {
   // and volume.
   uint32_t np;
   float *dref, *xref;
+  // Steps run fused inside one call (candidate lists and the cooperative grid build): with `fuse`
+  // the force kernel also does the next step's position update, into the other step parity's
+  // buffers; with `turn_prev` the grid build first does the end of the step before (walls, logs,
+  // counters, that parity's boxes and rebuild flag).
+  int32_t fuse, turn_prev;
+  double* cur_n;
+  float *curf_n, *dref_n;
+  unsigned long long* bbox_n;
+  uint32_t* rebuild_n;
   float *acc_f, *force_f, *extf_f, *vol_f;
   float dt_f, hdt2_f, half_dt_f;
 };

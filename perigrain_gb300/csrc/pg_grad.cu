@@ -55,7 +55,6 @@ static int ensure_regions(pg_handle* h) {
   if (h->precision == PG_MIXED) {
     const size_t SF = (D == 2) ? 2 : 4;
     add(P.acc_f, N * SF * 4);
-    add(P.dref, (size_t)P.np * (D == 2 ? HL_FLOATS<2> : HL_FLOATS<3>) * 4);
   }
   CU(cudaEventCreate(&G->e0));
   CU(cudaEventCreate(&G->e1));
@@ -139,11 +138,9 @@ static void enqueue_rec_step(pg_handle* h, int parity, uint32_t* off, uint8_t* c
                              double* v = nullptr, double* w = nullptr, uint32_t* tstep = nullptr,
                              float* df = nullptr) {
   const Dev P = rec_dev(h, parity, off, cnt, wall, ent, ent_n, cap, x, v, w, tstep, df);
-  if (h->precision == PG_MIXED) {
-    launch_step_mixed(P, h->L, h->stream, launches, nullptr, nullptr, true);
-  } else {
-    launch_step(P, h->L, h->stream, launches, true);
-  }
+  enqueue_predict(h, P, launches);
+  enqueue_body(h, P, launches, true);
+  enqueue_finalize(h, P, launches);
 }
 
 // one FP64 step replaying masks number `idx` of m
@@ -228,28 +225,18 @@ static int enqueue_recompute(pg_handle* h, int parity, uint32_t len, uint32_t fi
       enqueue_replay_step(h, parity, G->frozen, first_idx + i, G->frozen->end_alive, G->frozen->break_step, nullptr,
                           launches);
       const double* vin = parity == 0 ? h->vel_a : h->vel_b;
-      CU(cudaMemcpyAsync(X, h->P.cur, N * S * 8, cudaMemcpyDeviceToDevice, h->stream));
+      CU(cudaMemcpyAsync(X, h->cur_pp[parity], N * S * 8, cudaMemcpyDeviceToDevice, h->stream));
       CU(cudaMemcpyAsync(V, vin, N * S * 8, cudaMemcpyDeviceToDevice, h->stream));
-    } else if (h->overlap) {
-      // the recording steps with each finalize beside the next position update, as in the
-      // forward graphs (bit-identical to the serial order)
+    } else if (h->fused) {
+      // a fused run of recording steps, as run_steps
       float* DF = G->DF ? G->DF + (size_t)i * df_floats(h) : nullptr;
-      const Dev P = rec_dev(h, parity, G->off + (size_t)i * N, G->cnt + (size_t)i * N, G->wall + (size_t)i * N,
-                            G->ent, G->ent_n, G->ent_cap, X, V, W, G->tstep + i, DF);
-      if (i == 0) launch_mixed_predict(P, h->stream, true, launches);
-      if (i > 0) cudaStreamWaitEvent(h->stream, h->ev_join, 0);
-      launch_mixed_body(P, h->L, h->stream, true, launches, true);
-      if (i + 1 < len) {
-        cudaEventRecord(h->ev_fork, h->stream);
-        cudaStreamWaitEvent(h->side, h->ev_fork, 0);
-        launch_mixed_finalize(P, h->side, false, launches);
-        cudaEventRecord(h->ev_join, h->side);
-        Dev Pn = h->P;
-        set_vel(h, Pn, parity ^ 1);
-        launch_mixed_predict(Pn, h->stream, true, launches);
-      } else {
-        launch_mixed_finalize(P, h->stream, true, launches);
-      }
+      Dev P = rec_dev(h, parity, G->off + (size_t)i * N, G->cnt + (size_t)i * N, G->wall + (size_t)i * N, G->ent,
+                      G->ent_n, G->ent_cap, X, V, W, G->tstep + i, DF);
+      if (i == 0) enqueue_predict(h, P, launches);
+      P.turn_prev = i > 0;
+      P.fuse = i + 1 < len;
+      enqueue_body(h, P, launches, true);
+      if (i + 1 == len) enqueue_finalize(h, P, launches);
     } else {
       // the recording force kernel writes the tape itself
       float* DF = G->DF ? G->DF + (size_t)i * df_floats(h) : nullptr;
@@ -387,6 +374,7 @@ int pg_grad_reset(pg_handle* h) {
   if (!h) return fail(PG_EINVAL, "null handle");
   if (!h->grad || !h->grad->have_origin) return fail(PG_EINVAL, "no origin: call pg_grad_begin first");
   int rc = restore_state(h, 0);
+  if (!rc) rc = refresh_currpos(h);
   if (rc) return rc;
   CU(cudaStreamSynchronize(h->stream));
   return PG_OK;
@@ -499,18 +487,8 @@ int pg_grad_forward(pg_handle* h, uint32_t n_steps, uint32_t checkpoint_every, c
         h->next_t += 1;
       }
     } else {
-      uint32_t i = 0;
-      while (i < len) {
-        if (len - i >= (uint32_t)pg_handle::GRAPH_STEPS) {
-          CU(cudaGraphLaunch(h->graph[h->vel_parity], h->stream));
-          launches += h->graph_launches_per;
-          i += pg_handle::GRAPH_STEPS;
-        } else {
-          enqueue_step(h, h->vel_parity, &launches);
-          h->vel_parity ^= 1;
-          ++i;
-        }
-      }
+      rc = run_steps(h, len, &launches);
+      if (rc) return rc;
       h->next_t += len;
     }
   }
@@ -645,6 +623,7 @@ int pg_grad_backward(pg_handle* h, const double* disp_bar, const double* vel_bar
     h->last_launches = launches;
     CU(cudaMemcpy(grad, G->gradd, NG * NPARAM * 8, cudaMemcpyDeviceToHost));
     rc = restore_state(h, G->final_slot);
+    if (!rc) rc = refresh_currpos(h);
     if (rc) return rc;
     CU(cudaStreamSynchronize(h->stream));
     return PG_OK;

@@ -160,14 +160,17 @@ struct pg_handle {
   int vel_parity = 0;  // 0: current velocity in vel_a
   double* vel_a = nullptr;
   double* vel_b = nullptr;
-  // per step parity (the parity of vel_in): grain boxes and the list-rebuild flag of the step's
-  // positions, so the next step's position update can run beside this step's finalize
+  // per step parity (the parity of vel_in): the step's positions and their images, grain boxes and
+  // list-rebuild flag, so the force kernel of one step can do the next step's position update
+  double* cur_pp[2] = {nullptr, nullptr};
+  float* curf_pp[2] = {nullptr, nullptr};
+  float* dref_pp[2] = {nullptr, nullptr};
   unsigned long long* bbox_pp[2] = {nullptr, nullptr};
   uint32_t* rebuild_pp[2] = {nullptr, nullptr};
-  // the finalize of one step beside the next step's position update (graphs of the mixed path)
-  cudaStream_t side = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-  bool overlap = false;
+  // steps of one call run fused (Dev::fuse, Dev::turn_prev): candidate lists and the cooperative build
+  bool fused = false;
+  // CurrPos of the last step: the buffer of its parity
+  double* cur() const { return cur_pp[vel_parity ^ 1]; }
   bool xpos_separate = false;
   // set when a status check saw PG_ETIMEOUT (a bounded device wait ran out): pg_step refuses
   bool halted = false;
@@ -210,9 +213,6 @@ struct pg_handle {
     for (auto e : ev) cudaEventDestroy(e);
     if (ev_t0) cudaEventDestroy(ev_t0);
     if (ev_t1) cudaEventDestroy(ev_t1);
-    if (ev_fork) cudaEventDestroy(ev_fork);
-    if (ev_join) cudaEventDestroy(ev_join);
-    if (side) cudaStreamDestroy(side);
     for (void* p : allocs) cudaFree(p);
     if (xpos_separate) cudaFree(P.xpos);
     if (stream) cudaStreamDestroy(stream);
@@ -230,6 +230,14 @@ struct pg_handle {
 void set_vel(pg_handle* h, pg::Dev& P, int parity);
 // Enqueue one engine step with the current velocity parity `parity` (does not flip it).
 void enqueue_step(pg_handle* h, int parity, uint64_t* launches);
+// The parts of a step in the handle's precision.
+void enqueue_predict(pg_handle* h, const pg::Dev& P, uint64_t* launches);
+void enqueue_body(pg_handle* h, const pg::Dev& P, uint64_t* launches, bool rec);
+void enqueue_finalize(pg_handle* h, const pg::Dev& P, uint64_t* launches);
+// Run n steps from the handle's state: the graphs where they fit. Advances the parity, not next_t.
+int run_steps(pg_handle* h, uint32_t n, uint64_t* launches);
+// CurrPos = pos + disp of the state at hand into its buffer (a restored state brings only disp).
+int refresh_currpos(pg_handle* h);
 int build_graphs(pg_handle* h);
 int check_device_status(pg_handle* h);
 // PG_OK for st == 0, else records the device status message and returns st.

@@ -25,6 +25,41 @@
 
 namespace pg {
 
+// CurrPos of node d from its displacement, the FP32 image, and either the list-rebuild check (with
+// candidate lists: once any node has moved 0.45 skin since the last build) or the node's grid key.
+template <int D>
+__device__ __forceinline__ void place_node(const Dev& P, uint32_t d, const InstDev& in, const double (&dp)[D],
+                                           double* cur, float* curf, uint32_t* rebuild, double (&cu)[D]) {
+  double ps[D];
+  ldv<D>(P.pos, d, ps);
+  for (int c = 0; c < D; ++c) cu[c] = ps[c] + dp[c];
+  stv<D>(cur, d, cu);
+  // the FP32 offset to the grid origin
+  float rf[D];
+  bool ok = true;
+  for (int c = 0; c < D; ++c) {
+    if (!isfinite(cu[c])) ok = false;
+    rf[c] = (float)(cu[c] - in.origin[c]);
+  }
+  if (!ok) set_status(P.status, PG_ENAN);
+  stf<D>(curf, d, rf);
+  if (P.cand_q) {
+    constexpr uint32_t SF = (D == 2) ? 2 : 4;
+    float m2 = 0.f;
+    for (int c = 0; c < D; ++c) {
+      const float dd = (float)dp[c] - P.disp_b[(size_t)d * SF + c];
+      m2 += dd * dd;
+    }
+    if (m2 > in.skin_lim2) *rebuild = 1;
+  } else {
+    int32_t ci[3] = {0, 0, 0};
+    for (int c = 0; c < D; ++c) ci[c] = cell_coord(rf[c] + in.frame_off_f[c], in.inv_cell_f, in.dims[c]);
+    const uint32_t key = in.table_off + ((uint32_t)ci[2] * in.dims[1] + (uint32_t)ci[1]) * in.dims[0] + (uint32_t)ci[0];
+    P.cell_key[d] = key;
+    P.cell_rank[d] = atomicAdd(&P.cell_count[key], 1u);
+  }
+}
+
 // ---------------------------------------------------------------------------------------------
 // k_predict: disp += dt*vel + (dt*dt*0.5)*acc for movable grains; CurrPos = pos + disp.
 // ---------------------------------------------------------------------------------------------
@@ -32,14 +67,14 @@ template <int D>
 __global__ void __launch_bounds__(256) k_predict(const Dev P) {
   pdl_enter();
   const uint32_t d = blockIdx.x * blockDim.x + threadIdx.x;
-  const uint32_t lane = threadIdx.x & 31;
   const bool act = d < P.N;
   uint32_t g = 0;
-  unsigned long long kmin[D], kmax[D];
+  double cu[D];
+  for (int c = 0; c < D; ++c) cu[c] = 0.0;
   if (act) {
     g = P.node_grain[d];
     const GrainDev& gr = P.grain[g];
-    double dp[D], ps[D], cu[D];
+    double dp[D];
     ldv<D>(P.disp, d, dp);
     bool wrote = false;
     if (P.clamp_pending[d]) {
@@ -56,74 +91,9 @@ __global__ void __launch_bounds__(256) k_predict(const Dev P) {
       wrote = true;
     }
     if (wrote) stv<D>(P.disp, d, dp);
-    ldv<D>(P.pos, d, ps);
-    for (int c = 0; c < D; ++c) cu[c] = ps[c] + dp[c];
-    stv<D>(P.cur, d, cu);
-
-    // grid cell from the FP32 offset to this step's grid origin
-    const InstDev& in = P.inst[gr.inst];
-    float rf[4] = {0.f, 0.f, 0.f, 0.f};
-    int32_t ci[3] = {0, 0, 0};
-    bool ok = true;
-    for (int c = 0; c < D; ++c) {
-      if (!isfinite(cu[c])) ok = false;
-      rf[c] = (float)(cu[c] - in.origin[c]);
-      ci[c] = cell_coord(rf[c] + in.frame_off_f[c], in.inv_cell_f, in.dims[c]);
-    }
-    if (!ok) set_status(P.status, PG_ENAN);
-    if constexpr (D == 2) {
-      reinterpret_cast<float2*>(P.curf)[d] = make_float2(rf[0], rf[1]);
-    } else {
-      reinterpret_cast<float4*>(P.curf)[d] = make_float4(rf[0], rf[1], rf[2], 0.f);
-    }
-    const uint32_t key = in.table_off + ((uint32_t)ci[2] * in.dims[1] + (uint32_t)ci[1]) * in.dims[0] + (uint32_t)ci[0];
-    if (P.cand_q) {
-      // candidate lists: keys only on rebuild steps (k_keys); rebuild once any node has moved
-      // 0.45 skin since the last build
-      constexpr uint32_t SF = (D == 2) ? 2 : 4;
-      float m2 = 0.f;
-      for (int c = 0; c < D; ++c) {
-        const float dd = (float)dp[c] - P.disp_b[(size_t)d * SF + c];
-        m2 += dd * dd;
-      }
-      if (m2 > in.skin_lim2) *P.rebuild = 1;
-    } else {
-      P.cell_key[d] = key;
-      P.cell_rank[d] = atomicAdd(&P.cell_count[key], 1u);
-    }
-    for (int c = 0; c < D; ++c) {
-      kmin[c] = dbl_to_ordered(cu[c]);
-      kmax[c] = kmin[c];
-    }
-  } else {
-    for (int c = 0; c < D; ++c) {
-      kmin[c] = ~0ull;
-      kmax[c] = 0ull;
-    }
+    place_node<D>(P, d, P.inst[gr.inst], dp, P.cur, P.curf, P.rebuild, cu);
   }
-  // per-grain bounding box (contact.h:1024-1062), min/max are exact so atomics are deterministic
-  const uint32_t full = 0xffffffffu;
-  uint32_t g0 = __shfl_sync(full, g, 0);
-  bool lane0_act = __shfl_sync(full, act ? 1 : 0, 0);
-  if (!lane0_act) return;
-  uint32_t same = __ballot_sync(full, !act || g == g0);
-  if (same == full) {
-    for (int c = 0; c < D; ++c) {
-      kmin[c] = warp_min_u64(kmin[c]);
-      kmax[c] = warp_max_u64(kmax[c]);
-    }
-    if (lane == 0) {
-      for (int c = 0; c < D; ++c) {
-        atomicMin(&P.bbox[(size_t)g0 * 2 * D + c], kmin[c]);
-        atomicMax(&P.bbox[(size_t)g0 * 2 * D + D + c], kmax[c]);
-      }
-    }
-  } else if (act) {
-    for (int c = 0; c < D; ++c) {
-      atomicMin(&P.bbox[(size_t)g * 2 * D + c], kmin[c]);
-      atomicMax(&P.bbox[(size_t)g * 2 * D + D + c], kmax[c]);
-    }
-  }
+  grow_box<D>(P.bbox, g, act, cu);
 }
 
 // Addend of one bond of a node, the reference's operations in its order, for any operands: the
@@ -265,6 +235,7 @@ __global__ void __launch_bounds__(256) k_bonds(const Dev P) {
 template <int D, bool REC, bool GC>
 __global__ void __launch_bounds__(128) k_force(const Dev P) {
   pdl_enter();
+  pdl_release();
   const uint32_t d = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t chunk = d >> 5;
@@ -594,8 +565,11 @@ __global__ void __launch_bounds__(128) k_force(const Dev P) {
     }
   }
 
-  // ---- velocity update (timeloop.h:834-863) ----
+  // ---- velocity update (timeloop.h:834-863); with P.fuse the next step's position update too ----
+  double cu[D], dp[D];
+  for (int c = 0; c < D; ++c) cu[c] = 0.0;
   if (act) {
+    if (P.fuse) ldv<D>(P.disp, d, dp);
     if (mov) {
       double ao[D], a[D], v[D];
       ldv<D>(P.acc, d, ao);
@@ -610,16 +584,29 @@ __global__ void __launch_bounds__(128) k_force(const Dev P) {
           a[c] = 0.0;
           v[c] = 0.0;
         }
-        P.clamp_pending[d] = 1;
+        if (P.fuse) {
+          for (int c = 0; c < D; ++c) dp[c] = 0.0;
+        } else {
+          P.clamp_pending[d] = 1;
+        }
       }
       if (P.worm) worm_clamp<D>(orig_of(P, d) - gr.node_begin, worm_phase(t), a, v);
       stv<D>(P.acc, d, a);
       stv<D>(P.vel_out, d, v);
+      if (P.fuse) {
+        for (int c = 0; c < D; ++c) dp[c] = dp[c] + ((P.dt * v[c]) + (P.hdt2 * a[c]));
+        stv<D>(P.disp, d, dp);
+      }
     } else {
       stv<D>(P.vel_out, d, vp);
     }
-    stv<D>(P.force, d, f);  // zero for grains that are not movable
+    if (P.fuse) {
+      place_node<D>(P, d, in, dp, P.cur_n, P.curf_n, P.rebuild_n, cu);
+    } else {
+      stv<D>(P.force, d, f);  // zero for grains that are not movable
+    }
   }
+  if (P.fuse) grow_box<D>(P.bbox_n, g, act, cu);
 
   if constexpr (REC) {
     record_masks(P, d, act, lane, rent, nrec, wbits);
@@ -644,14 +631,13 @@ __global__ void __launch_bounds__(128) k_force(const Dev P) {
 // host-side launchers
 // ---------------------------------------------------------------------------------------------
 template <int D>
-static void launch_step_t(const Dev& P, const LaunchCfg& L, cudaStream_t s, uint64_t* launches,
-                          cudaEvent_t e0 = nullptr, cudaEvent_t e1 = nullptr, bool rec = false) {
-  const uint32_t nthr_nodes = P.n_chunks * 32;
-  // programmatic dependent launch between the kernels of a step, except where events are
-  // recorded between them (timed mode)
-  const bool pdl = !e0 && !e1;
+static void predict_t(const Dev& P, cudaStream_t s, uint64_t* launches, bool pdl) {
   launch_k(k_predict<D>, cdiv(P.N, 256), 256, 0, s, pdl, P);
   *launches += 1;
+}
+template <int D>
+static void body_t(const Dev& P, const LaunchCfg& L, cudaStream_t s, uint64_t* launches, bool pdl, bool rec,
+                   cudaEvent_t e0, cudaEvent_t e1) {
   launch_grid_build<D>(P, s, launches, pdl);
   if (P.enable_torque) {
     launch_k(k_torque_center<D>, cdiv(P.G, 128), 128, 0, s, pdl, P);
@@ -662,7 +648,7 @@ static void launch_step_t(const Dev& P, const LaunchCfg& L, cudaStream_t s, uint
     launch_k(k_bonds<D>, cdiv(P.n_edges, 256), 256, 0, s, pdl, P);
     *launches += 1;
   }
-  const dim3 grid(cdiv(nthr_nodes, L.force_block)), block(L.force_block);
+  const dim3 grid(cdiv(P.n_chunks * 32, L.force_block)), block(L.force_block);
   if (P.grain_contact) {
     if (rec) launch_k(k_force<D, true, true>, grid, block, 0, s, pdl, P);
     else launch_k(k_force<D, false, true>, grid, block, 0, s, pdl, P);
@@ -670,9 +656,13 @@ static void launch_step_t(const Dev& P, const LaunchCfg& L, cudaStream_t s, uint
     if (rec) launch_k(k_force<D, true, false>, grid, block, 0, s, pdl, P);
     else launch_k(k_force<D, false, false>, grid, block, 0, s, pdl, P);
   }
+  *launches += 1;
   if (e1) cudaEventRecord(e1, s);
+}
+template <int D>
+static void finalize_t(const Dev& P, cudaStream_t s, uint64_t* launches, bool pdl) {
   launch_k(k_finalize<D>, finalize_blocks(P.I), FINAL_THREADS, P.wrec_smem ? FINAL_SMEM : 0, s, pdl, P);
-  *launches += 2;
+  *launches += 1;
 }
 
 cudaError_t kernels_init() {
@@ -689,30 +679,24 @@ cudaError_t kernels_init() {
   return e == cudaSuccess ? ensure_local_bytes(need) : e;
 }
 
-void launch_step(const Dev& P, const LaunchCfg& L, cudaStream_t s, uint64_t* launches, bool rec) {
-  if (P.dim == 2) {
-    launch_step_t<2>(P, L, s, launches, nullptr, nullptr, rec);
-  } else {
-    launch_step_t<3>(P, L, s, launches, nullptr, nullptr, rec);
-  }
+void launch_predict(const Dev& P, cudaStream_t s, uint64_t* launches, bool pdl) {
+  P.dim == 2 ? predict_t<2>(P, s, launches, pdl) : predict_t<3>(P, s, launches, pdl);
 }
-
-void launch_step_timed(const Dev& P, const LaunchCfg& L, cudaStream_t s, uint64_t* launches,
-                       cudaEvent_t e0, cudaEvent_t e1) {
-  if (P.dim == 2) {
-    launch_step_t<2>(P, L, s, launches, e0, e1);
-  } else {
-    launch_step_t<3>(P, L, s, launches, e0, e1);
-  }
+void launch_body(const Dev& P, const LaunchCfg& L, cudaStream_t s, uint64_t* launches, bool pdl, bool rec,
+                 cudaEvent_t e0, cudaEvent_t e1) {
+  P.dim == 2 ? body_t<2>(P, L, s, launches, pdl, rec, e0, e1) : body_t<3>(P, L, s, launches, pdl, rec, e0, e1);
+}
+void launch_finalize(const Dev& P, cudaStream_t s, uint64_t* launches, bool pdl) {
+  P.dim == 2 ? finalize_t<2>(P, s, launches, pdl) : finalize_t<3>(P, s, launches, pdl);
 }
 
 uint32_t grid_coop_blocks(const Dev& P, int device) {
   int per_sm = 0, sms = 0, coop = 0;
   const void* k = P.dim == 2 ? (const void*)k_grid_coop<2> : (const void*)k_grid_coop<3>;
   if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) != cudaSuccess || !coop) return 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, SCAN_THREADS, 0) != cudaSuccess || per_sm < 1) return 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, COOP_THREADS, 0) != cudaSuccess || per_sm < 1) return 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || sms < 1) return 0;
-  const uint32_t want = std::max(cdiv(P.N, SCAN_THREADS), cdiv(P.table_total, SCAN_TILE));
+  const uint32_t want = cdiv(P.N, COOP_THREADS);
   // three blocks per SM: threads enough for the candidate-list phase, few blocks to schedule on
   // the (common) steps without a rebuild and to meet at the grid barriers (same box, collision
   // ensemble: 2 -> 3 blocks 0.0793 -> 0.0780 ms/step at skin 0.25; 4 and 5 blocks were slower

@@ -35,12 +35,15 @@ inline cudaError_t max_local_bytes(const void* const* fs, int n, size_t* out) {
 }
 
 cudaError_t kernels_init();
-// Enqueue one FP64 time step on stream s. Adds the number of kernel launches to *launches. With
-// rec the force kernel also records the step's contact and wall masks (Dev::rec_*).
-void launch_step(const Dev& P, const LaunchCfg& L, cudaStream_t s, uint64_t* launches, bool rec = false);
-// Same as launch_step, with CUDA events e0/e1 recorded around the fused force kernel.
-void launch_step_timed(const Dev& P, const LaunchCfg& L, cudaStream_t s, uint64_t* launches,
-                       cudaEvent_t e0, cudaEvent_t e1);
+// The parts of an FP64 step, each enqueued on stream s: the position update; the grid build and the
+// force kernels; the end of the step. Add the number of kernel launches to *launches. pdl:
+// programmatic dependent launch behind the kernel before. With rec the force kernel also records
+// the step's contact and wall masks (Dev::rec_*); e0/e1 (may be null) are recorded around the force
+// kernels (pdl must be false then).
+void launch_predict(const Dev& P, cudaStream_t s, uint64_t* launches, bool pdl);
+void launch_body(const Dev& P, const LaunchCfg& L, cudaStream_t s, uint64_t* launches, bool pdl, bool rec = false,
+                 cudaEvent_t e0 = nullptr, cudaEvent_t e1 = nullptr);
+void launch_finalize(const Dev& P, cudaStream_t s, uint64_t* launches, bool pdl);
 const void* force_kernel_ptr(uint32_t dim);
 // Blocks of the cooperative grid build (k_grid_coop): every block resident at once (occupancy x
 // SMs), no more than the work needs; 0 when the device has no cooperative launch.

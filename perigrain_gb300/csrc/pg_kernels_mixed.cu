@@ -115,6 +115,60 @@ __device__ __forceinline__ float dotf(const float (&a)[D], const float (&b)[D]) 
   return s;
 }
 
+// CurrPos of node d from its displacement, its FP32 images, and either the list-rebuild check or the
+// node's grid key.
+template <int D>
+__device__ __forceinline__ void place_node_mx(const Dev& P, uint32_t d, const InstDev& in, const double (&dp)[D],
+                                              const double (&ps)[D], const float (&db)[D], double* cur, float* curf,
+                                              float* dref, uint32_t* rebuild, double (&cu)[D]) {
+  float dh[D], dl[D];
+  for (int c = 0; c < D; ++c) split_hl(dp[c], &dh[c], &dl[c]);
+  st_hl<D>(dref, P.np, d, dh, dl);
+  for (int c = 0; c < D; ++c) cu[c] = ps[c] + dp[c];
+  stv<D>(cur, d, cu);
+  // the FP32 position image: offset from the fixed frame with candidate lists, else from this step's
+  // grid origin; formed in FP32 from the truncated CurrPos (integer instructions) -- an FP64
+  // subtraction here would run on the narrow FP64 pipe, and the image only feeds the cell keys and
+  // the FP32 prefilter
+  float rf[D];
+  bool ok = true;
+  for (int c = 0; c < D; ++c) {
+    if (((__double_as_longlong(cu[c]) >> 52) & 0x7ff) == 0x7ff) ok = false;  // inf or NaN
+    double cut;
+    rf[c] = trunc_f32(cu[c], &cut) - in.org_f[c];
+  }
+  if (!ok) set_status(P.status, PG_ENAN);
+  stf<D>(curf, d, rf);
+  if (P.cand_q) {
+    // rebuild once any node has moved 0.45 skin since the last build
+    float m2 = 0.f;
+    for (int c = 0; c < D; ++c) {
+      double dpt;
+      const float dd = trunc_f32(dp[c], &dpt) - db[c];  // truncation (integer ops), not an FP64 conversion
+      m2 += dd * dd;
+    }
+    if (m2 > in.skin_lim2) *rebuild = 1;
+  } else {
+    int32_t ci[3] = {0, 0, 0};
+    for (int c = 0; c < D; ++c) ci[c] = cell_coord(rf[c] + in.frame_off_f[c], in.inv_cell_f, in.dims[c]);
+    const uint32_t key =
+        in.table_off + ((uint32_t)ci[2] * in.dims[1] + (uint32_t)ci[1]) * in.dims[0] + (uint32_t)ci[0];
+    P.cell_key[d] = key;
+    P.cell_rank[d] = atomicAdd(&P.cell_count[key], 1u);
+  }
+}
+
+// disp += dt*v + (dt*dt/2)*a: the increment is formed in FP32 (relative error ~1e-7 of a step's
+// motion); the accumulation into disp stays FP64
+template <int D>
+__device__ __forceinline__ void advance_mx(const Dev& P, const double (&v)[D], const float (&a)[D], double (&dp)[D]) {
+  double vd;
+  for (int c = 0; c < D; ++c) {
+    const float vf = trunc_f32(v[c], &vd);
+    dp[c] = dp[c] + widen(fmaf(P.dt_f, vf, P.hdt2_f * a[c]));
+  }
+}
+
 // ---------------------------------------------------------------------------------------------
 // position update: FP64 disp and CurrPos, plus their FP32 hi/lo images and the grid key
 // ---------------------------------------------------------------------------------------------
@@ -122,117 +176,33 @@ template <int D>
 __global__ void __launch_bounds__(256) k_predict_mx(const Dev P) {
   pdl_enter();
   const uint32_t d = blockIdx.x * blockDim.x + threadIdx.x;
-  const uint32_t lane = threadIdx.x & 31;
   const bool act = d < P.N;
   uint32_t g = 0;
-  unsigned long long kmin[D], kmax[D];
+  double cu[D];
+  for (int c = 0; c < D; ++c) cu[c] = 0.0;
   if (act) {
     // every per-node load is issued before the grain's flags are known, so they overlap
     g = P.node_grain[d];
-    double dp[D], ps[D], cu[D], v[D];
-    float a[D];
+    double dp[D], ps[D], v[D];
+    float a[D], db[D];
     ldv<D>(P.disp, d, dp);
     ldv<D>(P.vel_in, d, v);
     ldvf<D>(P.acc_f, d, a);
     ldv<D>(P.pos, d, ps);
-    constexpr uint32_t SFB = (D == 2) ? 2 : 4;
-    float db[D];
-    for (int c = 0; c < D; ++c) db[c] = P.cand_q ? P.disp_b[(size_t)d * SFB + c] : 0.f;
+    for (int c = 0; c < D; ++c) db[c] = 0.f;
+    if (P.cand_q) ldf<D>(P.disp_b, d, db);
     const bool pend = P.clamp_pending[d] != 0;
     const GrainDev& gr = P.grain[g];
-    bool wrote = false;
+    const bool mov = gr.flags & GF_MOVABLE;
     if (pend) {
       for (int c = 0; c < D; ++c) dp[c] = 0.0;
       P.clamp_pending[d] = 0;
-      wrote = true;
     }
-    if (gr.flags & GF_MOVABLE) {
-      // the increment dt*v + (dt*dt/2)*a is formed in FP32 (relative error ~1e-7 of a step's
-      // motion); the accumulation into disp stays FP64
-      double vd;
-      for (int c = 0; c < D; ++c) {
-        const float vf = trunc_f32(v[c], &vd);
-        dp[c] = dp[c] + widen(fmaf(P.dt_f, vf, P.hdt2_f * a[c]));
-      }
-      wrote = true;
-    }
-    if (wrote) {
-      stv<D>(P.disp, d, dp);
-      float dh[D], dl[D];
-      for (int c = 0; c < D; ++c) split_hl(dp[c], &dh[c], &dl[c]);
-      st_hl<D>(P.dref, P.np, d, dh, dl);
-    }
-    for (int c = 0; c < D; ++c) cu[c] = ps[c] + dp[c];
-    stv<D>(P.cur, d, cu);
-    const InstDev& in = P.inst[gr.inst];
-    // the FP32 position image: offset from the fixed frame with candidate lists (independent of
-    // the grid refit of the step before), else from this step's grid origin; formed in FP32 from
-    // the truncated CurrPos (integer instructions) -- an FP64 subtraction here would run on the
-    // narrow FP64 pipe, and the image only feeds the cell keys and the FP32 prefilter
-    float rf[4] = {0.f, 0.f, 0.f, 0.f};
-    bool ok = true;
-    for (int c = 0; c < D; ++c) {
-      if (((__double_as_longlong(cu[c]) >> 52) & 0x7ff) == 0x7ff) ok = false;  // inf or NaN
-      double cut;
-      rf[c] = trunc_f32(cu[c], &cut) - in.org_f[c];
-    }
-    if (!ok) set_status(P.status, PG_ENAN);
-    if constexpr (D == 2) {
-      reinterpret_cast<float2*>(P.curf)[d] = make_float2(rf[0], rf[1]);
-    } else {
-      reinterpret_cast<float4*>(P.curf)[d] = make_float4(rf[0], rf[1], rf[2], 0.f);
-    }
-    if (P.cand_q) {
-      // candidate lists: keys only on rebuild steps (k_keys); rebuild once any node has moved
-      // 0.45 skin since the last build. Nothing here reads the grid, which the previous step's
-      // finalize may be refitting at the same time.
-      float m2 = 0.f;
-      for (int c = 0; c < D; ++c) {
-        double dpt;
-        const float dd = trunc_f32(dp[c], &dpt) - db[c];  // truncation (integer ops), not an FP64 conversion
-        m2 += dd * dd;
-      }
-      if (m2 > in.skin_lim2) *P.rebuild = 1;
-    } else {
-      int32_t ci[3] = {0, 0, 0};
-      for (int c = 0; c < D; ++c) ci[c] = cell_coord(rf[c] + in.frame_off_f[c], in.inv_cell_f, in.dims[c]);
-      const uint32_t key =
-          in.table_off + ((uint32_t)ci[2] * in.dims[1] + (uint32_t)ci[1]) * in.dims[0] + (uint32_t)ci[0];
-      P.cell_key[d] = key;
-      P.cell_rank[d] = atomicAdd(&P.cell_count[key], 1u);
-    }
-    for (int c = 0; c < D; ++c) {
-      kmin[c] = dbl_to_ordered(cu[c]);
-      kmax[c] = kmin[c];
-    }
-  } else {
-    for (int c = 0; c < D; ++c) {
-      kmin[c] = ~0ull;
-      kmax[c] = 0ull;
-    }
+    if (mov) advance_mx<D>(P, v, a, dp);
+    if (mov || pend) stv<D>(P.disp, d, dp);
+    place_node_mx<D>(P, d, P.inst[gr.inst], dp, ps, db, P.cur, P.curf, P.dref, P.rebuild, cu);
   }
-  const uint32_t full = 0xffffffffu;
-  uint32_t g0 = __shfl_sync(full, g, 0);
-  bool lane0_act = __shfl_sync(full, act ? 1 : 0, 0);
-  if (!lane0_act) return;
-  uint32_t same = __ballot_sync(full, !act || g == g0);
-  if (same == full) {
-    for (int c = 0; c < D; ++c) {
-      kmin[c] = warp_min_u64(kmin[c]);
-      kmax[c] = warp_max_u64(kmax[c]);
-    }
-    if (lane == 0) {
-      for (int c = 0; c < D; ++c) {
-        atomicMin(&P.bbox[(size_t)g0 * 2 * D + c], kmin[c]);
-        atomicMax(&P.bbox[(size_t)g0 * 2 * D + D + c], kmax[c]);
-      }
-    }
-  } else if (act) {
-    for (int c = 0; c < D; ++c) {
-      atomicMin(&P.bbox[(size_t)g * 2 * D + c], kmin[c]);
-      atomicMax(&P.bbox[(size_t)g * 2 * D + D + c], kmax[c]);
-    }
-  }
+  grow_box<D>(P.bbox, g, act, cu);
 }
 
 // One bond: stretch s = (2 xi.eta + eta.eta) / (|xi| (|xi+eta| + |xi|)), force density
@@ -271,6 +241,7 @@ __device__ __forceinline__ uint32_t input_index(const Dev& P, uint32_t i) {
 template <int D, bool REC, bool GC, bool PERM>
 __global__ void __launch_bounds__(128) k_force_mx(const Dev P) {
   pdl_enter();
+  pdl_release();
   const uint32_t d = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t chunk = d >> 5;
@@ -680,7 +651,11 @@ __global__ void __launch_bounds__(128) k_force_mx(const Dev P) {
     }
   }
 
+  // velocity update (timeloop.h:834-863); with P.fuse the next step's position update too
+  double cu[D], dp[D];
+  for (int c = 0; c < D; ++c) cu[c] = 0.0;
   if (act) {
+    if (P.fuse) ldv<D>(P.disp, d, dp);
     if (mov) {
       float ao[D], a[D];
       double v[D];
@@ -699,16 +674,33 @@ __global__ void __launch_bounds__(128) k_force_mx(const Dev P) {
           a[c] = 0.f;
           v[c] = 0.0;
         }
-        P.clamp_pending[d] = 1;
+        if (P.fuse) {
+          for (int c = 0; c < D; ++c) dp[c] = 0.0;
+        } else {
+          P.clamp_pending[d] = 1;
+        }
       }
       if (P.worm) worm_clamp<D>(input_index<PERM>(P, d) - gr.node_begin, worm_phase(t), a, v);
       stvf<D>(P.acc_f, d, a);
       stv<D>(P.vel_out, d, v);
+      if (P.fuse) {
+        advance_mx<D>(P, v, a, dp);
+        stv<D>(P.disp, d, dp);
+      }
     } else {
       stv<D>(P.vel_out, d, vpd);
     }
-    stvf<D>(P.force_f, d, f);
+    if (P.fuse) {
+      double ps[D];
+      float db[D];
+      ldv<D>(P.pos, d, ps);
+      ldf<D>(P.disp_b, d, db);
+      place_node_mx<D>(P, d, in, dp, ps, db, P.cur_n, P.curf_n, P.dref_n, P.rebuild_n, cu);
+    } else {
+      stvf<D>(P.force_f, d, f);
+    }
   }
+  if (P.fuse) grow_box<D>(P.bbox_n, g, act, cu);
 
   if constexpr (REC) {
     record_masks(P, d, act, lane, rent, nrec, wbits);
@@ -751,28 +743,6 @@ static void launch_force_mx(const Dev& P, dim3 grid, dim3 block, cudaStream_t s,
   }
 }
 
-template <int D>
-static void launch_mx(const Dev& P, const LaunchCfg& L, cudaStream_t s, uint64_t* launches, cudaEvent_t e0,
-                      cudaEvent_t e1, bool rec) {
-  const uint32_t nthr = P.n_chunks * 32;
-  // programmatic dependent launch between the kernels of a step, except where events are
-  // recorded between them (timed mode)
-  const bool pdl = !e0 && !e1;
-  launch_k(k_predict_mx<D>, cdiv(P.N, 256), 256, 0, s, pdl, P);
-  *launches += 1;
-  launch_grid_build<D>(P, s, launches, pdl);
-  if (P.enable_torque) {
-    launch_k(k_torque_center<D>, cdiv(P.G, 128), 128, 0, s, pdl, P);
-    *launches += 1;
-  }
-  if (e0) cudaEventRecord(e0, s);
-  const dim3 grid(cdiv(nthr, L.force_block)), block(L.force_block);
-  launch_force_mx<D>(P, grid, block, s, pdl, rec);
-  if (e1) cudaEventRecord(e1, s);
-  launch_k(k_finalize<D>, finalize_blocks(P.I), FINAL_THREADS, P.wrec_smem ? FINAL_SMEM : 0, s, pdl, P);
-  *launches += 2;
-}
-
 cudaError_t kernels_mixed_init() {
   cudaError_t e = cudaFuncSetAttribute(k_finalize<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, FINAL_SMEM);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_finalize<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, FINAL_SMEM);
@@ -792,53 +762,40 @@ cudaError_t kernels_mixed_init() {
   return e == cudaSuccess ? ensure_local_bytes(need) : e;
 }
 
-void launch_step_mixed(const Dev& P, const LaunchCfg& L, cudaStream_t s, uint64_t* launches, cudaEvent_t e0,
-                       cudaEvent_t e1, bool rec) {
-  if (P.dim == 2) {
-    launch_mx<2>(P, L, s, launches, e0, e1, rec);
-  } else {
-    launch_mx<3>(P, L, s, launches, e0, e1, rec);
-  }
-}
-
-void launch_mixed_predict(const Dev& P, cudaStream_t s, bool pdl, uint64_t* launches) {
-  if (P.dim == 2) {
-    launch_k(k_predict_mx<2>, cdiv(P.N, 256), 256, 0, s, pdl, P);
-  } else {
-    launch_k(k_predict_mx<3>, cdiv(P.N, 256), 256, 0, s, pdl, P);
-  }
+template <int D>
+static void predict_t(const Dev& P, cudaStream_t s, uint64_t* launches, bool pdl) {
+  launch_k(k_predict_mx<D>, cdiv(P.N, 256), 256, 0, s, pdl, P);
   *launches += 1;
 }
-
 template <int D>
-static void launch_mx_body(const Dev& P, const LaunchCfg& L, cudaStream_t s, bool pdl, uint64_t* launches,
-                           bool rec) {
+static void body_t(const Dev& P, const LaunchCfg& L, cudaStream_t s, uint64_t* launches, bool pdl, bool rec,
+                   cudaEvent_t e0, cudaEvent_t e1) {
   launch_grid_build<D>(P, s, launches, pdl);
   if (P.enable_torque) {
     launch_k(k_torque_center<D>, cdiv(P.G, 128), 128, 0, s, pdl, P);
     *launches += 1;
   }
+  if (e0) cudaEventRecord(e0, s);
   const dim3 grid(cdiv(P.n_chunks * 32, L.force_block)), block(L.force_block);
   launch_force_mx<D>(P, grid, block, s, pdl, rec);
   *launches += 1;
+  if (e1) cudaEventRecord(e1, s);
 }
-
-void launch_mixed_body(const Dev& P, const LaunchCfg& L, cudaStream_t s, bool pdl, uint64_t* launches, bool rec) {
-  if (P.dim == 2) {
-    launch_mx_body<2>(P, L, s, pdl, launches, rec);
-  } else {
-    launch_mx_body<3>(P, L, s, pdl, launches, rec);
-  }
-}
-
-void launch_mixed_finalize(const Dev& P, cudaStream_t s, bool pdl, uint64_t* launches) {
-  const uint32_t sm = P.wrec_smem ? FINAL_SMEM : 0;
-  if (P.dim == 2) {
-    launch_k(k_finalize<2>, finalize_blocks(P.I), FINAL_THREADS, sm, s, pdl, P);
-  } else {
-    launch_k(k_finalize<3>, finalize_blocks(P.I), FINAL_THREADS, sm, s, pdl, P);
-  }
+template <int D>
+static void finalize_t(const Dev& P, cudaStream_t s, uint64_t* launches, bool pdl) {
+  launch_k(k_finalize<D>, finalize_blocks(P.I), FINAL_THREADS, P.wrec_smem ? FINAL_SMEM : 0, s, pdl, P);
   *launches += 1;
+}
+
+void launch_mixed_predict(const Dev& P, cudaStream_t s, uint64_t* launches, bool pdl) {
+  P.dim == 2 ? predict_t<2>(P, s, launches, pdl) : predict_t<3>(P, s, launches, pdl);
+}
+void launch_mixed_body(const Dev& P, const LaunchCfg& L, cudaStream_t s, uint64_t* launches, bool pdl, bool rec,
+                       cudaEvent_t e0, cudaEvent_t e1) {
+  P.dim == 2 ? body_t<2>(P, L, s, launches, pdl, rec, e0, e1) : body_t<3>(P, L, s, launches, pdl, rec, e0, e1);
+}
+void launch_mixed_finalize(const Dev& P, cudaStream_t s, uint64_t* launches, bool pdl) {
+  P.dim == 2 ? finalize_t<2>(P, s, launches, pdl) : finalize_t<3>(P, s, launches, pdl);
 }
 
 }  // namespace pg

@@ -90,7 +90,8 @@ extern "C" int pg_postprocess(pg_handle* h, const pg_post* out) {
   if (!h || !out) return pg_fail(PG_EINVAL, "null argument");
   int rc = pg_synchronize(h);
   if (rc) return rc;
-  const Dev& P = h->P;
+  Dev P = h->P;
+  P.cur = h->cur();
   const uint32_t D = h->dim, G = P.G, I = P.I, N = P.N, NS = 2 * D;
   const int NQ = (D == 2) ? post_nq<2>() : post_nq<3>();
   if (!h->post_sum) CU(h->dalloc(&h->post_sum, (size_t)G * NQ));

@@ -150,7 +150,7 @@ int pg_snapshot(pg_handle* h, const pg_snapshot_desc* d) {
   auto add = [&](double* dst, const void* src, bool f32) {
     if (dst) req[nf++] = {dst, src, f32};
   };
-  add(d->currpos, h->P.cur, false);
+  add(d->currpos, h->cur(), false);
   add(d->vel, h->vel_parity == 0 ? h->vel_a : h->vel_b, false);
   add(d->acc, mixed ? (const void*)h->P.acc_f : (const void*)h->P.acc, mixed);
   add(d->force, mixed ? (const void*)h->P.force_f : (const void*)h->P.force, mixed);
