@@ -154,6 +154,7 @@ struct WallRec {
 struct Dev {
   uint32_t dim, N, G, I;
   uint32_t n_chunks;
+  uint32_t n_sms;  // multiprocessors of the device
   uint32_t table_total;
   // node arrays
   double *xpos, *pos, *disp, *cur, *vel_in, *vel_out, *acc, *force, *extf, *vol;

@@ -652,6 +652,11 @@ static int create_impl(const pg_setup_desc* s, const pg_config* cfg_in, pg_handl
   P.G = G;
   P.I = I;
   P.n_chunks = (N + 31) / 32;
+  {
+    int sms = 0;
+    CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
+    P.n_sms = (uint32_t)std::max(1, sms);
+  }
   P.dt = cfg.dt;
   P.hdt2 = (cfg.dt * cfg.dt) * 0.5;
   P.half_dt = 0.5 * cfg.dt;

@@ -232,8 +232,8 @@ __global__ void __launch_bounds__(256) k_bonds(const Dev P) {
   }
 }
 
-template <int D, bool REC, bool GC>
-__global__ void __launch_bounds__(128) k_force(const Dev P) {
+template <int D, bool REC, bool GC, bool LIST, int BPS>
+__global__ void __launch_bounds__(128, BPS) k_force(const Dev P) {
   pdl_enter();
   pdl_release();
   const uint32_t d = blockIdx.x * blockDim.x + threadIdx.x;
@@ -278,65 +278,90 @@ __global__ void __launch_bounds__(128) k_force(const Dev P) {
 
   // ---- node-node contact: self-contact first, then grains j ascending (timeloop.h:709-747) ----
   // with candidate lists a node whose list is empty has no contact this step
-  const uint32_t ncl = (P.cand_q && act) ? (uint32_t)P.cand_n[d] : 0u;
-  if ((selfc || other) && p_bdry && (!P.cand_q || ncl > 0)) {
+  const uint32_t ncl = (LIST && act) ? (uint32_t)P.cand_n[d] : 0u;
+  if ((selfc || other) && p_bdry && (!LIST || ncl > 0)) {
     double bmn[D], bmx[D];
     grain_box<D>(P, g, bmn, bmx);
     float pf[D];
     ldf<D>(P.curf, d, pf);
-    int32_t cc[3] = {0, 0, 0};
-    for (int c = 0; c < D; ++c) cc[c] = cell_coord(pf[c] + in.frame_off_f[c], in.inv_cell_f, in.dims[c]);
     const float thr2 = in.pre_f * in.pre_f;
-    unsigned long long keys[MAX_CAND];
-    uint32_t idx[MAX_CAND];
-    int nc = 0;
-    // one candidate q of node d: the FP32 prefilter, the contact rules and the grain-box test,
-    // then insertion in the reference's visit order
-    auto consider = [&](uint32_t q) {
+    // does candidate q pass the FP32 prefilter, the contact rules and the grain-box test? (the box
+    // test of the grain asked about last is kept: a list is sorted by grain)
+    uint32_t box_g = NONE;
+    bool box_ok = false;
+    auto passes = [&](uint32_t q) {
       float qf[D];
       ldf<D>(P.curf, q, qf);
+      const uint32_t gq = P.node_grain[q];  // issued with the position, used after the prefilter
       float d2 = 0.f;
       for (int c = 0; c < D; ++c) {
         float dd = qf[c] - pf[c];
         d2 += dd * dd;
       }
-      if (d2 > thr2) return;
-      const uint32_t gq = P.node_grain[q];
+      if (d2 > thr2) return false;
       const bool same = (gq == g);
-      if (same ? !selfc : !other) return;
-      if (P.nl_bdry_only && P.bdry_rank[q] == NONE) return;
-      if (!same) {
+      if (same ? !selfc : !other) return false;
+      if (P.nl_bdry_only && P.bdry_rank[q] == NONE) return false;
+      if (same) return true;
+      if (gq != box_g) {
         double qmn[D], qmx[D];
         grain_box<D>(P, gq, qmn, qmx);
-        if (!boxes_touch<D>(bmn, bmx, qmn, qmx, in.contact_rad)) return;
+        box_g = gq;
+        box_ok = boxes_touch<D>(bmn, bmx, qmn, qmx, in.contact_rad);
       }
-      const uint32_t sub = P.node_sub[q];
-      const unsigned long long key =
-          ((unsigned long long)(same ? 0u : 1u) << 63) | ((unsigned long long)gq << 32) | sub;
-      insert_cand<D>(keys, idx, nc, key, q, P);
+      return box_ok;
     };
-    if (P.cand_q) {
-      // candidate list of the last rebuild (a superset of the grid search's candidates)
-      const size_t cbase = (size_t)chunk * P.cand_cap * 32 + lane;
-      for (uint32_t k = 0; k < ncl; ++k) consider(P.cand_q[cbase + (size_t)k * 32]);
-    } else {
-    const int z0 = (D == 3) ? max(cc[2] - 1, 0) : 0, z1 = (D == 3) ? min(cc[2] + 1, (int)in.dims[2] - 1) : 0;
-    const int y0 = max(cc[1] - 1, 0), y1 = min(cc[1] + 1, (int)in.dims[1] - 1);
-    const int x0 = max(cc[0] - 1, 0), x1 = min(cc[0] + 1, (int)in.dims[0] - 1);
-    for (int z = z0; z <= z1; ++z)
-      for (int y = y0; y <= y1; ++y) {
-        const uint32_t row = in.table_off + ((uint32_t)z * in.dims[1] + (uint32_t)y) * in.dims[0];
-        const uint32_t b0 = P.cell_start[row + x0], b1 = P.cell_start[row + x1 + 1];
-        for (uint32_t b = b0; b < b1; ++b) {
-          const uint32_t q = P.sorted[b];
-          if (q != d) consider(q);
+    // the contacts of this step in the reference's visit order: with candidate lists (LIST) a bit per
+    // entry of the list, which is in that order; else the grid search's nodes sorted by key
+    const size_t cbase = (size_t)chunk * P.cand_cap * 32 + lane;
+    uint32_t hits = 0;
+    uint32_t idx[LIST ? 1 : MAX_CAND];
+    int nc = 0;
+    if constexpr (LIST) {
+      uint32_t qn = P.cand_q[cbase];  // the next entry is loaded one candidate ahead
+      for (uint32_t k = 0; k < ncl; ++k) {
+        const uint32_t q = qn;
+        if (k + 1 < ncl) qn = P.cand_q[cbase + (size_t)(k + 1) * 32];
+        if (!passes(q)) continue;
+        if (nc >= (int)P.max_cand) {
+          set_status(P.status, PG_ECAPACITY);
+          break;
         }
+        hits |= 1u << k;
+        ++nc;
       }
+    } else {
+      unsigned long long keys[MAX_CAND];
+      int32_t cc[3] = {0, 0, 0};
+      for (int c = 0; c < D; ++c) cc[c] = cell_coord(pf[c] + in.frame_off_f[c], in.inv_cell_f, in.dims[c]);
+      const int z0 = (D == 3) ? max(cc[2] - 1, 0) : 0, z1 = (D == 3) ? min(cc[2] + 1, (int)in.dims[2] - 1) : 0;
+      const int y0 = max(cc[1] - 1, 0), y1 = min(cc[1] + 1, (int)in.dims[1] - 1);
+      const int x0 = max(cc[0] - 1, 0), x1 = min(cc[0] + 1, (int)in.dims[0] - 1);
+      for (int z = z0; z <= z1; ++z)
+        for (int y = y0; y <= y1; ++y) {
+          const uint32_t row = in.table_off + ((uint32_t)z * in.dims[1] + (uint32_t)y) * in.dims[0];
+          const uint32_t b0 = P.cell_start[row + x0], b1 = P.cell_start[row + x1 + 1];
+          for (uint32_t b = b0; b < b1; ++b) {
+            const uint32_t q = P.sorted[b];
+            if (q == d || !passes(q)) continue;
+            const uint32_t gq = P.node_grain[q];
+            const unsigned long long key =
+                ((unsigned long long)(gq == g ? 0u : 1u) << 63) | ((unsigned long long)gq << 32) | P.node_sub[q];
+            insert_cand<D>(keys, idx, nc, key, q, P);
+          }
+        }
     }
     const uint32_t mydeg = P.node_deg[d];
     for (int ci = 0; ci < nc; ++ci) {
-      const uint32_t q = idx[ci];
-      const bool same = (keys[ci] >> 63) == 0;
+      uint32_t q;
+      if constexpr (LIST) {
+        q = P.cand_q[cbase + (size_t)(__ffs(hits) - 1) * 32];
+        hits &= hits - 1;
+      } else {
+        q = idx[ci];
+      }
+      const uint32_t gqi = P.node_grain[q];
+      const bool same = gqi == g;
       double xq[D], dir[D];
       ldv<D>(P.cur, q, xq);
       for (int c = 0; c < D; ++c) dir[c] = xq[c] - xpc[c];
@@ -349,7 +374,7 @@ __global__ void __launch_bounds__(128) k_force(const Dev P) {
       double Rc = in.contact_rad, Kn = in.normal_stiffness;
       double zeta = in.damping_ratio, mu = in.friction_coefficient;
       if constexpr (GC) {
-        const GrainDev& gq = P.grain[(uint32_t)(keys[ci] >> 32) & 0x7fffffffu];
+        const GrainDev& gq = P.grain[gqi];
         Kn = (gr.kn + gq.kn) * 0.5;
         zeta = (gr.zeta + gq.zeta) * 0.5;
         mu = (gr.mu + gq.mu) * 0.5;
@@ -630,6 +655,21 @@ __global__ void __launch_bounds__(128) k_force(const Dev P) {
 // ---------------------------------------------------------------------------------------------
 // host-side launchers
 // ---------------------------------------------------------------------------------------------
+// The force kernel's variants: mask recording (REC), per-grain contact parameters (GC), candidate
+// lists or the grid search (LIST); the plain kernel with lists for 5 or 7 blocks of 128 threads per
+// SM (96 or 72 registers): the latency of its own chain counts where the chunks do not fill the GPU
+// (two disks: 20.5 us a step at 5 blocks, 21.1 at 7), occupancy where they do (3D spheres 366 and 359).
+template <int D>
+static const void* force_ptr(bool rec, bool gc, bool list, int bps) {
+  static const void* const fs[8] = {
+      (const void*)k_force<D, false, false, false, 6>, (const void*)k_force<D, false, false, true, 5>,
+      (const void*)k_force<D, false, true, false, 5>,  (const void*)k_force<D, false, true, true, 5>,
+      (const void*)k_force<D, true, false, false, 5>,  (const void*)k_force<D, true, false, true, 5>,
+      (const void*)k_force<D, true, true, false, 5>,   (const void*)k_force<D, true, true, true, 5>};
+  if (!rec && !gc && list && bps > 5) return (const void*)k_force<D, false, false, true, 7>;
+  return fs[(rec ? 4 : 0) | (gc ? 2 : 0) | (list ? 1 : 0)];
+}
+
 template <int D>
 static void predict_t(const Dev& P, cudaStream_t s, uint64_t* launches, bool pdl) {
   launch_k(k_predict<D>, cdiv(P.N, 256), 256, 0, s, pdl, P);
@@ -649,13 +689,8 @@ static void body_t(const Dev& P, const LaunchCfg& L, cudaStream_t s, uint64_t* l
     *launches += 1;
   }
   const dim3 grid(cdiv(P.n_chunks * 32, L.force_block)), block(L.force_block);
-  if (P.grain_contact) {
-    if (rec) launch_k(k_force<D, true, true>, grid, block, 0, s, pdl, P);
-    else launch_k(k_force<D, false, true>, grid, block, 0, s, pdl, P);
-  } else {
-    if (rec) launch_k(k_force<D, true, false>, grid, block, 0, s, pdl, P);
-    else launch_k(k_force<D, false, false>, grid, block, 0, s, pdl, P);
-  }
+  using K = void (*)(const Dev);
+  launch_k((K)force_ptr<D>(rec, P.grain_contact, P.cand_q, force_bps(P.n_chunks, P.n_sms)), grid, block, 0, s, pdl, P);
   *launches += 1;
   if (e1) cudaEventRecord(e1, s);
 }
@@ -670,12 +705,15 @@ cudaError_t kernels_init() {
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_finalize<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, FINAL_SMEM);
   if (e != cudaSuccess) return e;
   // the recording variants of the force kernel have local frames of about 1.1 KB
-  const void* fs[] = {(const void*)k_force<2, false, false>, (const void*)k_force<2, false, true>,
-                      (const void*)k_force<2, true, false>,  (const void*)k_force<2, true, true>,
-                      (const void*)k_force<3, false, false>, (const void*)k_force<3, false, true>,
-                      (const void*)k_force<3, true, false>,  (const void*)k_force<3, true, true>};
+  const void* fs[32];
+  int n = 0;
+  for (int k = 0; k < 8; ++k)
+    for (int b = 5; b <= 7; b += 2) {
+      fs[n++] = force_ptr<2>(k & 4, k & 2, k & 1, b);
+      fs[n++] = force_ptr<3>(k & 4, k & 2, k & 1, b);
+    }
   size_t need = 0;
-  e = max_local_bytes(fs, 8, &need);
+  e = max_local_bytes(fs, n, &need);
   return e == cudaSuccess ? ensure_local_bytes(need) : e;
 }
 
@@ -702,10 +740,6 @@ uint32_t grid_coop_blocks(const Dev& P, int device) {
   // ensemble: 2 -> 3 blocks 0.0793 -> 0.0780 ms/step at skin 0.25; 4 and 5 blocks were slower
   // than 3, other workloads unchanged)
   return std::max(1u, std::min((uint32_t)(std::min(per_sm, 3) * sms), want));
-}
-
-const void* force_kernel_ptr(uint32_t dim) {
-  return dim == 2 ? (const void*)k_force<2, false, false> : (const void*)k_force<3, false, false>;
 }
 
 // ---------------------------------------------------------------------------------------------

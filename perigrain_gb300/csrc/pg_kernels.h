@@ -34,6 +34,25 @@ inline cudaError_t max_local_bytes(const void* const* fs, int n, size_t* out) {
   return cudaSuccess;
 }
 
+// Blocks of 128 threads per SM the force kernels are compiled for that suit a handle of n_chunks
+// warps: a warp holds its slot for its whole chunk, so the time goes as the number of rounds of
+// resident warps times the warps that share an SM in each, rounds * bps; the smallest product wins,
+// the larger register budget on a tie. Mixed, us a step at 5 / 6 / 7 blocks: collision ensemble (80
+// warps an SM) 70 / 71 / 62, 3D spheres (26) 87 / 110 / 86, settling (24) 20.7 / 17.9 / 19.0, two
+// disks (1) 12.5 / 13.9 / 14.0.
+inline int force_bps(uint32_t n_chunks, uint32_t sms) {
+  int best = 5;
+  uint64_t best_cost = ~0ull;
+  for (int b = 5; b <= 7; ++b) {
+    const uint64_t slots = (uint64_t)sms * 4 * b, cost = (n_chunks + slots - 1) / slots * b;
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = b;
+    }
+  }
+  return best;
+}
+
 cudaError_t kernels_init();
 // The parts of an FP64 step, each enqueued on stream s: the position update; the grid build and the
 // force kernels; the end of the step. Add the number of kernel launches to *launches. pdl:
@@ -44,7 +63,6 @@ void launch_predict(const Dev& P, cudaStream_t s, uint64_t* launches, bool pdl);
 void launch_body(const Dev& P, const LaunchCfg& L, cudaStream_t s, uint64_t* launches, bool pdl, bool rec = false,
                  cudaEvent_t e0 = nullptr, cudaEvent_t e1 = nullptr);
 void launch_finalize(const Dev& P, cudaStream_t s, uint64_t* launches, bool pdl);
-const void* force_kernel_ptr(uint32_t dim);
 // Blocks of the cooperative grid build (k_grid_coop): every block resident at once (occupancy x
 // SMs), no more than the work needs; 0 when the device has no cooperative launch.
 uint32_t grid_coop_blocks(const Dev& P, int device);

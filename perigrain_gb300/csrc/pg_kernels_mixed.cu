@@ -238,8 +238,8 @@ __device__ __forceinline__ uint32_t input_index(const Dev& P, uint32_t i) {
   return i;
 }
 
-template <int D, bool REC, bool GC, bool PERM>
-__global__ void __launch_bounds__(128) k_force_mx(const Dev P) {
+template <int D, bool REC, bool GC, bool PERM, bool LIST, int BPS>
+__global__ void __launch_bounds__(128, BPS) k_force_mx(const Dev P) {
   pdl_enter();
   pdl_release();
   const uint32_t d = blockIdx.x * blockDim.x + threadIdx.x;
@@ -285,33 +285,37 @@ __global__ void __launch_bounds__(128) k_force_mx(const Dev P) {
     if constexpr (REC) {
       if (mov && P.rec_df) st_hl<D>(P.rec_df, P.np, d, dh, dl);
     }
-    // the alive words and neighbour indices of the next pair are loaded one iteration ahead, so
-    // only the neighbour gathers wait on memory in each iteration. A lane past the last node (d >= N
-    // in the last chunk) gathers its own index for bonds it never uses: dref, xref and vol_f are allocated
-    // in whole chunks (zero padding), so those reads stay inside the arrays.
-    uint32_t wa_n = 0u, wb_n = 0u, ca_n = d, cb_n = d;
-    if (cdeg > 0) {
-      wa_n = P.alive[w0];
-      ca_n = P.bcol[slot0];
-    }
-    if (cdeg > 1) {
-      wb_n = P.alive[w0 + 1];
-      cb_n = P.bcol[slot0 + 32u];
-    }
+    // The alive words and neighbour indices are loaded two pairs ahead (they stream from memory, the
+    // longest latency of the loop; one pair ahead took the collision ensemble's step from 59.6 to
+    // 62.3 us and the 3D spheres' from 81.4 to 85.4), so only the neighbour gathers wait in an
+    // iteration. A lane past the last node (d >= N in the last chunk) gathers its own index for bonds
+    // it never uses: dref, xref and vol_f are allocated in whole chunks (zero padding), so those
+    // reads stay inside the arrays.
+    auto ahead = [&](uint32_t k, uint32_t& w, uint32_t& c) {
+      w = 0u;
+      c = d;
+      if (k < cdeg) {
+        w = P.alive[w0 + k];
+        c = P.bcol[slot0 + 32u * k];
+      }
+    };
+    uint32_t wa_n, wb_n, ca_n, cb_n, wa_m, wb_m, ca_m, cb_m;
+    ahead(0, wa_n, ca_n);
+    ahead(1, wb_n, cb_n);
+    ahead(2, wa_m, ca_m);
+    ahead(3, wb_m, cb_m);
     for (uint32_t k = 0; k < cdeg; k += 2) {
       const bool two = (k + 1) < cdeg;
       const uint32_t wa = wa_n, wb = wb_n, ca = ca_n, cb = cb_n;
-      if (k + 2 < cdeg) {
-        wa_n = P.alive[w0 + k + 2];
-        ca_n = P.bcol[slot0 + 32u * (k + 2)];
+      wa_n = wa_m;
+      wb_n = wb_m;
+      ca_n = ca_m;
+      cb_n = cb_m;
+      if (k + 4 < cdeg) {
+        wa_m = P.alive[w0 + k + 4];
+        ca_m = P.bcol[slot0 + 32u * (k + 4)];
       }
-      if (k + 3 < cdeg) {
-        wb_n = P.alive[w0 + k + 3];
-        cb_n = P.bcol[slot0 + 32u * (k + 3)];
-      } else {
-        wb_n = 0u;
-        cb_n = d;
-      }
+      ahead(k + 5, wb_m, cb_m);
       bool ba = (wa >> lane) & 1u, bb = (wb >> lane) & 1u;
       const bool ua = mov && ba, ub = mov && bb;
       const uint32_t sa = slot0 + 32u * k, sb = sa + 32u;
@@ -359,21 +363,18 @@ __global__ void __launch_bounds__(128) k_force_mx(const Dev P) {
   const bool other = mov && (P.worm || (gr.flags & GF_STOPPABLE));
 
   // with candidate lists a node whose list is empty has no contact this step
-  const uint32_t ncl = (P.cand_q && act) ? (uint32_t)P.cand_n[d] : 0u;
-  if ((selfc || other) && p_bdry && (!P.cand_q || ncl > 0)) {
+  const uint32_t ncl = (LIST && act) ? (uint32_t)P.cand_n[d] : 0u;
+  if ((selfc || other) && p_bdry && (!LIST || ncl > 0)) {
     double bmn[D], bmx[D];
     grain_box<D>(P, g, bmn, bmx);
     float ph[D];
     ldf<D>(P.curf, d, ph);
-    int32_t cc[3] = {0, 0, 0};
-    for (int c = 0; c < D; ++c) cc[c] = cell_coord(ph[c] + in.frame_off_f[c], in.inv_cell_f, in.dims[c]);
     const float thr2 = in.pre_f * in.pre_f;
-    unsigned long long keys[MAX_CAND];
-    uint32_t idx[MAX_CAND];
-    int nc = 0;
-    // one candidate q of node d: the FP32 prefilter, the contact rules and the grain-box test,
-    // then insertion in the reference's visit order
-    auto consider = [&](uint32_t q) {
+    // does candidate q pass the FP32 prefilter, the contact rules and the grain-box test? (the box
+    // test of the grain asked about last is kept: a list is sorted by grain)
+    uint32_t box_g = NONE;
+    bool box_ok = false;
+    auto passes = [&](uint32_t q) {
       float qf[D];
       ldf<D>(P.curf, q, qf);
       const uint32_t gq = P.node_grain[q];  // issued with the position, used after the prefilter
@@ -382,42 +383,58 @@ __global__ void __launch_bounds__(128) k_force_mx(const Dev P) {
         float dd = qf[c] - ph[c];
         d2 = fmaf(dd, dd, d2);
       }
-      if (d2 > thr2) return;
+      if (d2 > thr2) return false;
       const bool same = (gq == g);
-      if (same ? !selfc : !other) return;
-      if (P.nl_bdry_only && P.bdry_rank[q] == NONE) return;
-      if (!same) {
+      if (same ? !selfc : !other) return false;
+      if (P.nl_bdry_only && P.bdry_rank[q] == NONE) return false;
+      if (same) return true;
+      if (gq != box_g) {
         double qmn[D], qmx[D];
         grain_box<D>(P, gq, qmn, qmx);
-        if (!boxes_touch<D>(bmn, bmx, qmn, qmx, in.contact_rad)) return;
+        box_g = gq;
+        box_ok = boxes_touch<D>(bmn, bmx, qmn, qmx, in.contact_rad);
       }
-      const uint32_t sub = P.node_sub[q];
-      const unsigned long long key =
-          ((unsigned long long)(same ? 0u : 1u) << 63) | ((unsigned long long)gq << 32) | sub;
-      insert_cand<D>(keys, idx, nc, key, q, P);
+      return box_ok;
     };
-    if (P.cand_q) {
-      // candidate list of the last rebuild (a superset of the grid search's candidates)
-      const size_t cbase = (size_t)chunk * P.cand_cap * 32 + lane;
-      uint32_t qn = ncl ? P.cand_q[cbase] : d;  // the next entry is loaded one candidate ahead
+    // the contacts of this step in the reference's visit order: with candidate lists (LIST) a bit per
+    // entry of the list, which is in that order; else the grid search's nodes sorted by key
+    const size_t cbase = (size_t)chunk * P.cand_cap * 32 + lane;
+    uint32_t hits = 0;
+    uint32_t idx[LIST ? 1 : MAX_CAND];
+    int nc = 0;
+    if constexpr (LIST) {
+      uint32_t qn = P.cand_q[cbase];  // the next entry is loaded one candidate ahead
       for (uint32_t k = 0; k < ncl; ++k) {
         const uint32_t q = qn;
         if (k + 1 < ncl) qn = P.cand_q[cbase + (size_t)(k + 1) * 32];
-        consider(q);
+        if (!passes(q)) continue;
+        if (nc >= (int)P.max_cand) {
+          set_status(P.status, PG_ECAPACITY);
+          break;
+        }
+        hits |= 1u << k;
+        ++nc;
       }
     } else {
-    const int z0 = (D == 3) ? max(cc[2] - 1, 0) : 0, z1 = (D == 3) ? min(cc[2] + 1, (int)in.dims[2] - 1) : 0;
-    const int y0 = max(cc[1] - 1, 0), y1 = min(cc[1] + 1, (int)in.dims[1] - 1);
-    const int x0 = max(cc[0] - 1, 0), x1 = min(cc[0] + 1, (int)in.dims[0] - 1);
-    for (int z = z0; z <= z1; ++z)
-      for (int y = y0; y <= y1; ++y) {
-        const uint32_t row = in.table_off + ((uint32_t)z * in.dims[1] + (uint32_t)y) * in.dims[0];
-        const uint32_t b0 = P.cell_start[row + x0], b1 = P.cell_start[row + x1 + 1];
-        for (uint32_t b = b0; b < b1; ++b) {
-          const uint32_t q = P.sorted[b];
-          if (q != d) consider(q);
+      unsigned long long keys[MAX_CAND];
+      int32_t cc[3] = {0, 0, 0};
+      for (int c = 0; c < D; ++c) cc[c] = cell_coord(ph[c] + in.frame_off_f[c], in.inv_cell_f, in.dims[c]);
+      const int z0 = (D == 3) ? max(cc[2] - 1, 0) : 0, z1 = (D == 3) ? min(cc[2] + 1, (int)in.dims[2] - 1) : 0;
+      const int y0 = max(cc[1] - 1, 0), y1 = min(cc[1] + 1, (int)in.dims[1] - 1);
+      const int x0 = max(cc[0] - 1, 0), x1 = min(cc[0] + 1, (int)in.dims[0] - 1);
+      for (int z = z0; z <= z1; ++z)
+        for (int y = y0; y <= y1; ++y) {
+          const uint32_t row = in.table_off + ((uint32_t)z * in.dims[1] + (uint32_t)y) * in.dims[0];
+          const uint32_t b0 = P.cell_start[row + x0], b1 = P.cell_start[row + x1 + 1];
+          for (uint32_t b = b0; b < b1; ++b) {
+            const uint32_t q = P.sorted[b];
+            if (q == d || !passes(q)) continue;
+            const uint32_t gq = P.node_grain[q];
+            const unsigned long long key =
+                ((unsigned long long)(gq == g ? 0u : 1u) << 63) | ((unsigned long long)gq << 32) | P.node_sub[q];
+            insert_cand<D>(keys, idx, nc, key, q, P);
+          }
         }
-      }
     }
     const uint32_t mydeg = P.node_deg[d];
     // the pair log hashes input indices (the node's own looked up once; recorded runs only)
@@ -428,8 +445,15 @@ __global__ void __launch_bounds__(128) k_force_mx(const Dev P) {
     double xp64[D];
     if (nc) ldv<D>(P.cur, d, xp64);
     for (int ci = 0; ci < nc; ++ci) {
-      const uint32_t q = idx[ci];
-      const bool same = (keys[ci] >> 63) == 0;
+      uint32_t q;
+      if constexpr (LIST) {
+        q = P.cand_q[cbase + (size_t)(__ffs(hits) - 1) * 32];
+        hits &= hits - 1;
+      } else {
+        q = idx[ci];
+      }
+      const uint32_t gqi = P.node_grain[q];
+      const bool same = gqi == g;
       // The contact decision |x_q - x_p| <= R_c' is made with the reference's FP64 arithmetic:
       // contact damping switches on at full strength at that boundary, so a decision flipped by
       // FP32 rounding would kick a node by metres per second.
@@ -445,7 +469,7 @@ __global__ void __launch_bounds__(128) k_force_mx(const Dev P) {
       double Rc64 = in.contact_rad;
       float Kn = Kn0, zeta = zeta0, mu = mu0;
       if constexpr (GC) {
-        const GrainDev& gq = P.grain[(uint32_t)(keys[ci] >> 32) & 0x7fffffffu];
+        const GrainDev& gq = P.grain[gqi];
         Kn = (float)((gr.kn + gq.kn) * 0.5);
         zeta = (float)((gr.zeta + gq.zeta) * 0.5);
         mu = (float)((gr.mu + gq.mu) * 0.5);
@@ -724,23 +748,28 @@ __global__ void __launch_bounds__(128) k_force_mx(const Dev P) {
   if (my_close) atomicAdd(P.too_close, my_close);
 }
 
-// The force kernel's variants: mask recording (REC), per-grain contact parameters (GC) and a node
-// layout other than the input order (PERM) are compiled in only where used, so the plain kernel
-// keeps its register budget.
+// The force kernel's variants: mask recording (REC), per-grain contact parameters (GC), a node
+// layout other than the input order (PERM) and candidate lists or the grid search (LIST) are compiled
+// in only where used, so the plain kernel keeps its register budget; the plain kernel with lists
+// also for BPS = 5, 6 or 7 blocks of 128 threads per SM (96, 80 or 72 registers), see force_bps().
+template <int D>
+static const void* force_mx_ptr(bool rec, bool gc, bool perm, bool list, int bps) {
+#define PG_F(r, g, p, l, b) (const void*)k_force_mx<D, r, g, p, l, b>
+  static const void* const plain[2][3] = {{PG_F(0, 0, 0, 1, 5), PG_F(0, 0, 0, 1, 6), PG_F(0, 0, 0, 1, 7)},
+                                          {PG_F(0, 0, 1, 1, 5), PG_F(0, 0, 1, 1, 6), PG_F(0, 0, 1, 1, 7)}};
+  static const void* const others[14] = {
+      PG_F(0, 0, 0, 0, 6), PG_F(0, 0, 1, 0, 6), PG_F(0, 1, 0, 0, 5), PG_F(0, 1, 0, 1, 5), PG_F(0, 1, 1, 0, 5),
+      PG_F(0, 1, 1, 1, 5), PG_F(1, 0, 0, 0, 5), PG_F(1, 0, 0, 1, 5), PG_F(1, 0, 1, 0, 5), PG_F(1, 0, 1, 1, 5),
+      PG_F(1, 1, 0, 0, 5), PG_F(1, 1, 0, 1, 5), PG_F(1, 1, 1, 0, 5), PG_F(1, 1, 1, 1, 5)};
+#undef PG_F
+  if (!rec && !gc) return list ? plain[perm ? 1 : 0][bps - 5] : others[perm ? 1 : 0];
+  return others[2 + (rec ? (gc ? 8 : 4) : 0) + (perm ? 2 : 0) + (list ? 1 : 0)];
+}
 template <int D>
 static void launch_force_mx(const Dev& P, dim3 grid, dim3 block, cudaStream_t s, bool pdl, bool rec) {
-  const bool perm = P.node_orig != nullptr;
-  if (P.grain_contact) {
-    if (rec) perm ? launch_k(k_force_mx<D, true, true, true>, grid, block, 0, s, pdl, P)
-                  : launch_k(k_force_mx<D, true, true, false>, grid, block, 0, s, pdl, P);
-    else perm ? launch_k(k_force_mx<D, false, true, true>, grid, block, 0, s, pdl, P)
-              : launch_k(k_force_mx<D, false, true, false>, grid, block, 0, s, pdl, P);
-  } else {
-    if (rec) perm ? launch_k(k_force_mx<D, true, false, true>, grid, block, 0, s, pdl, P)
-                  : launch_k(k_force_mx<D, true, false, false>, grid, block, 0, s, pdl, P);
-    else perm ? launch_k(k_force_mx<D, false, false, true>, grid, block, 0, s, pdl, P)
-              : launch_k(k_force_mx<D, false, false, false>, grid, block, 0, s, pdl, P);
-  }
+  using K = void (*)(const Dev);
+  launch_k((K)force_mx_ptr<D>(rec, P.grain_contact, P.node_orig, P.cand_q, force_bps(P.n_chunks, P.n_sms)), grid, block,
+           0, s, pdl, P);
 }
 
 cudaError_t kernels_mixed_init() {
@@ -748,17 +777,15 @@ cudaError_t kernels_mixed_init() {
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_finalize<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, FINAL_SMEM);
   if (e != cudaSuccess) return e;
   // the recording variants of the force kernel have local frames of about 1.1 KB
-  const void* fs[] = {
-      (const void*)k_force_mx<2, false, false, false>, (const void*)k_force_mx<2, false, true, false>,
-      (const void*)k_force_mx<2, true, false, false>,  (const void*)k_force_mx<2, true, true, false>,
-      (const void*)k_force_mx<3, false, false, false>, (const void*)k_force_mx<3, false, true, false>,
-      (const void*)k_force_mx<3, true, false, false>,  (const void*)k_force_mx<3, true, true, false>,
-      (const void*)k_force_mx<2, false, false, true>,  (const void*)k_force_mx<2, false, true, true>,
-      (const void*)k_force_mx<2, true, false, true>,   (const void*)k_force_mx<2, true, true, true>,
-      (const void*)k_force_mx<3, false, false, true>,  (const void*)k_force_mx<3, false, true, true>,
-      (const void*)k_force_mx<3, true, false, true>,   (const void*)k_force_mx<3, true, true, true>};
+  const void* fs[2 * 48];
+  int n = 0;
+  for (int k = 0; k < 16; ++k)
+    for (int b = 5; b <= 7; ++b) {
+      fs[n++] = force_mx_ptr<2>(k & 8, k & 4, k & 2, k & 1, b);
+      fs[n++] = force_mx_ptr<3>(k & 8, k & 4, k & 2, k & 1, b);
+    }
   size_t need = 0;
-  e = max_local_bytes(fs, 16, &need);
+  e = max_local_bytes(fs, n, &need);
   return e == cudaSuccess ? ensure_local_bytes(need) : e;
 }
 
