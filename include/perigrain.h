@@ -362,7 +362,7 @@ const char* pg_bond_last_error(void);
  * and hosts that reserve all device memory up front or run under a hard device-memory quota. This
  * entry point has no counterpart in the reference. Same arguments and results as pg_build_bonds;
  * its scratch is a file-scope device array sized for one grain of at most PG_NOALLOC_MAX_NODES
- * nodes (about 1.7 MB, held by every GPU that loads the library until exit); larger n returns
+ * nodes (about 1.4 MB, held by every GPU that loads the library until exit); larger n returns
  * PG_EINVAL. Calls share that array, so calls that overlap on the GPU race; each call clears what
  * it needs. The first call on a device looks the array's device address up and caches it for the
  * CUDA context (make that first call before any stream capture; do not call it again on a device

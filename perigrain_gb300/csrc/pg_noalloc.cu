@@ -29,11 +29,7 @@
 namespace {
 
 constexpr uint32_t kMaxNodes = PG_NOALLOC_MAX_NODES;
-constexpr uint32_t kCells = pg::bond_grid_cells_c(kMaxNodes);
-constexpr uint32_t kTiles = pg::bond_scan_tiles_c(kCells > kMaxNodes ? kCells : kMaxNodes);
-// box (6 x u64) + counts + starts + 5 per-node arrays (+1 for the offsets' total) + tile sums +
-// ticket + error word
-constexpr size_t kWords = 12 + (size_t)kCells + ((size_t)kCells + 1) + (size_t)kMaxNodes * 5 + 1 + kTiles + 1 + 1;
+constexpr size_t kWords = pg::bond_scratch_words(kMaxNodes);
 
 __device__ __align__(256) uint32_t g_bond_scratch[kWords];
 
@@ -75,36 +71,11 @@ extern "C" int pg_build_bonds_noalloc(const double* pos, uint32_t n, uint32_t di
     g_scratch_addr[dev].store(p, std::memory_order_release);
     base = p;
   }
-  pg::BondScratch S;
-  S.cells = pg::bond_grid_cells(n);
-  const uint32_t tiles = pg::bond_scan_tiles(S.cells > n ? S.cells : n);
-  uint32_t* w = base;
-  S.box = (unsigned long long*)w;  // 256-byte aligned start
-  w += 12;
-  S.cell_count = w;
-  w += S.cells;
-  S.cell_start = w;
-  w += S.cells + 1;
-  S.key = w;
-  w += n;
-  S.rank = w;
-  w += n;
-  S.sorted = w;
-  w += n;
-  S.pcount = w;
-  w += n;
-  S.poff = w;
-  w += n + 1;
-  S.tile_sum = w;
-  w += tiles;
-  S.done = w;
-  w += 1;
-  S.error = (int32_t*)w;
-  w += 1;
-  if ((size_t)(w - base) > kWords) {  // cannot happen for n <= kMaxNodes (sizes are monotone in n)
+  if (pg::bond_scratch_words(n) > kWords) {  // cannot happen for n <= kMaxNodes (sizes are monotone in n)
     g_err = "internal: scratch layout exceeds the static array";
     return PG_EINVAL;
   }
+  const pg::BondScratch S = pg::bond_scratch(base, n);
   std::string err;
   const int rc = pg::run_bond_build(pos, n, dim, delta, pairs, capacity, n_pairs, (cudaStream_t)stream, S, &err);
   if (rc) g_err = err;
