@@ -350,8 +350,10 @@ int pg_grad_times(pg_handle* h, double* forward_ms, double* backward_ms, uint64_
  * reference's setup writes (exp_dict.py:171-222: itertools.combinations + single_bond, which
  * compares the same FP64 distance). pos: device pointer, n x dim doubles; pairs: device pointer,
  * capacity x 2 uint32. *n_pairs receives the number of pairs (also when it exceeds capacity, then
- * PG_ECAPACITY and the first `capacity` rows are written). Temporary device memory is allocated
- * and freed inside the call. Runs on `stream` (a cudaStream_t, NULL for the default stream) and
+ * PG_ECAPACITY and the first `capacity` rows are written). Its scratch is one device array of
+ * 11.6 MB that the library keeps on each GPU that has run a build, for grains of up to 262144 nodes;
+ * larger grains, and calls that overlap another one, allocate and free device memory inside the
+ * call. Runs on `stream` (a cudaStream_t, NULL for the default stream) and
  * returns after it completes. pg_bond_last_error() describes a failure. */
 int pg_build_bonds(const double* pos, uint32_t n, uint32_t dim, double delta, uint32_t* pairs,
                    uint64_t capacity, uint64_t* n_pairs, void* stream);

@@ -12,7 +12,7 @@
 // Bound by launch and memory latency: 200k nodes in 2D are 21 MB of pairs, a few us of bandwidth.
 // 200k nodes, 3 spacings, us a call: 545 with the grid fitted on the host (a wait in the middle),
 // FP64 distances in both pair passes (164 + 162) and rows sorted in global memory; 244 now, 23 + 43 in
-// the pair passes and about 130 in allocating and freeing the scratch.
+// the pair passes; 115 with the scratch kept (pg_bond_scratch.cu).
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -577,13 +577,16 @@ extern "C" int pg_build_bonds(const double* pos, uint32_t n, uint32_t dim, doubl
   *n_pairs = 0;
   if (n < 2) return PG_OK;
   cudaStream_t st = (cudaStream_t)stream;
+  const KeptBondScratch kept(n);  // released after run_bond_build, which waits for the stream
   void* block = nullptr;
-  cudaError_t e = cudaMalloc(&block, bond_scratch_words(n) * 4);
-  if (e != cudaSuccess) {
-    g_bond_err = cudaGetErrorString(e);
-    return PG_ENOMEM;
+  if (!kept.base) {
+    const cudaError_t e = cudaMalloc(&block, bond_scratch_words(n) * 4);
+    if (e != cudaSuccess) {
+      g_bond_err = cudaGetErrorString(e);
+      return PG_ENOMEM;
+    }
   }
-  const BondScratch S = bond_scratch((uint32_t*)block, n);
+  const BondScratch S = bond_scratch(kept.base ? kept.base : (uint32_t*)block, n);
   std::string err;
   int rc = run_bond_build(pos, n, dim, delta, pairs, capacity, n_pairs, st, S, &err);
   cudaFree(block);

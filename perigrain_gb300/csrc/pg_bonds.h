@@ -59,6 +59,15 @@ BondScratch bond_scratch(uint32_t* base, uint32_t n);
 cudaError_t scan_u32_dev(const uint32_t* in, uint32_t len, uint32_t* out, uint32_t* tile_sum, uint32_t* done,
                          cudaStream_t st);
 uint32_t bond_scan_tiles(uint32_t len);
+// The kept scratch, held while the object lives: base is null if n is too large for it, another call
+// has it, or it cannot be had on this device.
+struct KeptBondScratch {
+  uint32_t* base = nullptr;
+  explicit KeptBondScratch(uint32_t n);
+  ~KeptBondScratch();
+  KeptBondScratch(const KeptBondScratch&) = delete;
+  KeptBondScratch& operator=(const KeptBondScratch&) = delete;
+};
 int run_bond_build(const double* pos, uint32_t n, uint32_t dim, double delta, uint32_t* pairs, uint64_t capacity,
                    uint64_t* n_pairs, cudaStream_t st, const BondScratch& S, std::string* err);
 

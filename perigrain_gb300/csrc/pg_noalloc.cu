@@ -6,7 +6,7 @@
 // computes, with its scratch in one file-scope device array instead of cudaMalloc'd memory, and
 // calls no cudaMalloc, cudaFree or other allocating routine.
 //
-// The array holds the scratch of one grain of up to PG_NOALLOC_MAX_NODES nodes (about 1.7 MB);
+// The array holds the scratch of one grain of up to PG_NOALLOC_MAX_NODES nodes (about 1.4 MB);
 // every GPU that loads the library keeps it until the process exits. Calls share it: two calls
 // that overlap on the GPU (different streams, or different host threads on one device) race and
 // must be serialised by the caller. Whatever a call needs zeroed (cell counts, flags, the

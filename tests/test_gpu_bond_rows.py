@@ -95,3 +95,37 @@ def test_too_many_partners_and_too_many_cells():
     assert rc == N.PG_ECAPACITY and m == 4200 * 4199 // 2 and b"4096 partners" in N.lib().pg_bond_last_error()
     rc, m, _ = _call(np.random.default_rng(11).random((200, 3)), 1e-60, 16)
     assert rc == N.PG_ECAPACITY and m == 0 and b"grid" in N.lib().pg_bond_last_error()
+
+
+def test_builds_side_by_side():
+    """Calls of several threads, each on its own stream: one holds the kept scratch at a time, the
+    others bring their own; every one gives its grain's rows."""
+    import threading
+
+    import torch
+
+    grains = [(np.random.default_rng(20 + k).random((3000 + 500 * k, 2 + k % 2)), 0.05 + 0.05 * (k % 2)) for k in range(4)]
+    refs = [_oracle(p, d) for p, d in grains]
+    wrong = []
+
+    def work(k):
+        p, delta = grains[k]
+        stream = torch.cuda.Stream()
+        with torch.cuda.stream(stream):
+            d_pos = torch.from_numpy(p).cuda()
+            d_pairs = torch.empty((len(refs[k]), 2), dtype=torch.int32, device="cuda")
+            for _ in range(20):
+                d_pairs.fill_(-7)
+                m = C.c_uint64()
+                rc = N.lib().pg_build_bonds(C.c_void_p(d_pos.data_ptr()), len(p), p.shape[1], delta,
+                                            C.c_void_p(d_pairs.data_ptr()), len(refs[k]), C.byref(m),
+                                            C.c_void_p(stream.cuda_stream))
+                if rc != N.PG_OK or m.value != len(refs[k]) or not np.array_equal(d_pairs.cpu().numpy(), refs[k]):
+                    wrong.append(k)
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
