@@ -117,3 +117,28 @@ def test_dropin_timestep_data_matches_output_files():
         _close(fields["f_sum"][t - 1], fsum, fabs)
         wi = tc["wall_info"]
         _close(fields["volume_fraction"][t - 1], vol.sum() / ((wi[1] - wi[0]) * (wi[2] - wi[3])))
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+@pytest.mark.parametrize("nodes", [30, 255, 256, 257, 900])
+def test_grain_sums_at_block_edges(dim, nodes):
+    """Grains below, at and above one round of a block's threads, several per instance, with bonds
+    broken and a node that never had any."""
+    k = setups.settling_2d if dim == 2 else setups.spheres_3d
+    s = setups.concat([k(**{"n_grains" if dim == 2 else "n": 3, "nodes_per_grain": nodes}) for _ in range(2)])
+    sim = Simulation(s, dt=2e-8, enable_fracture=1, precision="fp64")
+    alive = np.random.default_rng(nodes).random(s.n_bonds) < 0.8
+    deg = np.diff(s.bond_offset.astype(np.int64))
+    lo, hi = s.bond_offset[0], s.bond_offset[1]
+    alive[int(lo):int(hi)] = False  # node 0 loses its whole row
+    sim.set_bond_alive(alive.astype(np.uint8))
+    p = sim.postprocess(node_damage=True)
+    dmg = _damage(s, alive)
+    ok = deg > 0
+    assert np.array_equal(p["node_damage"][ok], dmg[ok]) and np.isnan(p["node_damage"][~ok]).all()
+    off = np.asarray(s.grain_node_offset, np.int64)
+    for g in range(s.n_grains):
+        sl = slice(off[g], off[g + 1])
+        _close(p["grain_mean_currpos"][g], sim.field("CurrPos")[sl].mean(0), np.abs(s.pos).max())
+        if ok[sl].all():
+            _close(p["grain_damage"][g], dmg[sl].mean())
