@@ -144,14 +144,14 @@ __device__ __forceinline__ void wall_geom(double R, double dd, double* A, double
 // reach the state (grains that are not movable, clamped nodes)
 template <int D>
 __device__ __forceinline__ bool force_bar(const Dev& P, const AdjStep& A, uint32_t j, double* Fb) {
+  double ab[D], vb[D];
+  ldv<D>(A.ab, j, ab);
+  ldv<D>(A.vb, j, vb);
   const GrainDev& gj = P.grain[P.node_grain[j]];
   if (!(gj.flags & GF_MOVABLE) || P.clamped[j]) {
     for (int c = 0; c < D; ++c) Fb[c] = 0.0;
     return false;
   }
-  double ab[D], vb[D];
-  ldv<D>(A.ab, j, ab);
-  ldv<D>(A.vb, j, vb);
   for (int c = 0; c < D; ++c) Fb[c] = gj.one_over_rho * (ab[c] + P.half_dt * vb[c]);
   return true;
 }
@@ -295,18 +295,83 @@ __global__ void __launch_bounds__(32 * SUB) k_adj_bonds(const Dev P, const AdjSt
   A.pcb[d] = pcs;
 }
 
-// Contact, wall and integrator part of the reverse step: one block per 32-node chunk, SUB warps;
-// warp w takes the node's contact entries i = w, w+SUB, ..., warp 0 also the walls; the partial
-// cotangents are summed in shared memory in a fixed order and warp 0 adds the bond share from
-// k_adj_bonds and runs the integrator. For the FP32 bond path it also writes the force cotangent
-// of the next reverse step to fbf. In 2D at most 128 registers, 4 blocks per SM (138 unbounded,
-// 3 per SM: a 592-chunk handle then ran 1.3 waves); 3D keeps its 168 registers, 3 blocks per SM.
+// Contact, wall and integrator part of the reverse step, one block per 32-node chunk. A contact of a
+// pair acts on the node through two forces, its own and its partner's, and each is a task of a few
+// hundred dependent FP64 operations. The chunk's tasks are laid out over the block's threads, 64
+// entries of the nodes' lists a round with the own forces on warps 0 and 1 and the partners' on 2 and
+// 3, so a chunk with contacts takes one such chain where a lane a node took two for every SUB
+// entries of its node. The walls are a chain of their own, on a warp that mostly has no task. The
+// node lanes add the results in a fixed order, warp w the entries i = w, w+SUB, ...; warp 0 adds the
+// warps' sums and the bond share from k_adj_bonds and runs the integrator. For the FP32 bond path it
+// also writes the force cotangent of the next reverse step to fbf. Bound by that latency: 592 chunks
+// are one wave of one or two active warps a block; 20k nodes in 50 grains, us: 21.6 -> 13.7 (about 5 with
+// neither contacts nor walls).
+constexpr uint32_t ADJ_ENTRIES = 16 * SUB;  // entries of a round
+
+// The contact tasks of entry e of node p (grain g, force cotangent Fb): its own force, or the
+// partner's. r[0..D): position share, r[D..2D): velocity share, then the parameters'.
+template <int D>
+__device__ __forceinline__ void contact_task(const Dev& P, const AdjStep& A, uint32_t p, uint32_t g, const double* Fb,
+                                             uint32_t entry, bool partner, double* out) {
+  const uint32_t q = entry & ENT_NODE;
+  const uint32_t gqi = P.node_grain[q], oq = A.off[q], nq = A.cnt[q];
+  double xp[D], xq[D], vp[D], vq[D], F[D], y[D], r[D], yb[D], rb[D], pb[3] = {0.0, 0.0, 0.0};
+  ldv<D>(A.X, p, xp);
+  ldv<D>(A.X, q, xq);
+  ldv<D>(A.V, p, vp);
+  ldv<D>(A.V, q, vq);
+  const double vol = P.vol[partner ? p : q];
+  const GrainDev &gr = P.grain[g], &gq = P.grain[gqi];
+  uint32_t fr = entry >> 30;
+  if (partner) {
+    // the partner's force from this node, if the partner recorded it
+    if (!force_bar<D>(P, A, q, F)) return;
+    fr = 4u;
+#pragma unroll 4
+    for (uint32_t k = 0; k < nq; ++k) {
+      const uint32_t eq = A.ent[oq + k];
+      if ((eq & ENT_NODE) == p) fr = eq >> 30;
+    }
+    if (fr == 4u) return;
+  }
+  const bool same = gqi == g;
+  double Kn, Rc, zeta, mu;
+  pair_params<D>(P, P.inst[gr.inst], gr, gq, same, p, q, &Kn, &Rc, &zeta, &mu);
+  const double sg = partner ? -1.0 : 1.0;
+#pragma unroll
+  for (int c = 0; c < D; ++c) {
+    if (!partner) F[c] = Fb[c];
+    y[c] = sg * (xq[c] - xp[c]);
+    r[c] = sg * (vp[c] - vq[c]);
+    yb[c] = 0.0;
+    rb[c] = 0.0;
+  }
+  pair_vjp<D>(y, r, F, Kn, Rc, zeta, mu, vol, partner ? gq.rho : gr.rho, fr, P.allow_damping, P.allow_friction, P.dt,
+              yb, rb, pb);
+#pragma unroll
+  for (int c = 0; c < D; ++c) {
+    out[c] = -sg * yb[c];
+    out[D + c] = sg * rb[c];
+  }
+  double* pc = out + 2 * D;
+  if (!same) {
+    pc[1] = 0.5 * pb[0];
+    pc[2] = 0.5 * pb[1];
+    pc[3] = 0.5 * pb[2];
+  } else if (!partner) {
+    pc[0] = pb[0] / Rc;  // K_n' = cnot / R_c'
+    pc[2] = pb[1];
+    pc[3] = pb[2];
+  }
+}
+
 template <int D>
 __global__ void __launch_bounds__(32 * SUB, D == 2 ? 4 : 3) k_adj_rest(const Dev P, const AdjStep A) {
   pdl_enter();
   constexpr int NS = 2 * D;
   constexpr int NV = 2 * D + NPARAM;  // xb[D], vfb[D], pc[NPARAM]
   __shared__ double red[SUB][NV][32];
+  __shared__ double res[NV][32 * SUB];
   const uint32_t lane = threadIdx.x & 31, sub = threadIdx.x >> 5;
   const uint32_t d = blockIdx.x * 32 + lane;
   const bool act = d < P.N;
@@ -315,166 +380,145 @@ __global__ void __launch_bounds__(32 * SUB, D == 2 ? 4 : 3) k_adj_rest(const Dev
   double* xb = acc;
   double* vfb = acc + D;
   double* pc = acc + 2 * D;
-  double Fb[D];
-  uint32_t g = 0;
+  double Fb[D] = {};
+  uint32_t g = 0, o = 0, n = 0, wbits = 0;
   bool live = false;
   if (act) {
     g = P.node_grain[d];
+    o = A.off[d];
+    n = A.cnt[d];
+    wbits = A.wall[d];
     live = force_bar<D>(P, A, d, Fb);
+    if (!live) n = wbits = 0;
   }
-  if (live) {
-    const GrainDev gr = P.grain[g];
+  uint32_t incl = n;
+#pragma unroll
+  for (int s = 1; s < 32; s <<= 1) {
+    const uint32_t v = __shfl_up_sync(0xffffffffu, incl, s);
+    if (lane >= (uint32_t)s) incl += v;
+  }
+  const uint32_t first = incl - n, total = __shfl_sync(0xffffffffu, incl, 31);
+  const bool pairs = total || __any_sync(0xffffffffu, wbits);  // the same in every warp
+  if (!pairs && sub != 0) return;
+
+  // walls: the node's force and, at the objective's step, its share of the wall reactions
+  if (sub == SUB - 1 && wbits) {
+    const GrainDev& gr = P.grain[g];
     const InstDev& in = P.inst[gr.inst];
     double xp[D], vp[D];
     ldv<D>(A.X, d, xp);
     ldv<D>(A.V, d, vp);
     const double volp = P.vol[d];
-
-    // contacts: the node's own forces (its list) and the partners' forces from it (their lists)
     const bool damp = P.allow_damping, fric = P.allow_friction;
-    const uint32_t o = A.off[d], n = A.cnt[d];
-    for (uint32_t i = sub; i < n; i += SUB) {
-      const uint32_t e = A.ent[o + i];
-      const uint32_t q = e & ENT_NODE, fr = e >> 30;
-      const uint32_t gqi = P.node_grain[q];
-      const bool same = gqi == g;
-      const GrainDev gq = P.grain[gqi];
-      double Kn, Rc, zeta, mu;
-      pair_params<D>(P, in, gr, gq, same, d, q, &Kn, &Rc, &zeta, &mu);
-      double xq[D], vq[D], y[D], r[D];
-      ldv<D>(A.X, q, xq);
-      ldv<D>(A.V, q, vq);
-      for (int c = 0; c < D; ++c) {
-        y[c] = xq[c] - xp[c];
-        r[c] = vp[c] - vq[c];
+    const double R = in.contact_rad, Kn = gr.kn, rho = gr.rho;
+    for (int k = 0; k < NS; ++k) {
+      if (!wb_contact(wbits, k)) continue;
+      int side, dir;
+      wall_side<D>(k, &side, &dir);
+      double gv[D];
+      for (int c = 0; c < D; ++c) gv[c] = Fb[c];
+      if (A.rbar) {
+        // reaction[side] -= vol_p * (the node's wall force of this side)
+        for (int c = 0; c < D; ++c) gv[c] -= volp * A.rbar[((size_t)gr.inst * NS + side) * D + c];
       }
-      double yb[D], rb[D], pb[3] = {0.0, 0.0, 0.0};
-      for (int c = 0; c < D; ++c) {
-        yb[c] = 0.0;
-        rb[c] = 0.0;
-      }
-      pair_vjp<D>(y, r, Fb, Kn, Rc, zeta, mu, P.vol[q], gr.rho, fr, damp, fric, P.dt, yb, rb, pb);
-      for (int c = 0; c < D; ++c) {
-        xb[c] -= yb[c];
-        vfb[c] += rb[c];
-      }
-      if (same) {
-        pc[0] += pb[0] / Rc;  // K_n' = cnot / R_c'
-        pc[2] += pb[1];
-        pc[3] += pb[2];
-      } else {
-        pc[1] += 0.5 * pb[0];
-        pc[2] += 0.5 * pb[1];
-        pc[3] += 0.5 * pb[2];
-      }
-      // the partner's force from this node, if the partner recorded it
-      const uint32_t oq = A.off[q], nq = A.cnt[q];
-      uint32_t frq = 4u;
-      for (uint32_t k = 0; k < nq; ++k) {
-        const uint32_t eq = A.ent[oq + k];
-        if ((eq & ENT_NODE) == d) {
-          frq = eq >> 30;
-          break;
-        }
-      }
-      if (frq == 4u) continue;
-      double Fq[D];
-      if (!force_bar<D>(P, A, q, Fq)) continue;
-      double y2[D], r2[D], yb2[D], rb2[D], pb2[3] = {0.0, 0.0, 0.0};
-      for (int c = 0; c < D; ++c) {
-        y2[c] = xp[c] - xq[c];
-        r2[c] = vq[c] - vp[c];
-        yb2[c] = 0.0;
-        rb2[c] = 0.0;
-      }
-      pair_vjp<D>(y2, r2, Fq, Kn, Rc, zeta, mu, volp, gq.rho, frq, damp, fric, P.dt, yb2, rb2, pb2);
-      for (int c = 0; c < D; ++c) {
-        xb[c] += yb2[c];
-        vfb[c] -= rb2[c];
-      }
-      if (!same) {
-        pc[1] += 0.5 * pb2[0];
-        pc[2] += 0.5 * pb2[1];
-        pc[3] += 0.5 * pb2[2];
-      }
-    }
-
-    // walls: the node's force and, at the objective's step, its share of the wall reactions
-    const uint32_t wbits = A.wall[d];
-    if (sub == 0 && wbits) {
-      const double R = in.contact_rad, Kn = gr.kn, rho = gr.rho;
-      for (int k = 0; k < NS; ++k) {
-        if (!wb_contact(wbits, k)) continue;
-        int side, dir;
-        wall_side<D>(k, &side, &dir);
-        double gv[D];
-        for (int c = 0; c < D; ++c) gv[c] = Fb[c];
-        if (A.rbar) {
-          // reaction[side] -= vol_p * (the node's wall force of this side)
-          for (int c = 0; c < D; ++c) gv[c] -= volp * A.rbar[((size_t)gr.inst * NS + side) * D + c];
-        }
-        const double dist = xp[dir] - A.W[(size_t)gr.inst * NS + side];
-        const double dd = fmin(fabs(dist), R);  // the replay's extension beyond R
-        const double cs = dist > 0 ? 1.0 : -1.0;
-        double Ar, Ap, FK, FKp;
-        wall_geom<D>(R, dd, &Ar, &Ap, &FK, &FKp);
-        const double F = Kn * FK, Fp = Kn * FKp;  // dF/d(dd); d(dd)/dX = cs
-        // normal: f[dir] += cs F
-        xb[dir] += gv[dir] * Fp;
-        pc[1] += gv[dir] * cs * FK;
-        double rv[D];
-        for (int c = 0; c < D; ++c) rv[c] = vp[c];
-        rv[dir] -= in.wall_speed[side];
-        if (fric && wb_fric(wbits, k)) {
-          const bool stick = wb_stick(wbits, k);
-          const double sF = F > 0 ? 1.0 : (F < 0 ? -1.0 : 0.0);
-          if constexpr (D == 2) {
-            const int tg = (dir + 1) % 2;
-            if (stick) {
-              vfb[tg] += gv[tg] * (-rho / P.dt);
-            } else {
-              const double vts = wb_neg(wbits, k) ? -1.0 : 1.0;
-              xb[dir] += gv[tg] * (-gr.mu * vts * sF * Fp * cs);
-              pc[3] += gv[tg] * (-fabs(F) * vts);
-              pc[1] += gv[tg] * (-gr.mu * vts * sF * FK);
-            }
+      const double dist = xp[dir] - A.W[(size_t)gr.inst * NS + side];
+      const double dd = fmin(fabs(dist), R);  // the replay's extension beyond R
+      const double cs = dist > 0 ? 1.0 : -1.0;
+      double Ar, Ap, FK, FKp;
+      wall_geom<D>(R, dd, &Ar, &Ap, &FK, &FKp);
+      const double F = Kn * FK, Fp = Kn * FKp;  // dF/d(dd); d(dd)/dX = cs
+      // normal: f[dir] += cs F
+      xb[dir] += gv[dir] * Fp;
+      pc[1] += gv[dir] * cs * FK;
+      double rv[D];
+      for (int c = 0; c < D; ++c) rv[c] = vp[c];
+      rv[dir] -= in.wall_speed[side];
+      if (fric && wb_fric(wbits, k)) {
+        const bool stick = wb_stick(wbits, k);
+        const double sF = F > 0 ? 1.0 : (F < 0 ? -1.0 : 0.0);
+        if constexpr (D == 2) {
+          const int tg = (dir + 1) % 2;
+          if (stick) {
+            vfb[tg] += gv[tg] * (-rho / P.dt);
           } else {
-            const int t1 = (dir + 1) % 3, t2 = (dir + 2) % 3;
-            if (stick) {
-              vfb[t1] += gv[t1] * (-1.0 / (rho * P.dt));
-              vfb[t2] += gv[t2] * (-1.0 / (rho * P.dt));
-            } else {
-              const double v1 = rv[t1], v2 = rv[t2];
-              const double vn = sqrt(v1 * v1 + v2 * v2);
-              if (vn > 0) {
-                const double u1 = v1 / vn, u2 = v2 / vn;
-                const double a = gv[t1] * u1 + gv[t2] * u2;
-                xb[dir] += -gr.mu * a * sF * Fp * cs;
-                pc[3] += -fabs(F) * a;
-                pc[1] += -gr.mu * a * sF * FK;
-                vfb[t1] += -gr.mu * fabs(F) * (gv[t1] - a * u1) / vn;
-                vfb[t2] += -gr.mu * fabs(F) * (gv[t2] - a * u2) / vn;
-              }
+            const double vts = wb_neg(wbits, k) ? -1.0 : 1.0;
+            xb[dir] += gv[tg] * (-gr.mu * vts * sF * Fp * cs);
+            pc[3] += gv[tg] * (-fabs(F) * vts);
+            pc[1] += gv[tg] * (-gr.mu * vts * sF * FK);
+          }
+        } else {
+          const int t1 = (dir + 1) % 3, t2 = (dir + 2) % 3;
+          if (stick) {
+            vfb[t1] += gv[t1] * (-1.0 / (rho * P.dt));
+            vfb[t2] += gv[t2] * (-1.0 / (rho * P.dt));
+          } else {
+            const double v1 = rv[t1], v2 = rv[t2];
+            const double vn = sqrt(v1 * v1 + v2 * v2);
+            if (vn > 0) {
+              const double u1 = v1 / vn, u2 = v2 / vn;
+              const double a = gv[t1] * u1 + gv[t2] * u2;
+              xb[dir] += -gr.mu * a * sF * Fp * cs;
+              pc[3] += -fabs(F) * a;
+              pc[1] += -gr.mu * a * sF * FK;
+              vfb[t1] += -gr.mu * fabs(F) * (gv[t1] - a * u1) / vn;
+              vfb[t2] += -gr.mu * fabs(F) * (gv[t2] - a * u2) / vn;
             }
           }
         }
-        if (damp) {
-          // df = -dc rv[dir], dc = 2 zeta sqrt(K_n rho) sqrt(|Area|)
-          const double sq = sqrt(Kn * rho);
-          const double sa = sqrt(fabs(Ar));
-          const double dc = 2.0 * gr.zeta * sq * sa;
-          vfb[dir] += gv[dir] * (-dc);
-          if (sa > 0) xb[dir] += gv[dir] * (-rv[dir]) * gr.zeta * sq * (Ap / sa) * cs;
-          pc[2] += gv[dir] * (-rv[dir]) * 2.0 * sq * sa;
-          if (Kn != 0.0) pc[1] += gv[dir] * (-rv[dir]) * dc / (2.0 * Kn);
-        }
+      }
+      if (damp) {
+        // df = -dc rv[dir], dc = 2 zeta sqrt(K_n rho) sqrt(|Area|)
+        const double sq = sqrt(Kn * rho);
+        const double sa = sqrt(fabs(Ar));
+        const double dc = 2.0 * gr.zeta * sq * sa;
+        vfb[dir] += gv[dir] * (-dc);
+        if (sa > 0) xb[dir] += gv[dir] * (-rv[dir]) * gr.zeta * sq * (Ap / sa) * cs;
+        pc[2] += gv[dir] * (-rv[dir]) * 2.0 * sq * sa;
+        if (Kn != 0.0) pc[1] += gv[dir] * (-rv[dir]) * dc / (2.0 * Kn);
       }
     }
   }
 
+  // contacts: the node's own forces (its list) and the partners' forces from it (their lists)
+  for (uint32_t e0 = 0; e0 < total; e0 += ADJ_ENTRIES) {
+    const uint32_t m = min(total - e0, ADJ_ENTRIES);
+    const bool partner = threadIdx.x >= m;
+    const uint32_t e = e0 + (partner ? threadIdx.x - m : threadIdx.x);
+    uint32_t pl = 0;  // the lane of entry e: as many lanes' lists end at or before it
+#pragma unroll
+    for (uint32_t s = 16; s; s >>= 1)
+      if (__shfl_sync(0xffffffffu, incl, pl + s - 1) <= e) pl += s;
+    const uint32_t gp = __shfl_sync(0xffffffffu, g, pl);
+    const uint32_t at = __shfl_sync(0xffffffffu, o - first, pl) + e;
+    double Fp[D];
+#pragma unroll
+    for (int c = 0; c < D; ++c) Fp[c] = __shfl_sync(0xffffffffu, Fb[c], pl);
+    if (threadIdx.x < 2 * m) {
+      double out[NV];
+#pragma unroll
+      for (int v = 0; v < NV; ++v) out[v] = 0.0;
+      contact_task<D>(P, A, blockIdx.x * 32 + pl, gp, Fp, A.ent[at], partner, out);
+#pragma unroll
+      for (int v = 0; v < NV; ++v) res[v][threadIdx.x] = out[v];
+    }
+    __syncthreads();
+    // entries of this round: [e0, e0 + ADJ_ENTRIES)
+    const uint32_t i1 = min(n, e0 + ADJ_ENTRIES > first ? e0 + ADJ_ENTRIES - first : 0u);
+    uint32_t i = sub;
+    if (e0 > first + sub) i += (e0 - first - sub + SUB - 1) / SUB * SUB;
+    for (; i < i1; i += SUB) {
+      const uint32_t k = first + i - e0;
+#pragma unroll
+      for (int v = 0; v < NV; ++v) acc[v] = (acc[v] + res[v][k]) + res[v][m + k];
+    }
+    __syncthreads();
+  }
+
   // fixed-order sum of the SUB partial cotangents, then the integrator (warp 0)
-  for (int v = 0; v < NV; ++v) red[sub][v][lane] = acc[v];
-  __syncthreads();
+  if (pairs) {
+    for (int v = 0; v < NV; ++v) red[sub][v][lane] = acc[v];
+    __syncthreads();
+  }
   if (sub != 0 || !act) return;
   if (!live) {
     // the state of this node does not depend on the parameters
@@ -490,11 +534,12 @@ __global__ void __launch_bounds__(32 * SUB, D == 2 ? 4 : 3) k_adj_rest(const Dev
     }
     return;
   }
-  for (int v = 0; v < NV; ++v) {
-    double sm = red[0][v][lane];
-    for (int w = 1; w < SUB; ++w) sm += red[w][v][lane];
-    acc[v] = sm;
-  }
+  if (pairs)
+    for (int v = 0; v < NV; ++v) {
+      double sm = red[0][v][lane];
+      for (int w = 1; w < SUB; ++w) sm += red[w][v][lane];
+      acc[v] = sm;
+    }
   double xbond[D];
   ldv<D>(A.xbb, d, xbond);
   for (int c = 0; c < D; ++c) xb[c] += xbond[c];
