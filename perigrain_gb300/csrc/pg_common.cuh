@@ -352,7 +352,7 @@ template <int D>
 __device__ __forceinline__ bool boxes_touch(const double (&mni)[D], const double (&mxi)[D],
                                             const double (&mnj)[D], const double (&mxj)[D], double c) {
   bool r = true;
-  for (int a = 0; a < D; ++a) r = r && ((mni[a] - c) <= mxj[a]) && ((mxi[a] + c) >= mnj[a]);
+  for (int a = 0; a < D; ++a) r = r & ((mni[a] - c) <= mxj[a]) & ((mxi[a] + c) >= mnj[a]);  // no branches
   return r;
 }
 
@@ -369,7 +369,7 @@ __device__ __forceinline__ bool within_interior(const double (&mn)[D], const dou
     A[0] = mn[0]; A[1] = mn[1]; A[2] = mn[2]; A[3] = mx[0];
   }
   double AL = A[0] - c, AR = A[1] + c, AT = A[2] + c, AB = A[3] - c;
-  return (W[0] < AL) && (AR < W[1]) && (W[2] > AT) && (W[3] < AB);
+  return (W[0] < AL) & (AR < W[1]) & (W[2] > AT) & (W[3] < AB);
 }
 
 template <int D>

@@ -53,6 +53,15 @@ inline int force_bps(uint32_t n_chunks, uint32_t sms) {
   return best;
 }
 
+// Whether the mixed force kernel puts a team of four warps on a chunk (candidate lists and the default
+// block of 128 threads only): where all teams are resident at once, 4 blocks of 128 threads (128
+// registers) an SM. us a step, a warp / a team a chunk: settling 179 chunks 11.9 / 8.0, 544 11.9 / 9.5,
+// 726 12.1 / 14.0, 1089 12.6 / 14.9; 3D spheres 242 chunks 27.8 / 16.6, 545 28.0 / 21.7, 847 30.1 /
+// 38.0; two disks (79 chunks) 13.3 / 9.7.
+inline bool force_team(const Dev& P, uint32_t block) {
+  return P.cand_q && block == 128 && P.n_chunks <= P.n_sms * 4u;
+}
+
 cudaError_t kernels_init();
 // The parts of an FP64 step, each enqueued on stream s: the position update; the grid build and the
 // force kernels; the end of the step. Add the number of kernel launches to *launches. pdl:

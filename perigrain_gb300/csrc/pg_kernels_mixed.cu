@@ -208,11 +208,11 @@ __global__ void __launch_bounds__(256) k_predict_mx(const Dev P) {
 // One bond: stretch s = (2 xi.eta + eta.eta) / (|xi| (|xi+eta| + |xi|)), force density
 // cnot * s * vol_j * (xi+eta)/|xi+eta| added to f when `use`. cv = cnot * vol_j.
 template <int D>
-__device__ __forceinline__ void bond_term(const float (&dh)[D], const float (&dl)[D], const float (&xh)[D],
+__device__ __forceinline__ float bond_term(const float (&dh)[D], const float (&dl)[D], const float (&xh)[D],
                                           const float (&xl)[D], const float (&jdh)[D], const float (&jdl)[D],
                                           const float (&jxh)[D], const float (&jxl)[D], float cv, bool use,
-                                          float (&f)[D], float* str_out) {
-  float xi[D], et[D], y[D];
+                                          float (&y)[D], float* str_out) {
+  float xi[D], et[D];
   for (int c = 0; c < D; ++c) {
     xi[c] = (jxh[c] - xh[c]) + (jxl[c] - xl[c]);
     et[c] = (jdh[c] - dh[c]) + (jdl[c] - dl[c]);
@@ -222,9 +222,175 @@ __device__ __forceinline__ void bond_term(const float (&dh)[D], const float (&dl
   const float ixn = rsqrtf(xx), iyn = rsqrtf(yy);
   const float num = fmaf(2.f, dotf<D>(xi, et), dotf<D>(et, et));
   const float str = __fdividef(num * ixn, fmaf(yy, iyn, xx * ixn));
-  const float sc = use ? cv * str * iyn : 0.f;
-  for (int c = 0; c < D; ++c) f[c] = fmaf(sc, y[c], f[c]);
   *str_out = str;
+  return use ? cv * str * iyn : 0.f;
+}
+
+// (float)sqrt(x), the FP64 square root rounded again, without it: c = sqrtf((float)x) is at most one
+// float off, and the exact remainder x - c c tells on which side of the halfway point between two
+// floats the root lies. Only within 2^-18 ulp of that point (where the second rounding could matter),
+// at a power of two and outside 1e-30..1e30 is the FP64 root itself taken. 300 cycles against 760: an
+// FP64 operation has a latency of 63 cycles here, and a square root chains ten.
+__device__ __forceinline__ float sqrt_to_float(double x) {
+  const float a = (float)x;
+  const float c = sqrtf(a);
+  const double cd = widen(c);
+  const float off = (float)fma(-cd, cd, x) * __fdividef(0.5f, c);  // sqrt(x) - c
+  const uint32_t cb = __float_as_uint(c);
+  const float up = __uint_as_float(cb + 1u) - c, h = 0.5f * up, ao = fabsf(off);
+  if (a > 1e-30f && a < 1e30f && (cb & 0x7fffffu) > 1u && (cb & 0x7fffffu) < 0x7ffffeu) {
+    if (ao < h * 0.999996f) return c;
+    if (ao > h * 1.000004f && ao < 1.4f * up) return __uint_as_float(off > 0.f ? cb + 1u : cb - 1u);
+  }
+  return (float)sqrt(x);
+}
+
+// What a contact reads of its partner q; loaded before anything is known of it, so that one latency
+// is waited for instead of one a test.
+template <int D>
+struct Partner {
+  double x[D], v[D];
+  float vol;
+  __device__ __forceinline__ Partner(const Dev& P, uint32_t q) {
+    ldv<D>(P.cur, q, x);
+    ldv<D>(P.vel_in, q, v);
+    vol = P.vol_f[q];
+  }
+  // The same for a team, whose tests follow one another on an idle SM: volatile loads stay where they
+  // are written (the compiler moves plain ones behind the tests that precede their use), so that all
+  // are in flight at once. gq: the partner's grain.
+  __device__ __forceinline__ Partner(const Dev& P, uint32_t q, uint32_t& gq, float (&qf)[D]) {
+    gq = *(const volatile uint32_t*)(P.node_grain + q);
+    constexpr uint32_t SF = D == 2 ? 2 : 4, S = D == 2 ? 2 : 4;
+    if constexpr (D == 2)
+      asm volatile("ld.volatile.global.v2.f32 {%0, %1}, [%2];" : "=f"(qf[0]), "=f"(qf[1]) : "l"(P.curf + (size_t)q * SF));
+    else
+      for (int c = 0; c < D; ++c) qf[c] = *(const volatile float*)(P.curf + (size_t)q * SF + c);
+    const double *px = P.cur + (size_t)q * S, *pv = P.vel_in + (size_t)q * S;
+    asm volatile("ld.volatile.global.v2.f64 {%0, %1}, [%2];" : "=d"(x[0]), "=d"(x[1]) : "l"(px));
+    if constexpr (D == 3) x[2] = *(const volatile double*)(px + 2);
+    asm volatile("ld.volatile.global.v2.f64 {%0, %1}, [%2];" : "=d"(v[0]), "=d"(v[1]) : "l"(pv));
+    if constexpr (D == 3) v[2] = *(const volatile double*)(pv + 2);
+    vol = *(const volatile float*)(P.vol_f + q);
+  }
+};
+
+// What a contact needs of the node itself: its state, its row of the bond slab and the contact
+// parameters of its grain and instance in FP32.
+template <int D>
+struct Side {
+  double x[D], v[D], rad, s_max;
+  float Kn, zeta, mu, rho, Rc, pre2, pf[D];
+  uint32_t g, deg, w0, slot0, lane;
+  uint32_t rules;  // SIDE_*
+  __device__ __forceinline__ void of(const Dev& P, const InstDev& in, const GrainDev& gr) {
+    rad = in.contact_rad;
+    s_max = in.contact_s_max;
+    Kn = (float)in.normal_stiffness;
+    zeta = (float)in.damping_ratio;
+    mu = (float)in.friction_coefficient;
+    rho = (float)gr.rho;
+    Rc = (float)in.contact_rad;
+  }
+};
+
+// Node q's contact with node d (s): false if there is none, else what the force receives, to be added in this order:
+// s1 u, sd u where damp, sf tg where fr. None of it depends on the force so far, so a team of warps
+// can form it for all contacts of a chunk at once.
+template <int D>
+struct ContactTerm {
+  float s1, sd, sf, u[D], tg[D];
+  float far;       // the largest component of x_q - x_p
+  uint32_t close;  // the two nodes are at the same place
+  uint32_t fr;     // FR_* of the friction branch taken, 0: none
+};
+template <int D, bool GC>
+__device__ __forceinline__ bool contact_term(const Dev& P, const Side<D>& s, uint32_t gqi, uint32_t d, uint32_t q,
+                                             const Partner<D>& pq, ContactTerm<D>& o) {
+  const bool same = gqi == s.g;
+  // The contact decision |x_q - x_p| <= R_c' is made with the reference's FP64 arithmetic:
+  // contact damping switches on at full strength at that boundary, so a decision flipped by
+  // FP32 rounding would kick a node by metres per second.
+  double dir64[D];
+  for (int c = 0; c < D; ++c) dir64[c] = pq.x[c] - s.x[c];
+  double n2 = dir64[0] * dir64[0];
+  for (int c = 1; c < D; ++c) n2 = n2 + dir64[c] * dir64[c];
+  // |x_q - x_p| <= contact_rad as n2 <= contact_s_max, the same outcome without the square root
+  if (!(n2 <= s.s_max)) return false;
+  float Kn = s.Kn, zeta = s.zeta, mu = s.mu;
+  if constexpr (GC) {
+    const GrainDev &gr = P.grain[s.g], &gq = P.grain[gqi];
+    Kn = (float)((gr.kn + gq.kn) * 0.5);
+    zeta = (float)((gr.zeta + gq.zeta) * 0.5);
+    mu = (float)((gr.mu + gq.mu) * 0.5);
+  }
+  float Rc = s.Rc;
+  if (same) {
+    double pp[D], ps[D], r[D];
+    ldv<D>(P.pos, d, pp);
+    ldv<D>(P.pos, q, ps);
+    for (int c = 0; c < D; ++c) r[c] = pp[c] - ps[c];
+    double r2 = r[0] * r[0];
+    for (int c = 1; c < D; ++c) r2 = r2 + r[c] * r[c];
+    // |x_q - x_p| <= R_c' = min(ref, contact_rad), ref = sqrt(r2): the roots compare as n2 and r2 do
+    // unless these are within a few units in the last place (1 + 2^-50: roots two such units apart)
+    if (n2 > r2 * 1.0000000000000009) return false;
+    bool bonded = false;
+    for (uint32_t k = 0; k < s.deg && !bonded; k += 8)  // eight at a time: independent loads
+#pragma unroll
+      for (uint32_t j = 0; j < 8; ++j) {
+        const uint32_t kk = min(k + j, s.deg - 1);
+        bonded |= ((P.alive[s.w0 + kk] >> s.lane) & 1u) && P.bcol[s.slot0 + 32u * kk] == q;
+      }
+    if (bonded) return false;
+    const double ref = sqrt(r2);
+    const double Rc64 = ref < s.rad ? ref : s.rad;
+    if (!(n2 <= r2) && !(sqrt(n2) <= Rc64)) return false;
+    Kn = (float)(P.grain[s.g].cnot / Rc64);
+    Rc = (float)Rc64;
+  }
+  const float dn = sqrt_to_float(n2);
+  float dir[D];
+  for (int c = 0; c < D; ++c) dir[c] = (float)dir64[c];
+  o.far = 0.f;
+  for (int c = 0; c < D; ++c) o.far = fmaxf(o.far, fabsf(dir[c]));
+  o.close = dn == 0.f;
+  const float inv = 1.f / dn;
+  float(&u)[D] = o.u;
+  for (int c = 0; c < D; ++c) u[c] = dir[c] * inv;
+  const float nvol = pq.vol;
+  const float s1 = -Kn * (Rc - dn) * nvol;
+  o.s1 = s1;
+  const float cfn = fabsf(s1);
+  const float rho = s.rho, dtf = (float)P.dt;
+  o.sd = o.sf = 0.f;
+  for (int c = 0; c < D; ++c) o.tg[c] = 0.f;
+  uint32_t fr = 0;
+  if (P.allow_damping || P.allow_friction) {
+    float rv[D];
+    for (int c = 0; c < D; ++c) rv[c] = (float)(s.v[c] - pq.v[c]);
+    const float rvp = dotf<D>(rv, u);
+    if (P.allow_damping) {
+      const float dc = 2.f * zeta * sqrtf(Kn * rho) * sqrtf(nvol);
+      o.sd = -dc * rvp;
+    }
+    if (P.allow_friction) {
+      float(&tg)[D] = o.tg;
+      for (int c = 0; c < D; ++c) tg[c] = fmaf(-rvp, u[c], rv[c]);
+      const float tn = sqrtf(dotf<D>(tg, tg));
+      if (tn > 0.f) {
+        float sfr = -mu * cfn;
+        fr = (D == 2 && (tg[1] * u[0] - tg[0] * u[1]) < 0.f) ? FR_SLIDE_NEG : FR_SLIDE;
+        if (tn < mu * cfn * dtf / rho) {
+          sfr = -tn / rho / dtf;
+          fr = FR_STICK;
+        }
+        o.sf = sfr / tn;
+      }
+    }
+  }
+  o.fr = fr;
+  return true;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -237,15 +403,147 @@ __device__ __forceinline__ uint32_t input_index(const Dev& P, uint32_t i) {
   if constexpr (PERM) return P.node_orig[i];
   return i;
 }
+// ---------------------------------------------------------------------------------------------
+// Teams: a chunk worked on by a block of four warps, where the chunks alone leave the GPU nearly idle
+// and a step's time is one warp's chain (force_team()). Each warp forms a quarter of the bond terms
+// and warp 0 adds them in the order of the bonds; the entries of the candidate lists are tasks for
+// all threads, and warp 0 adds the contacts in the order of the lists: the force is the same to the
+// bit. Bound by latency: an FP64 operation takes 63 cycles, a load that misses L1 250 to 500. Cycles
+// of a chunk with contacts, two disks, a warp / a team: bonds 7200 / 2800, contacts 8000-10900 /
+// 3300, the rest (start, walls, position update) 5200 / 4700.
+constexpr uint32_t TEAM_WARPS = 4;
+constexpr uint32_t TEAM_BONDS = 32;  // bonds between two barriers
 
-template <int D, bool REC, bool GC, bool PERM, bool LIST, int BPS>
+// The contacts a node may have; whether its list can overflow max_cand; whether its coordinates are
+// below 1e9 contact radii.
+constexpr uint32_t SIDE_SELF = 1u, SIDE_OTHER = 2u, SIDE_COUNT = 4u, SIDE_NEAR = 8u;
+
+template <int D, bool ON>
+struct TeamMem {
+  float sc[2][TEAM_BONDS][32], y[2][TEAM_BONDS][D][32];
+  uint32_t what[32 * TEAM_WARPS], node[32 * TEAM_WARPS];
+  ContactTerm<D> term[32 * TEAM_WARPS];
+  Side<D> side[32];
+  __device__ __forceinline__ void put(uint32_t k, uint32_t lane, float s, const float (&v)[D]) {
+    const uint32_t b = k / TEAM_BONDS % 2, i = k % TEAM_BONDS;
+    sc[b][i][lane] = s;
+    for (int c = 0; c < D; ++c) y[b][i][c][lane] = v[c];
+  }
+};
+template <int D>
+struct TeamMem<D, false> {};
+
+// All warps have put the bonds [k0, k1), at most TEAM_BONDS, into their buffer; warp 0 adds them. The
+// other buffer may be filled meanwhile: this one is not written again before the next barrier.
+template <int D>
+__device__ __forceinline__ void team_add(TeamMem<D, true>& tm, uint32_t k0, uint32_t k1, uint32_t lane, uint32_t sub,
+                                         float (&f)[D]) {
+  __syncthreads();
+  if (sub != 0) return;
+  const uint32_t b = k0 / TEAM_BONDS % 2;
+#pragma unroll 8
+  for (uint32_t i = 0; i < k1 - k0; ++i)
+    for (int c = 0; c < D; ++c) f[c] = fmaf(tm.sc[b][i][lane], tm.y[b][i][c][lane], f[c]);
+}
+
+// A team's bonds: of each TEAM_BONDS the warp forms eight in a row, their indices and (GB at a time)
+// their neighbours loaded before any is used, so a warp waits for two latencies, not two a pair.
+template <int D>
+__device__ __forceinline__ void team_bonds(const Dev& P, TeamMem<D, true>& tm, uint32_t d, uint32_t lane, uint32_t sub,
+                                           uint32_t cdeg, uint32_t w0, uint32_t slot0, bool mov, const float (&dh)[D],
+                                           const float (&dl)[D], const float (&xh)[D], const float (&xl)[D], float cnot,
+                                           float snot, uint32_t t, float (&f)[D]) {
+  constexpr uint32_t W = TEAM_BONDS / TEAM_WARPS, GB = D == 2 ? 8 : 4;
+  const uint32_t full = (cdeg + 1) & ~1u;  // a row without a last bond ends on an unused one, as in the pairs of a lone warp
+  for (uint32_t kb = 0; kb < cdeg; kb += TEAM_BONDS) {
+    const uint32_t k0 = kb + W * sub;
+    uint32_t word[W], col[W];
+#pragma unroll
+    for (uint32_t i = 0; i < W; ++i) {
+      word[i] = 0u;
+      col[i] = d;
+      if (k0 + i < cdeg) {
+        word[i] = P.alive[w0 + k0 + i];
+        col[i] = P.bcol[slot0 + 32u * (k0 + i)];
+      }
+    }
+#pragma unroll
+    for (uint32_t h = 0; h < W; h += GB) {
+      if (k0 + h >= full) continue;
+      float jdh[GB][D], jdl[GB][D], jxh[GB][D], jxl[GB][D], vol[GB];
+#pragma unroll
+      for (uint32_t i = 0; i < GB; ++i) {
+        const uint32_t j = mov && ((word[h + i] >> lane) & 1u) ? col[h + i] : d;
+        ld_hl<D>(P.dref, P.np, j, jdh[i], jdl[i]);
+        ld_hl<D>(P.xref, P.np, j, jxh[i], jxl[i]);
+        vol[i] = P.vol_f[j];
+      }
+      uint32_t broken = 0;
+      float s[GB], y[GB][D];
+#pragma unroll
+      for (uint32_t i = 0; i < GB; ++i) {
+        const bool use = mov && ((word[h + i] >> lane) & 1u);
+        float str;
+        s[i] = bond_term<D>(dh, dl, xh, xl, jdh[i], jdl[i], jxh[i], jxl[i], cnot * vol[i], use, y[i], &str);
+        broken |= (uint32_t)(use && str > snot) << i;
+      }
+#pragma unroll
+      for (uint32_t i = 0; i < GB; ++i) tm.put(k0 + h + i, lane, s[i], y[i]);
+      if (!__any_sync(0xffffffffu, broken)) continue;
+#pragma unroll
+      for (uint32_t i = 0; i < GB; ++i) {
+        const uint32_t k = k0 + h + i;
+        if (broken >> i & 1u) P.break_step[slot0 + 32u * k] = t;
+        const uint32_t now = word[h + i] & ~__ballot_sync(0xffffffffu, broken >> i & 1u);
+        if (lane == 0 && now != word[h + i]) P.alive[w0 + k] = now;
+      }
+    }
+    team_add<D>(tm, kb, min(kb + TEAM_BONDS, full), lane, sub, f);
+  }
+  if (!cdeg) __syncthreads();  // the Side records
+}
+
+// Entry q of node p's list: 0 = not within the prefilter or the rules, 1 = passed, 2 = a contact (o).
+// The box test of the grains is left out where it cannot matter: a contact well within the radius
+// lies in both boxes (0.999998 leaves room for the test's two roundings, SIDE_NEAR), and an entry without contact only counts where the list could overflow.
+template <int D, bool GC>
+__device__ __forceinline__ uint32_t team_contact(const Dev& P, const Side<D>& s, uint32_t p, uint32_t q,
+                                                 ContactTerm<D>& o) {
+  float qf[D];
+  uint32_t gq;
+  const Partner<D> pq(P, q, gq, qf);
+  float d2 = 0.f;
+  for (int c = 0; c < D; ++c) {
+    float dd = qf[c] - s.pf[c];
+    d2 = fmaf(dd, dd, d2);
+  }
+  if (d2 > s.pre2) return 0;
+  const bool same = gq == s.g;
+  if (!(s.rules & (same ? SIDE_SELF : SIDE_OTHER))) return 0;
+  if (P.nl_bdry_only && P.bdry_rank[q] == NONE) return 0;
+  const bool hit = contact_term<D, GC>(P, s, gq, p, q, pq, o);
+  if (same) return hit ? 2 : 1;
+  const bool sure = hit ? (s.rules & SIDE_NEAR) && o.far < 0.999998f * s.Rc : !(s.rules & SIDE_COUNT);
+  if (!sure) {
+    double bmn[D], bmx[D], qmn[D], qmx[D];
+    grain_box<D>(P, s.g, bmn, bmx);
+    grain_box<D>(P, gq, qmn, qmx);
+    if (!boxes_touch<D>(bmn, bmx, qmn, qmx, s.rad)) return 0;
+  }
+  return hit ? 2 : 1;
+}
+
+template <int D, bool REC, bool GC, bool PERM, bool LIST, int BPS, bool TEAM>
 __global__ void __launch_bounds__(128, BPS) k_force_mx(const Dev P) {
+  static_assert(LIST || !TEAM, "a team works on candidate lists");
   pdl_enter();
   pdl_release();
-  const uint32_t d = blockIdx.x * blockDim.x + threadIdx.x;
-  const uint32_t lane = threadIdx.x & 31;
+  // a warp a chunk, or (TEAM) a block of four warps, of which warp 0 holds the force and ends the step
+  const uint32_t lane = threadIdx.x & 31, sub = TEAM ? threadIdx.x >> 5 : 0u;
+  const uint32_t d = TEAM ? blockIdx.x * 32 + lane : blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t chunk = d >> 5;
   if (chunk >= P.n_chunks) return;
+  __shared__ TeamMem<D, TEAM> tm;
   const bool act = d < P.N;
   const uint32_t t = *P.step;
   const uint32_t g = act ? P.node_grain[d] : 0;
@@ -258,14 +556,84 @@ __global__ void __launch_bounds__(128, BPS) k_force_mx(const Dev P) {
   if (act) ldv<D>(P.vel_in, d, vpd);
   // per-node inputs of the epilogue: in 2D loaded up front so their latency hides behind the bond
   // loop; in 3D where they are used (the extra live registers spill there and measured slower)
+  // (a team's warp 0 has registers to spare and loads the position update's inputs here as well)
+  double dp[D], ps[D];
+  float db[D];
+  if constexpr (TEAM) {
+    if (act && sub == 0 && P.fuse) {
+      ldv<D>(P.disp, d, dp);
+      ldv<D>(P.pos, d, ps);
+      ldf<D>(P.disp_b, d, db);
+    }
+  }
   constexpr int DE = (D == 2) ? D : 1;
   float ef_in[DE], ao_in[DE];
   bool clamped_in = false;
   if constexpr (D == 2) {
-    if (mov) {
+    if (mov && sub == 0) {
       ldvf<D>(P.extf_f, d, ef_in);
       ldvf<D>(P.acc_f, d, ao_in);
       clamped_in = P.clamped[d] != 0;
+    }
+  }
+
+  const InstDev& in = P.inst[gr.inst];
+  // which contacts the node may have; a team looks before its bonds, a lone warp after them (its
+  // registers are full until then: 1.5 % of a step of the collision ensemble)
+  bool p_bdry, selfc, other;
+  uint32_t ncl;
+  auto rules = [&] {
+    p_bdry = !P.nl_bdry_only || (act && P.bdry_rank[d] != NONE);
+    selfc = mov && P.enable_fracture && (gr.flags & GF_BREAKABLE) && P.self_contact;
+    other = mov && (P.worm || (gr.flags & GF_STOPPABLE));
+    // with candidate lists a node whose list is empty has no contact this step
+    ncl = (LIST && act) ? (uint32_t)P.cand_n[d] : 0u;
+  };
+  if constexpr (TEAM) rules();
+  // a team's last warp notes each node's side of its contacts; its loads overlap the others' bonds
+  [[maybe_unused]] auto team_side = [&] {
+    if constexpr (TEAM) {
+      if (sub != TEAM_WARPS - 1 || !act) return;
+      Side<D>& s = tm.side[lane];
+      s.of(P, in, gr);
+      ldv<D>(P.cur, d, s.x);
+      for (int c = 0; c < D; ++c) s.v[c] = vpd[c];
+      ldf<D>(P.curf, d, s.pf);
+      s.pre2 = in.pre_f * in.pre_f;
+      s.g = g;
+      s.deg = P.node_deg[d];
+      s.w0 = P.chunk_word[chunk];
+      s.slot0 = P.chunk_slot[chunk] + lane;
+      s.lane = lane;
+      s.rules = (selfc ? SIDE_SELF : 0u) | (other ? SIDE_OTHER : 0u) | (ncl > P.max_cand ? SIDE_COUNT : 0u) | SIDE_NEAR;
+      for (int c = 0; c < D; ++c)
+        if (!(fabs(s.x[c]) < 1e9 * s.rad)) s.rules &= ~SIDE_NEAR;
+    }
+  };
+
+  // a team's contacts: every list entry of the chunk is a task, the entries of the 32 lists, end to
+  // end, over the block's threads; a thread's first entry q (of lane pl's list) is loaded ahead
+  uint32_t total = 0, incl = 0, first = 0, pl = 0, q = 0;
+  auto entry = [&](uint32_t e) {
+    pl = 0;  // as many lanes' lists end at or before e
+#pragma unroll
+    for (uint32_t s = 16; s; s >>= 1)
+      if (__shfl_sync(0xffffffffu, incl, pl + s - 1) <= e) pl += s;
+    const uint32_t at = e - __shfl_sync(0xffffffffu, first, pl);
+    if (e < total) q = P.cand_q[((size_t)chunk * P.cand_cap + at) * 32 + pl];
+  };
+  if constexpr (TEAM) {
+    const uint32_t n = (selfc || other) && p_bdry ? ncl : 0u;
+    if (__any_sync(0xffffffffu, n)) {
+      incl = n;
+#pragma unroll
+      for (int s = 1; s < 32; s <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, s);
+        if (lane >= (uint32_t)s) incl += v;
+      }
+      first = incl - n;
+      total = __shfl_sync(0xffffffffu, incl, 31);
+      entry(threadIdx.x);
     }
   }
 
@@ -283,8 +651,12 @@ __global__ void __launch_bounds__(128, BPS) k_force_mx(const Dev P) {
       ld_hl<D>(P.xref, P.np, d, xh, xl);
     }
     if constexpr (REC) {
-      if (mov && P.rec_df) st_hl<D>(P.rec_df, P.np, d, dh, dl);
+      if (mov && sub == 0 && P.rec_df) st_hl<D>(P.rec_df, P.np, d, dh, dl);
     }
+    if constexpr (TEAM) {
+      team_side();
+      team_bonds<D>(P, tm, d, lane, sub, cdeg, w0, slot0, mov, dh, dl, xh, xl, cnot, snot, t, f);
+    } else {
     // The alive words and neighbour indices are loaded two pairs ahead (they stream from memory, the
     // longest latency of the loop; one pair ahead took the collision ensemble's step from 59.6 to
     // 62.3 us and the 3D spheres' from 81.4 to 85.4), so only the neighbour gathers wait in an
@@ -327,9 +699,10 @@ __global__ void __launch_bounds__(128, BPS) k_force_mx(const Dev P) {
       ld_hl<D>(P.dref, P.np, jb, bdh, bdl);
       ld_hl<D>(P.xref, P.np, jb, bxh, bxl);
       const float va = P.vol_f[ja], vb = P.vol_f[jb];
-      float stra, strb;
-      bond_term<D>(dh, dl, xh, xl, adh, adl, axh, axl, cnot * va, ua, f, &stra);
-      bond_term<D>(dh, dl, xh, xl, bdh, bdl, bxh, bxl, cnot * vb, ub, f, &strb);
+      float stra, strb, ya[D], yb[D];
+      const float fa = bond_term<D>(dh, dl, xh, xl, adh, adl, axh, axl, cnot * va, ua, ya, &stra);
+      const float fb = bond_term<D>(dh, dl, xh, xl, bdh, bdl, bxh, bxl, cnot * vb, ub, yb, &strb);
+      for (int c = 0; c < D; ++c) f[c] = fmaf(fb, yb[c], fmaf(fa, ya[c], f[c]));
       // the alive words change only where a bond of the warp breaks: one vote a pair instead of two
       // ballots and two conditional stores (step times: collision ensemble 74.9 -> 72.5 us, settling
       // 23.7 -> 22.3, 3D spheres 104.4 -> 99.0, two disks 16.8 -> 15.8)
@@ -350,21 +723,55 @@ __global__ void __launch_bounds__(128, BPS) k_force_mx(const Dev P) {
         if (two && nb != wb) P.alive[w0 + k + 1] = nb;
       }
     }
+    }
   }
-  __syncwarp();
   __syncwarp();
 
   unsigned long long my_pairs = 0, my_hash = 0, my_close = 0;
   uint32_t rent[REC ? MAX_CAND : 1];  // recorded contact entries of this node (REC only)
   uint32_t nrec = 0, wbits = 0;
-  const InstDev& in = P.inst[gr.inst];
-  const bool p_bdry = !P.nl_bdry_only || (act && P.bdry_rank[d] != NONE);
-  const bool selfc = mov && P.enable_fracture && (gr.flags & GF_BREAKABLE) && P.self_contact;
-  const bool other = mov && (P.worm || (gr.flags & GF_STOPPABLE));
-
-  // with candidate lists a node whose list is empty has no contact this step
-  const uint32_t ncl = (LIST && act) ? (uint32_t)P.cand_n[d] : 0u;
-  if ((selfc || other) && p_bdry && (!LIST || ncl > 0)) {
+  if constexpr (!TEAM) rules();
+  // the contact of node q (o) as it acts on the force
+  auto apply = [&](uint32_t q, const ContactTerm<D>& o) {
+    if (P.record_pairs) {  // the pair log hashes input indices
+      my_pairs += 1;
+      my_hash += splitmix64(((unsigned long long)input_index<PERM>(P, d) << 32) | input_index<PERM>(P, q));
+    }
+    if (o.close) my_close += 1;
+    for (int c = 0; c < D; ++c) f[c] = fmaf(o.s1, o.u[c], f[c]);
+    if (P.allow_damping)
+      for (int c = 0; c < D; ++c) f[c] = fmaf(o.sd, o.u[c], f[c]);
+    if (o.fr)
+      for (int c = 0; c < D; ++c) f[c] = fmaf(o.sf, o.tg[c], f[c]);
+    if constexpr (REC) rent[nrec++] = q | (o.fr << 30);
+  };
+  if constexpr (TEAM) {
+    uint32_t passed = 0;
+    bool over = false;
+    for (uint32_t e0 = 0; e0 < total; e0 += 32 * TEAM_WARPS) {
+      if (e0) entry(e0 + threadIdx.x);
+      if (e0 + threadIdx.x < total) {
+        tm.what[threadIdx.x] = team_contact<D, GC>(P, tm.side[pl], chunk * 32 + pl, q, tm.term[threadIdx.x]);
+        tm.node[threadIdx.x] = q;
+      }
+      __syncthreads();
+      if (sub == 0) {
+        const uint32_t b = max(first, e0), e1 = min(incl, e0 + 32 * TEAM_WARPS);
+        for (uint32_t x = b; x < e1; ++x) {
+          const uint32_t w = tm.what[x - e0];
+          if (w == 0 || over) continue;
+          if (passed++ >= P.max_cand) {
+            set_status(P.status, PG_ECAPACITY);
+            over = true;
+          } else if (w == 2) {
+            apply(tm.node[x - e0], tm.term[x - e0]);
+          }
+        }
+      }
+      __syncthreads();
+    }
+    if (sub != 0) return;
+  } else if ((selfc || other) && p_bdry && (!LIST || ncl > 0)) {
     double bmn[D], bmx[D];
     grain_box<D>(P, g, bmn, bmx);
     float ph[D];
@@ -436,16 +843,18 @@ __global__ void __launch_bounds__(128, BPS) k_force_mx(const Dev P) {
           }
         }
     }
-    const uint32_t mydeg = P.node_deg[d];
-    // the pair log hashes input indices (the node's own looked up once; recorded runs only)
-    const unsigned long long od_hash = P.record_pairs ? ((unsigned long long)input_index<PERM>(P, d) << 32) : 0ull;
-    const float Kn0 = (float)in.normal_stiffness;
-    const float mu0 = (float)in.friction_coefficient, zeta0 = (float)in.damping_ratio;
-    const float rho = (float)gr.rho, dtf = (float)P.dt;
-    double xp64[D];
-    if (nc) ldv<D>(P.cur, d, xp64);
+    Side<D> s;
+    if (nc) {
+      s.of(P, in, gr);
+      ldv<D>(P.cur, d, s.x);
+      for (int c = 0; c < D; ++c) s.v[c] = vpd[c];
+      s.g = g;
+      s.deg = P.node_deg[d];
+      s.w0 = w0;
+      s.slot0 = slot0;
+      s.lane = lane;
+    }
     for (int ci = 0; ci < nc; ++ci) {
-      uint32_t q;
       if constexpr (LIST) {
         q = P.cand_q[cbase + (size_t)(__ffs(hits) - 1) * 32];
         hits &= hits - 1;
@@ -453,87 +862,9 @@ __global__ void __launch_bounds__(128, BPS) k_force_mx(const Dev P) {
         q = idx[ci];
       }
       const uint32_t gqi = P.node_grain[q];
-      const bool same = gqi == g;
-      // The contact decision |x_q - x_p| <= R_c' is made with the reference's FP64 arithmetic:
-      // contact damping switches on at full strength at that boundary, so a decision flipped by
-      // FP32 rounding would kick a node by metres per second.
-      double xq64[D], dir64[D];
-      ldv<D>(P.cur, q, xq64);
-      for (int c = 0; c < D; ++c) dir64[c] = xq64[c] - xp64[c];
-      double n2 = dir64[0] * dir64[0];
-      for (int c = 1; c < D; ++c) n2 = n2 + dir64[c] * dir64[c];
-      // dn64 <= R_c' <= contact_rad needs n2 <= contact_s_max (the same outcome as the sqrt
-      // test): candidates beyond it skip the square root and the bonded-neighbour scan
-      if (!(n2 <= in.contact_s_max)) continue;
-      const double dn64 = sqrt(n2);
-      double Rc64 = in.contact_rad;
-      float Kn = Kn0, zeta = zeta0, mu = mu0;
-      if constexpr (GC) {
-        const GrainDev& gq = P.grain[gqi];
-        Kn = (float)((gr.kn + gq.kn) * 0.5);
-        zeta = (float)((gr.zeta + gq.zeta) * 0.5);
-        mu = (float)((gr.mu + gq.mu) * 0.5);
-      }
-      if (same) {
-        bool bonded = false;
-        for (uint32_t k = 0; k < mydeg && !bonded; ++k) {
-          if (((P.alive[w0 + k] >> lane) & 1u) && P.bcol[slot0 + 32u * k] == q) bonded = true;
-        }
-        if (bonded) continue;
-        double pp[D], pq[D], r[D];
-        ldv<D>(P.pos, d, pp);
-        ldv<D>(P.pos, q, pq);
-        for (int c = 0; c < D; ++c) r[c] = pp[c] - pq[c];
-        double r2 = r[0] * r[0];
-        for (int c = 1; c < D; ++c) r2 = r2 + r[c] * r[c];
-        const double ref = sqrt(r2);
-        Rc64 = ref < in.contact_rad ? ref : in.contact_rad;
-        Kn = (float)(gr.cnot / Rc64);
-      }
-      if (!(dn64 <= Rc64)) continue;
-      const float Rc = (float)Rc64, dn = (float)dn64;
-      float dir[D];
-      for (int c = 0; c < D; ++c) dir[c] = (float)dir64[c];
-      if (P.record_pairs) {
-        my_pairs += 1;
-        my_hash += splitmix64(od_hash | input_index<PERM>(P, q));
-      }
-      if (dn == 0.f) my_close += 1;
-      const float inv = 1.f / dn;
-      float u[D];
-      for (int c = 0; c < D; ++c) u[c] = dir[c] * inv;
-      const float nvol = P.vol_f[q];
-      const float s1 = -Kn * (Rc - dn) * nvol;
-      for (int c = 0; c < D; ++c) f[c] = fmaf(s1, u[c], f[c]);
-      const float cfn = fabsf(s1);
-      uint32_t fr = 0;
-      if (P.allow_damping || P.allow_friction) {
-        double vqd[D];
-        ldv<D>(P.vel_in, q, vqd);
-        float rv[D];
-        for (int c = 0; c < D; ++c) rv[c] = (float)(vpd[c] - vqd[c]);
-        const float rvp = dotf<D>(rv, u);
-        if (P.allow_damping) {
-          const float dc = 2.f * zeta * sqrtf(Kn * rho) * sqrtf(nvol);
-          for (int c = 0; c < D; ++c) f[c] = fmaf(-dc * rvp, u[c], f[c]);
-        }
-        if (P.allow_friction) {
-          float tg[D];
-          for (int c = 0; c < D; ++c) tg[c] = fmaf(-rvp, u[c], rv[c]);
-          const float tn = sqrtf(dotf<D>(tg, tg));
-          if (tn > 0.f) {
-            float sfr = -mu * cfn;
-            fr = (D == 2 && (tg[1] * u[0] - tg[0] * u[1]) < 0.f) ? FR_SLIDE_NEG : FR_SLIDE;
-            if (tn < mu * cfn * dtf / rho) {
-              sfr = -tn / rho / dtf;
-              fr = FR_STICK;
-            }
-            const float it = sfr / tn;
-            for (int c = 0; c < D; ++c) f[c] = fmaf(it, tg[c], f[c]);
-          }
-        }
-      }
-      if constexpr (REC) rent[nrec++] = q | (fr << 30);
+      ContactTerm<D> o;
+      if (!contact_term<D, GC>(P, s, gqi, d, q, Partner<D>(P, q), o)) continue;
+      apply(q, o);
     }
   }
 
@@ -676,10 +1007,10 @@ __global__ void __launch_bounds__(128, BPS) k_force_mx(const Dev P) {
   }
 
   // velocity update (timeloop.h:834-863); with P.fuse the next step's position update too
-  double cu[D], dp[D];
+  double cu[D];
   for (int c = 0; c < D; ++c) cu[c] = 0.0;
   if (act) {
-    if (P.fuse) ldv<D>(P.disp, d, dp);
+    if (!TEAM && P.fuse) ldv<D>(P.disp, d, dp);
     if (mov) {
       float ao[D], a[D];
       double v[D];
@@ -715,10 +1046,10 @@ __global__ void __launch_bounds__(128, BPS) k_force_mx(const Dev P) {
       stv<D>(P.vel_out, d, vpd);
     }
     if (P.fuse) {
-      double ps[D];
-      float db[D];
-      ldv<D>(P.pos, d, ps);
-      ldf<D>(P.disp_b, d, db);
+      if constexpr (!TEAM) {
+        ldv<D>(P.pos, d, ps);
+        ldf<D>(P.disp_b, d, db);
+      }
       place_node_mx<D>(P, d, in, dp, ps, db, P.cur_n, P.curf_n, P.dref_n, P.rebuild_n, cu);
     } else {
       stvf<D>(P.force_f, d, f);
@@ -750,11 +1081,17 @@ __global__ void __launch_bounds__(128, BPS) k_force_mx(const Dev P) {
 
 // The force kernel's variants: mask recording (REC), per-grain contact parameters (GC), a node
 // layout other than the input order (PERM) and candidate lists or the grid search (LIST) are compiled
-// in only where used, so the plain kernel keeps its register budget; the plain kernel with lists
-// also for BPS = 5, 6 or 7 blocks of 128 threads per SM (96, 80 or 72 registers), see force_bps().
+// in only where used, so the plain kernel keeps its register budget; the plain kernel with lists also
+// for BPS = 5, 6 or 7 blocks of 128 threads per SM (96, 80 or 72 registers), see force_bps(), and each
+// with lists also for teams of warps (TEAM).
 template <int D>
-static const void* force_mx_ptr(bool rec, bool gc, bool perm, bool list, int bps) {
-#define PG_F(r, g, p, l, b) (const void*)k_force_mx<D, r, g, p, l, b>
+static const void* force_mx_ptr(bool rec, bool gc, bool perm, bool list, int bps, bool team) {
+#define PG_F(r, g, p, l, b) (const void*)k_force_mx<D, r, g, p, l, b, false>
+#define PG_T(r, g, p) (const void*)k_force_mx<D, r, g, p, true, 4, true>
+  static const void* const teams[8] = {PG_T(0, 0, 0), PG_T(0, 0, 1), PG_T(0, 1, 0), PG_T(0, 1, 1),
+                                       PG_T(1, 0, 0), PG_T(1, 0, 1), PG_T(1, 1, 0), PG_T(1, 1, 1)};
+  if (team) return teams[(rec ? 4 : 0) + (gc ? 2 : 0) + (perm ? 1 : 0)];
+#undef PG_T
   static const void* const plain[2][3] = {{PG_F(0, 0, 0, 1, 5), PG_F(0, 0, 0, 1, 6), PG_F(0, 0, 0, 1, 7)},
                                           {PG_F(0, 0, 1, 1, 5), PG_F(0, 0, 1, 1, 6), PG_F(0, 0, 1, 1, 7)}};
   static const void* const others[14] = {
@@ -766,10 +1103,11 @@ static const void* force_mx_ptr(bool rec, bool gc, bool perm, bool list, int bps
   return others[2 + (rec ? (gc ? 8 : 4) : 0) + (perm ? 2 : 0) + (list ? 1 : 0)];
 }
 template <int D>
-static void launch_force_mx(const Dev& P, dim3 grid, dim3 block, cudaStream_t s, bool pdl, bool rec) {
+static void launch_force_mx(const Dev& P, uint32_t block, cudaStream_t s, bool pdl, bool rec) {
   using K = void (*)(const Dev);
-  launch_k((K)force_mx_ptr<D>(rec, P.grain_contact, P.node_orig, P.cand_q, force_bps(P.n_chunks, P.n_sms)), grid, block,
-           0, s, pdl, P);
+  const bool team = force_team(P, block);
+  launch_k((K)force_mx_ptr<D>(rec, P.grain_contact, P.node_orig, P.cand_q, force_bps(P.n_chunks, P.n_sms), team),
+           team ? P.n_chunks : cdiv(P.n_chunks * 32, block), block, 0, s, pdl, P);
 }
 
 cudaError_t kernels_mixed_init() {
@@ -777,13 +1115,17 @@ cudaError_t kernels_mixed_init() {
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_finalize<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, FINAL_SMEM);
   if (e != cudaSuccess) return e;
   // the recording variants of the force kernel have local frames of about 1.1 KB
-  const void* fs[2 * 48];
+  const void* fs[2 * 48 + 2 * 8];
   int n = 0;
   for (int k = 0; k < 16; ++k)
     for (int b = 5; b <= 7; ++b) {
-      fs[n++] = force_mx_ptr<2>(k & 8, k & 4, k & 2, k & 1, b);
-      fs[n++] = force_mx_ptr<3>(k & 8, k & 4, k & 2, k & 1, b);
+      fs[n++] = force_mx_ptr<2>(k & 8, k & 4, k & 2, k & 1, b, false);
+      fs[n++] = force_mx_ptr<3>(k & 8, k & 4, k & 2, k & 1, b, false);
     }
+  for (int k = 0; k < 8; ++k) {
+    fs[n++] = force_mx_ptr<2>(k & 4, k & 2, k & 1, true, 5, true);
+    fs[n++] = force_mx_ptr<3>(k & 4, k & 2, k & 1, true, 5, true);
+  }
   size_t need = 0;
   e = max_local_bytes(fs, n, &need);
   return e == cudaSuccess ? ensure_local_bytes(need) : e;
@@ -803,8 +1145,7 @@ static void body_t(const Dev& P, const LaunchCfg& L, cudaStream_t s, uint64_t* l
     *launches += 1;
   }
   if (e0) cudaEventRecord(e0, s);
-  const dim3 grid(cdiv(P.n_chunks * 32, L.force_block)), block(L.force_block);
-  launch_force_mx<D>(P, grid, block, s, pdl, rec);
+  launch_force_mx<D>(P, L.force_block, s, pdl, rec);
   *launches += 1;
   if (e1) cudaEventRecord(e1, s);
 }
