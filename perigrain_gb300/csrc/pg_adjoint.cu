@@ -181,11 +181,13 @@ __global__ void __launch_bounds__(128) k_rp_force(const Dev P, const ReplayStep 
         const double dd = fmin(fabs(dist), Rr);
         double Area, I;
         if constexpr (D == 2) {
-          Area = M_PI * pow(Rr, 2.0) / 2 - pow(Rr, 2.0) * asin(dd / Rr) - sqrt(Rr * Rr - dd * dd) * dd;
-          I = 0.0 * pow((Rr * Rr - dd * dd), 1.5);
+          const double R2 = Rr * Rr, h2 = R2 - dd * dd;  // products for the reference's pow, as k_force
+          Area = M_PI * R2 / 2 - R2 * asin(dd / Rr) - sqrt(h2) * dd;
+          I = 0.0 * h2;
         } else {
-          Area = M_PI / 3 * pow((Rr - dd), 2.0) * (2 * Rr - dd);
-          I = M_PI / 4 * pow(pow(Rr, 2.0) - pow(dd, 2.0), 2.0);
+          const double a = Rr - dd, h2 = Rr * Rr - dd * dd;
+          Area = M_PI / 3 * (a * a) * (2 * Rr - dd);
+          I = M_PI / 4 * (h2 * h2);
         }
         const double centroid = I / Area;
         const double crc = Rr - centroid;
@@ -209,7 +211,7 @@ __global__ void __launch_bounds__(128) k_rp_force(const Dev P, const ReplayStep 
           } else {
             const int t1 = (dir + 1) % 3, t2 = (dir + 2) % 3;
             const double v1 = rv[t1], v2 = rv[t2];
-            const double vn = sqrt(pow(v1, 2.0) + pow(v2, 2.0));
+            const double vn = sqrt(v1 * v1 + v2 * v2);
             if (vn > 0) {
               const double u1 = v1 / vn, u2 = v2 / vn;
               double ff1 = ((-mu) * fabs(F)) * u1;

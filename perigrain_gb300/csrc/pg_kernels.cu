@@ -472,13 +472,19 @@ __global__ void __launch_bounds__(128, BPS) k_force(const Dev P) {
         // segment_mass<dim>(R, d) (contact.h:16-41)
         double Area, I;
         if constexpr (D == 2) {
-          Area = M_PI * pow(R, 2.0) / 2 - pow(R, 2.0) * asin(dd / R) - sqrt(R * R - dd * dd) * dd;
-          I = 0.0 * pow((R * R - dd * dd), 1.5);  // 2 / 3 is integer division in the reference
+          // The reference's pow(x, 2.0) as products (the correctly rounded square): pow takes 6100
+          // cycles in a chain, and a node at a wall called it three times. Roots and quotients on the
+          // integer pipe. A chunk at a wall: 24000 -> 12000 cycles, the 500-grain compaction's step
+          // 41.9 -> 33.9 us.
+          const double R2 = R * R, h2 = R2 - dd * dd;
+          Area = M_PI * R2 / 2 - R2 * asin(ieee64::div_rn(dd, R)) - ieee64::sqrt_rn(h2) * dd;
+          I = 0.0 * h2;  // 0 * pow(h2, 1.5): 2 / 3 is integer division in the reference
         } else {
-          Area = M_PI / 3 * pow((R - dd), 2.0) * (2 * R - dd);
-          I = M_PI / 4 * pow(pow(R, 2.0) - pow(dd, 2.0), 2.0);
+          const double a = R - dd, h2 = R * R - dd * dd;
+          Area = M_PI / 3 * (a * a) * (2 * R - dd);
+          I = M_PI / 4 * (h2 * h2);
         }
-        const double centroid = I / Area;
+        const double centroid = ieee64::div_rn(I, Area);
         const double crc = R - centroid;
         const double pcrc = crc > 0 ? crc : 0;
         const double F = (Knw * pcrc) * Area;
@@ -505,8 +511,8 @@ __global__ void __launch_bounds__(128, BPS) k_force(const Dev P) {
               const double vts = rv[tg] > 0 ? 1 : -1;
               double ff = ((-mu) * fabs(F)) * vts;
               wbits |= (rv[tg] > 0 ? 2u : 10u) << (4 * k);
-              if (fabs(rv[tg]) < (((mu * fabs(F)) * P.dt) / gr.rho)) {
-                ff = ((-rv[tg]) * gr.rho) / P.dt;
+              if (fabs(rv[tg]) < ieee64::div_rn((mu * fabs(F)) * P.dt, gr.rho)) {
+                ff = ieee64::div_rn((-rv[tg]) * gr.rho, P.dt);
                 wbits |= 4u << (4 * k);
               }
               f[tg] = f[tg] + ff;
@@ -516,7 +522,7 @@ __global__ void __launch_bounds__(128, BPS) k_force(const Dev P) {
           } else {
             const int t1 = (dir + 1) % 3, t2 = (dir + 2) % 3;
             const double v1 = rv[t1], v2 = rv[t2];
-            const double vn = sqrt(pow(v1, 2.0) + pow(v2, 2.0));
+            const double vn = ieee64::sqrt_rn(v1 * v1 + v2 * v2);
             if (vn > 0) {
               const double u1 = v1 / vn, u2 = v2 / vn;
               double ff1 = ((-mu) * fabs(F)) * u1;
@@ -536,7 +542,7 @@ __global__ void __launch_bounds__(128, BPS) k_force(const Dev P) {
           }
         }
         if (P.allow_damping) {
-          const double dc = ((2.0 * zetaw) * sqrt(Knw * gr.rho)) * sqrt(fabs(Area));
+          const double dc = ((2.0 * zetaw) * ieee64::sqrt_rn(Knw * gr.rho)) * ieee64::sqrt_rn(fabs(Area));
           const double df = (-dc) * rv[dir];
           f[dir] = f[dir] + df;
           rec.a_damp = vol_i * df;
