@@ -11,10 +11,12 @@
 //   * the alive set is one 32-bit word per (chunk, k): bit `lane` is bond k of that lane, so a
 //     warp reads its alive bits with one broadcast load and writes them back with one ballot;
 //   * the contact grid is a dense row-major uniform grid per instance (cell >= 1.0625 R_c), refitted
-//     on the device every step to the instance's bounding box (plus two cells) and rebuilt by a
-//     counting sort of the nodes by cell (one radix digit spanning all cells), whose exclusive scan
-//     doubles as the cell-start table. Cell coordinates are clamped to the grid, so a node that
-//     moves outside the box still lands in an edge cell and every pair within R_c is still found.
+//     on the device to the instance's bounding box (plus two cells): with candidate lists when they
+//     are rebuilt, a cell's nodes as a chain (cell_start its head, cell_rank the next node); without
+//     lists every step, by a counting sort of the nodes by cell (one radix digit spanning all cells),
+//     whose exclusive scan doubles as the cell-start table. Cell coordinates are clamped to the grid,
+//     so a node that moves outside the box still lands in an edge cell and every pair within R_c is
+//     still found.
 #pragma once
 #include <vector_types.h>
 
