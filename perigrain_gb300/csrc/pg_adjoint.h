@@ -37,9 +37,14 @@ struct AdjStep {
   double* xbb;                       // [N][S] bond share of the position cotangent (scratch)
   double* pcb;                       // [N] bond share of the cnot cotangent (scratch)
   // FP32 bond path (mixed-precision handles; null = FP64 bond path): the step's displacement
-  // hi/lo pairs and the FP32 force cotangents (read for step t, rewritten for step t-1)
+  // hi/lo pairs and the FP32 force cotangents (fbf: of step t, fbf_o: of step t-1)
   const float* df;
-  float* fbf;
+  const float* fbf;
+  float* fbf_o;
+  // the contact blocks' sums of a chunk [n_chunks][2D + NPARAM][32] and its ticket [n_chunks], 0
+  // between steps
+  double* rest;
+  uint32_t* ticket;
 };
 
 // One FP64 forward step under frozen masks (the map the adjoint differentiates).
@@ -56,7 +61,7 @@ struct ReplayStep {
 
 void launch_replay_step(const Dev& P, const ReplayStep& R, cudaStream_t s, uint64_t* launches);
 void launch_adjoint_step(const Dev& P, const AdjStep& A, cudaStream_t s, uint64_t* launches);
-// fbf from the seed cotangent (A.ab, A.vb) before the first reverse step of the FP32 bond path
+// fbf_o from the seed cotangent (A.ab, A.vb) before the first reverse step of the FP32 bond path
 void launch_fb_init(const Dev& P, const AdjStep& A, cudaStream_t s, uint64_t* launches);
 // grad[g][k] = sum over the nodes of grain g of pacc[node][k]
 void launch_grad_reduce(const Dev& P, const double* pacc, double* grad, cudaStream_t s, uint64_t* launches);

@@ -11,13 +11,13 @@
 // its nodes (a node reads its own contact list and finds itself in each partner's list), so the
 // step is atomic-free and deterministic.
 //
-// Two kernels per reverse step. k_adj_bonds: one block per 32-node SELL chunk, SUB warps per
-// block, warp w taking the node's bond slots k = w, w+SUB, ... (one coalesced access per warp and
+// One kernel per reverse step, two blocks per 32-node SELL chunk. Bonds: SUB warps per block, warp w
+// taking the node's bond slots k = w, w+SUB, ... (one coalesced access per warp and
 // slot, as in the force kernels), partial sums added in shared memory in a fixed order; its bond
 // products run in FP32 for mixed-precision handles (GB300 runs FP64 at a small fraction of its
 // FP32 rate) and in FP64 for FP64 handles and frozen replays (the FP64 reference gradient).
-// k_adj_rest: same chunk x SUB-warp split for contacts (entries round-robin over the warps),
-// walls and the integrator, FP64; the cotangent state is FP64 throughout.
+// Contacts and walls: tasks over the block's threads, FP64. The later of the two blocks runs the
+// integrator; the cotangent state is FP64 throughout.
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -31,6 +31,9 @@
 namespace pg {
 
 constexpr int SUB = 4;
+// Cotangents a chunk's contact block adds up per node: xb[D], vfb[D], pc[NPARAM].
+template <int D>
+constexpr int ADJ_NV = 2 * D + NPARAM;
 
 // Adjoint of one node-node contact force phi(y, r) received by a node of density rho from a
 // partner of volume vq; y = x_partner - x_node, r = v_node - v_partner, g = cotangent of phi.
@@ -185,11 +188,8 @@ __device__ __forceinline__ void stfv(float* a, uint32_t i, const float (&v)[D]) 
 // the displacement difference from the tape's hi/lo pairs, the cancellation-free stretch
 // s = (2 xi.et + et.et) / (|xi| (|xi + et| + |xi|)), force cotangents from the FP32 array fbf.
 template <int D, bool F32>
-__global__ void __launch_bounds__(32 * SUB) k_adj_bonds(const Dev P, const AdjStep A) {
-  pdl_enter();
-  __shared__ double red[SUB][D + 1][32];
+__device__ __forceinline__ void adj_bonds(const Dev& P, const AdjStep& A, uint32_t chunk, double (*red)[D + 1][32]) {
   const uint32_t lane = threadIdx.x & 31, sub = threadIdx.x >> 5;
-  const uint32_t chunk = blockIdx.x;
   const uint32_t d = chunk * 32 + lane;
   const bool act = d < P.N;
   double part[D + 1];
@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(32 * SUB) k_adj_bonds(const Dev P, const AdjSt
   // fixed-order sum of the SUB partial cotangents
   for (int v = 0; v <= D; ++v) red[sub][v][lane] = part[v];
   __syncthreads();
-  if (sub != 0 || !act) return;
+  if (sub != 0) return;
   double out[D];
   for (int c = 0; c < D; ++c) {
     double s = red[0][c][lane];
@@ -291,21 +291,22 @@ __global__ void __launch_bounds__(32 * SUB) k_adj_bonds(const Dev P, const AdjSt
   }
   double pcs = red[0][D][lane];
   for (int w = 1; w < SUB; ++w) pcs += red[w][D][lane];
-  stv<D>(A.xbb, d, out);
-  A.pcb[d] = pcs;
+  if (act) {
+    stv<D>(A.xbb, d, out);
+    A.pcb[d] = pcs;
+  }
 }
 
-// Contact, wall and integrator part of the reverse step, one block per 32-node chunk. A contact of a
+// Contact and wall part of the reverse step, one block per 32-node chunk. A contact of a
 // pair acts on the node through two forces, its own and its partner's, and each is a task of a few
 // hundred dependent FP64 operations. The chunk's tasks are laid out over the block's threads, 64
 // entries of the nodes' lists a round with the own forces on warps 0 and 1 and the partners' on 2 and
 // 3, so a chunk with contacts takes one such chain where a lane a node took two for every SUB
 // entries of its node. The walls are a chain of their own, on a warp that mostly has no task. The
-// node lanes add the results in a fixed order, warp w the entries i = w, w+SUB, ...; warp 0 adds the
-// warps' sums and the bond share from k_adj_bonds and runs the integrator. For the FP32 bond path it
-// also writes the force cotangent of the next reverse step to fbf. Bound by that latency: 592 chunks
-// are one wave of one or two active warps a block; 20k nodes in 50 grains, us: 21.6 -> 13.7 (about 5 with
-// neither contacts nor walls).
+// node lanes add the results in a fixed order, warp w the entries i = w, w+SUB, ..., then warp 0 the
+// warps' sums. Bound by that latency: 592 chunks are one wave of one or two active warps a block;
+// 20k nodes in 50 grains, us, with the integrator and as a kernel of its own: 21.6 -> 13.7 (about 5
+// with neither contacts nor walls).
 constexpr uint32_t ADJ_ENTRIES = 16 * SUB;  // entries of a round
 
 // The contact tasks of entry e of node p (grain g, force cotangent Fb): its own force, or the
@@ -366,14 +367,11 @@ __device__ __forceinline__ void contact_task(const Dev& P, const AdjStep& A, uin
 }
 
 template <int D>
-__global__ void __launch_bounds__(32 * SUB, D == 2 ? 4 : 3) k_adj_rest(const Dev P, const AdjStep A) {
-  pdl_enter();
-  constexpr int NS = 2 * D;
-  constexpr int NV = 2 * D + NPARAM;  // xb[D], vfb[D], pc[NPARAM]
-  __shared__ double red[SUB][NV][32];
-  __shared__ double res[NV][32 * SUB];
+__device__ __forceinline__ void adj_contacts(const Dev& P, const AdjStep& A, uint32_t chunk,
+                                             double (*red)[ADJ_NV<D>][32], double (*res)[32 * SUB]) {
+  constexpr int NS = 2 * D, NV = ADJ_NV<D>;
   const uint32_t lane = threadIdx.x & 31, sub = threadIdx.x >> 5;
-  const uint32_t d = blockIdx.x * 32 + lane;
+  const uint32_t d = chunk * 32 + lane;
   const bool act = d < P.N;
   double acc[NV];
   for (int v = 0; v < NV; ++v) acc[v] = 0.0;
@@ -497,7 +495,7 @@ __global__ void __launch_bounds__(32 * SUB, D == 2 ? 4 : 3) k_adj_rest(const Dev
       double out[NV];
 #pragma unroll
       for (int v = 0; v < NV; ++v) out[v] = 0.0;
-      contact_task<D>(P, A, blockIdx.x * 32 + pl, gp, Fp, A.ent[at], partner, out);
+      contact_task<D>(P, A, chunk * 32 + pl, gp, Fp, A.ent[at], partner, out);
 #pragma unroll
       for (int v = 0; v < NV; ++v) res[v][threadIdx.x] = out[v];
     }
@@ -514,37 +512,52 @@ __global__ void __launch_bounds__(32 * SUB, D == 2 ? 4 : 3) k_adj_rest(const Dev
     __syncthreads();
   }
 
-  // fixed-order sum of the SUB partial cotangents, then the integrator (warp 0)
+  // fixed-order sum of the SUB partial cotangents (warp 0)
   if (pairs) {
     for (int v = 0; v < NV; ++v) red[sub][v][lane] = acc[v];
     __syncthreads();
   }
-  if (sub != 0 || !act) return;
-  if (!live) {
-    // the state of this node does not depend on the parameters
-    double zero[D];
-    for (int c = 0; c < D; ++c) zero[c] = 0.0;
-    stv<D>(A.db_o, d, zero);
-    stv<D>(A.vb_o, d, zero);
-    stv<D>(A.ab_o, d, zero);
-    if (A.fbf) {
-      float zf[D];
-      for (int c = 0; c < D; ++c) zf[c] = 0.f;
-      stfv<D>(A.fbf, d, zf);
-    }
-    return;
-  }
+  if (sub != 0) return;
   if (pairs)
     for (int v = 0; v < NV; ++v) {
       double sm = red[0][v][lane];
       for (int w = 1; w < SUB; ++w) sm += red[w][v][lane];
       acc[v] = sm;
     }
-  double xbond[D];
-  ldv<D>(A.xbb, d, xbond);
-  for (int c = 0; c < D; ++c) xb[c] += xbond[c];
-  pc[0] += A.pcb[d];
-  const GrainDev& gr = P.grain[g];
+  double* rs = A.rest + (size_t)chunk * NV * 32 + lane;
+  for (int v = 0; v < NV; ++v) rs[32 * v] = acc[v];
+}
+
+// The end of a reverse step for a chunk (one warp): both shares are there.
+template <int D>
+__device__ __forceinline__ void adj_finish(const Dev& P, const AdjStep& A, uint32_t chunk) {
+  constexpr int NV = ADJ_NV<D>;
+  const uint32_t lane = threadIdx.x & 31, d = chunk * 32 + lane;
+  if (d >= P.N) return;
+  const GrainDev& gr = P.grain[P.node_grain[d]];
+  if (!(gr.flags & GF_MOVABLE) || P.clamped[d]) {
+    // the state of this node does not depend on the parameters
+    double zero[D];
+    for (int c = 0; c < D; ++c) zero[c] = 0.0;
+    stv<D>(A.db_o, d, zero);
+    stv<D>(A.vb_o, d, zero);
+    stv<D>(A.ab_o, d, zero);
+    if (A.fbf_o) {
+      float zf[D];
+      for (int c = 0; c < D; ++c) zf[c] = 0.f;
+      stfv<D>(A.fbf_o, d, zf);
+    }
+    return;
+  }
+  const double* rs = A.rest + (size_t)chunk * NV * 32 + lane;
+  double acc[NV];
+  for (int v = 0; v < NV; ++v) acc[v] = __ldcg(rs + 32 * v);
+  double* xb = acc;
+  double* vfb = acc + D;
+  double* pc = acc + 2 * D;
+  const double* xbond = A.xbb + (size_t)d * (D == 2 ? 2 : 4);
+  for (int c = 0; c < D; ++c) xb[c] += __ldcg(xbond + c);
+  pc[0] += __ldcg(A.pcb + d);
 
   // integrator
   double db[D], vb[D], o1[D], o2[D], o3[D];
@@ -559,14 +572,44 @@ __global__ void __launch_bounds__(32 * SUB, D == 2 ? 4 : 3) k_adj_rest(const Dev
   stv<D>(A.db_o, d, o1);
   stv<D>(A.vb_o, d, o2);
   stv<D>(A.ab_o, d, o3);
-  if (A.fbf) {
-    // force cotangent of the previous step, for the FP32 bond kernel of the next reverse step
+  if (A.fbf_o) {
+    // force cotangent of the previous step, for the FP32 bond products of the next reverse step
     float nf[D];
     for (int c = 0; c < D; ++c) nf[c] = (float)(gr.one_over_rho * (o3[c] + P.half_dt * o2[c]));
-    stfv<D>(A.fbf, d, nf);
+    stfv<D>(A.fbf_o, d, nf);
   }
   double* pa = A.pacc + (size_t)d * NPARAM;
   for (int k = 0; k < NPARAM; ++k) pa[k] += pc[k];
+}
+
+// A reverse step: two blocks a chunk, the contacts and walls of all chunks first (the longer chains),
+// then the bonds, which run beside them. Each writes its share; the one that comes second (a ticket a
+// chunk, back at 0 when the step ends) runs the integrator. Nothing waits. In 2D 5 blocks per SM (96
+// registers), so that bond blocks are resident beside a wave of contact blocks. 592 chunks, 300 steps
+// forward, recomputed and reversed, ms: two kernels 15.8; one, at 4 / 5 / 6 / 8 blocks per SM
+// 15.1 / 14.0 / 14.2 / 14.5.
+template <int D, bool F32>
+__global__ void __launch_bounds__(32 * SUB, D == 2 ? 5 : 3) k_adj_step(const Dev P, const AdjStep A) {
+  pdl_enter();
+  constexpr int NV = ADJ_NV<D>;
+  __shared__ double red[SUB][NV][32];
+  __shared__ double res[NV][32 * SUB];
+  const bool bonds = blockIdx.x >= P.n_chunks;
+  const uint32_t chunk = bonds ? blockIdx.x - P.n_chunks : blockIdx.x;
+  if (bonds) {
+    adj_bonds<D, F32>(P, A, chunk, reinterpret_cast<double(*)[D + 1][32]>(&red[0][0][0]));
+  } else {
+    adj_contacts<D>(P, A, chunk, red, res);
+  }
+  if (threadIdx.x >= 32) return;
+  __threadfence();
+  __syncwarp();
+  uint32_t other = 0;
+  if (threadIdx.x == 0) other = atomicAdd(&A.ticket[chunk], 1u);
+  if (!__shfl_sync(0xffffffffu, other, 0)) return;
+  if (threadIdx.x == 0) A.ticket[chunk] = 0;
+  __threadfence();
+  adj_finish<D>(P, A, chunk);
 }
 
 // force cotangents of the first reverse step from the seed cotangent (FP32 bond path)
@@ -579,7 +622,7 @@ __global__ void k_fb_init(const Dev P, const AdjStep A) {
   force_bar<D>(P, A, d, Fb);
   float f[D];
   for (int c = 0; c < D; ++c) f[c] = (float)Fb[c];
-  stfv<D>(A.fbf, d, f);
+  stfv<D>(A.fbf_o, d, f);
 }
 
 // per-grain sums of the per-node parameter cotangents, one block per grain, fixed order
@@ -604,17 +647,13 @@ __global__ void __launch_bounds__(256) k_grad_reduce(const Dev P, const double* 
 
 void launch_adjoint_step(const Dev& P, const AdjStep& A, cudaStream_t s, uint64_t* launches) {
   // programmatic dependent launch: each kernel waits on its predecessor in pdl_enter()
-  const dim3 g(P.n_chunks), b(32 * SUB);
+  const dim3 g(2 * P.n_chunks), b(32 * SUB);
   if (P.dim == 2) {
-    if (A.fbf) launch_k(k_adj_bonds<2, true>, g, b, 0, s, true, P, A);
-    else launch_k(k_adj_bonds<2, false>, g, b, 0, s, true, P, A);
-    launch_k(k_adj_rest<2>, g, b, 0, s, true, P, A);
+    launch_k(A.fbf ? k_adj_step<2, true> : k_adj_step<2, false>, g, b, 0, s, true, P, A);
   } else {
-    if (A.fbf) launch_k(k_adj_bonds<3, true>, g, b, 0, s, true, P, A);
-    else launch_k(k_adj_bonds<3, false>, g, b, 0, s, true, P, A);
-    launch_k(k_adj_rest<3>, g, b, 0, s, true, P, A);
+    launch_k(A.fbf ? k_adj_step<3, true> : k_adj_step<3, false>, g, b, 0, s, true, P, A);
   }
-  *launches += 2;
+  *launches += 1;
 }
 
 void launch_fb_init(const Dev& P, const AdjStep& A, cudaStream_t s, uint64_t* launches) {

@@ -248,6 +248,9 @@ static int enqueue_recompute(pg_handle* h, int parity, uint32_t len, uint32_t fi
   return PG_OK;
 }
 
+// FP32 force cotangents of one cotangent slot.
+static size_t fbf_floats(const pg_handle* h) { return (size_t)h->P.N * (h->dim == 2 ? 2 : 4); }
+
 // Reverse steps over tape slots len-1..0; cotangents move cot[cur] -> cot[cur^1] each step.
 static void enqueue_reverse(pg_handle* h, int cur, uint32_t len, uint32_t first_idx, bool with_rbar,
                             uint64_t* launches) {
@@ -287,7 +290,10 @@ static void enqueue_reverse(pg_handle* h, int cur, uint32_t len, uint32_t first_
     A.pcb = G->pcb;
     const bool f32 = h->precision == PG_MIXED && !G->frozen;
     A.df = f32 ? G->DF + (size_t)ii * df_floats(h) : nullptr;
-    A.fbf = f32 ? G->fbf : nullptr;
+    A.fbf = f32 ? G->fbf + cur * fbf_floats(h) : nullptr;
+    A.fbf_o = f32 ? G->fbf + (cur ^ 1) * fbf_floats(h) : nullptr;
+    A.rest = G->rest;
+    A.ticket = G->ticket;
     launch_adjoint_step(h->P, A, h->stream, launches);
     cur ^= 1;
   }
@@ -526,7 +532,11 @@ int pg_grad_backward(pg_handle* h, const double* disp_bar, const double* vel_bar
     CU(G->mem.alloc(&G->rbar, I * NS * D));
     CU(G->mem.alloc(&G->xbb, N * S));
     CU(G->mem.alloc(&G->pcb, N));
-    CU(G->mem.alloc(&G->fbf, N * ((D == 2) ? 2 : 4)));
+    CU(G->mem.alloc(&G->fbf, 2 * fbf_floats(h)));
+    const uint32_t NC = h->P.n_chunks;
+    CU(G->mem.alloc(&G->rest, (size_t)NC * 32 * (2 * D + NPARAM)));
+    CU(G->mem.alloc(&G->ticket, NC));
+    CU(cudaMemsetAsync(G->ticket, 0, NC * sizeof(uint32_t), h->stream));
   }
   uint64_t cap = G->ent_cap ? G->ent_cap : std::max<uint64_t>(1u << 20, (uint64_t)C * N / 2);
   std::vector<uint32_t> need(nseg, 0);
@@ -559,7 +569,7 @@ int pg_grad_backward(pg_handle* h, const double* disp_bar, const double* vel_bar
       AdjStep A{};
       A.ab = G->cot[0][2];
       A.vb = G->cot[0][1];
-      A.fbf = G->fbf;
+      A.fbf_o = G->fbf;
       launch_fb_init(h->P, A, h->stream, &launches);
     }
     int cur = 0;

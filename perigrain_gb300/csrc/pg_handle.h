@@ -87,7 +87,9 @@ struct GradState {
   double* cot[2][3] = {{nullptr, nullptr, nullptr}, {nullptr, nullptr, nullptr}};
   double *pacc = nullptr, *gradd = nullptr, *rbar = nullptr, *wall_out = nullptr;
   double *xbb = nullptr, *pcb = nullptr;
-  float* fbf = nullptr;
+  float* fbf = nullptr;         // one per cotangent slot
+  double* rest = nullptr;       // AdjStep::rest, ::ticket
+  uint32_t* ticket = nullptr;
   // graphs of one full segment: recording (per velocity parity) and reverse (per cotangent slot)
   cudaGraphExec_t g_rec[2] = {nullptr, nullptr};
   cudaGraphExec_t g_adj[2] = {nullptr, nullptr};
