@@ -257,3 +257,28 @@ def test_full_compaction_gradient_at_its_horizon():
             assert abs(fd - ref[gi, a]) <= HORIZON_TOL * scale, (h, gi, a, fd, ref[gi, a])
     m.close()
     sim.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_gradient_with_more_contacts_in_a_chunk_than_a_round_takes(precision):
+    """The reverse step takes a chunk's contact entries 64 a round. In input order the grains' sides
+    fill chunks with more than a round of entries; a shuffled layout spreads the same contacts over all
+    chunks. A node's terms are summed in the order of its own list either way, and the parameters in
+    input order, so the gradients agree to FP64 rounding of their sums."""
+    s = _case(n_grains=4, nodes=120, seed=17)
+    s.contact_radius *= 5
+    pos = np.asarray(s.pos).reshape(s.n_nodes, s.dim)
+    grain = np.repeat(np.arange(s.n_grains), np.diff(s.grain_node_offset.astype(np.int64)))
+    near = np.linalg.norm(pos[:, None] - pos[None], axis=2) <= float(s.contact_radius[0])
+    entries = (near & (grain[:, None] != grain[None])).sum(1)
+    assert np.add.reduceat(entries, np.arange(0, s.n_nodes, 32)).max() > 64
+    rbar = np.random.default_rng(18).uniform(-1, 1, (s.n_instances, 2 * s.dim, s.dim))
+    grads = []
+    for order in ("input", "shuffle"):
+        sim = Simulation(s, dt=2e-8, enable_fracture=1, allow_damping=1, allow_friction=1, self_contact=1,
+                         precision=precision, contact_skin=0.0, node_order=order)
+        run = grad.GradRun(sim, 20, checkpoint_every=20)
+        run.forward()
+        grads.append(run.backward(reaction_bar=rbar, ke_bar=np.ones(s.n_instances)))
+    assert np.abs(grads[0]).max() > 0
+    assert np.abs(grads[0] - grads[1]).max() <= 1e-12 * np.abs(grads[0]).max()
