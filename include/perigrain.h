@@ -115,7 +115,8 @@ typedef struct pg_config {
   uint32_t pair_log_capacity; /* steps kept in the pair log ring (default 1024 when 0) */
   uint32_t first_step;     /* t of the first step taken (1, or resume_ind*modulo + 1) */
   uint32_t max_contacts;   /* per-node contact candidate capacity (default 48 when 0) */
-  uint32_t block_size;     /* threads per block of the fused force kernel (0: default 128) */
+  uint32_t block_size;     /* threads per block of the fused force kernel (0: default 128, with which a
+                              mixed handle of few nodes puts four warps on 32 nodes; same results) */
   int32_t autotune;        /* 1: pick block_size, cells_per_node and contact_skin by timing trial runs */
   uint32_t cells_per_node; /* contact-grid capacity per node (0: 4 in 2D, 8 in 3D) */
   double contact_skin;     /* > 0: keep per-node contact candidate lists built with radius
