@@ -844,6 +844,10 @@ __global__ void __launch_bounds__(MM_T) k_pack_ascent(const PackMeshDev P, const
   if (node) load_problem<PK, PL, NW>(P, i, M, &x0, &y0, &L);
   __syncwarp();
   const double fx = mm_ascent<PK, PL, NW>(M, node, &x, &y, &step);
+  // Launched programmatically, this grid may end before the classes launched ahead of it. What follows
+  // the last class on the stream needs all of them, so a grid does not complete before its predecessor
+  // has: one block waits for it (all of them would hold their places on the SMs meanwhile).
+  if (blockIdx.x == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
   if (!node) return;
   double2* o = reinterpret_cast<double2*>(asc) + 2 * (size_t)rank[i];
   o[0] = make_double2(x, y);
@@ -1029,7 +1033,8 @@ extern "C" int pg_pack_incenters(const pg_pack_mesh* m, int32_t modify_nodal_cir
       const PackMeshDev Q = {m->pos, centers, radii, off, adj, mask, bcnt, bedge, m->bdry_edges};
       // A warp of the ascent runs for about two milliseconds, so the classes run into one another: each
       // launch lets the next one's blocks in as its last ones start (the classes share no data; they
-      // all read what was complete before the first began): 13.4 -> 12.1 ms for 800 x 500 cells
+      // all read what was complete before the first began) and completes after it (k_pack_ascent):
+      // 13.4 -> 12.1 ms for 800 x 500 cells
       const bool few = nodes <= MM_FEW;
       bool first = true;
       auto ascent = [&](int k, auto* many_kernel, auto* few_kernel) {
