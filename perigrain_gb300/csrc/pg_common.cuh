@@ -372,6 +372,15 @@ __device__ __forceinline__ bool within_interior(const double (&mn)[D], const dou
   return (W[0] < AL) & (AR < W[1]) & (W[2] > AT) & (W[3] < AB);
 }
 
+// Nodes of a row of cells that the grid search of a handle without candidate lists takes at a time, so
+// that their positions are waited for together: the search is one chain of loads a node, and where the
+// grid is coarse (a sparse box, debris) it is most of a step. Same order, same bits. Mixed, ms per 100
+// steps at 1 (with the next index loaded ahead) / 2 / 3 / 4: 40 settling grains 3.93 / 3.15 / 2.59 / 2.44,
+// 60 3D spheres 13.1 / 10.1 / 10.0 / 10.0, 200 pairs 4.71 / 4.25 / 4.24 / 4.22, two disks 2.47 / 2.36 /
+// 2.36 / 2.35; FP64 two disks burst apart 55.1 / 49.2 / 41.5 / 37.5. At 1 and with the grain read before
+// the prefilter the small ones of these had fallen behind a search in the kernel without lists.
+constexpr uint32_t CELL_BATCH = 4;
+
 template <int D>
 __device__ __forceinline__ void insert_cand(unsigned long long (&keys)[MAX_CAND], uint32_t (&idx)[MAX_CAND],
                                             int& n, unsigned long long key, uint32_t q, const Dev& P) {

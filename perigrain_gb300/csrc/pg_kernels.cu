@@ -285,20 +285,19 @@ __global__ void __launch_bounds__(128, BPS) k_force(const Dev P) {
     float pf[D];
     ldf<D>(P.curf, d, pf);
     const float thr2 = in.pre_f * in.pre_f;
-    // does candidate q pass the FP32 prefilter, the contact rules and the grain-box test? (the box
-    // test of the grain asked about last is kept: a list is sorted by grain)
+    // is candidate q beyond the FP32 prefilter; is it within the contact rules and the grain-box test?
+    // (the box test of the grain asked about last is kept: a list is sorted by grain)
     uint32_t box_g = NONE;
     bool box_ok = false;
-    auto passes = [&](uint32_t q) {
-      float qf[D];
-      ldf<D>(P.curf, q, qf);
-      const uint32_t gq = P.node_grain[q];  // issued with the position, used after the prefilter
+    auto far = [&](const float (&qf)[D]) {
       float d2 = 0.f;
       for (int c = 0; c < D; ++c) {
         float dd = qf[c] - pf[c];
         d2 += dd * dd;
       }
-      if (d2 > thr2) return false;
+      return d2 > thr2;
+    };
+    auto allowed = [&](uint32_t q, uint32_t gq) {
       const bool same = (gq == g);
       if (same ? !selfc : !other) return false;
       if (P.nl_bdry_only && P.bdry_rank[q] == NONE) return false;
@@ -316,13 +315,17 @@ __global__ void __launch_bounds__(128, BPS) k_force(const Dev P) {
     const size_t cbase = (size_t)chunk * P.cand_cap * 32 + lane;
     uint32_t hits = 0;
     uint32_t idx[LIST ? 1 : MAX_CAND];
+    unsigned long long keys[LIST ? 1 : MAX_CAND];
     int nc = 0;
     if constexpr (LIST) {
       uint32_t qn = P.cand_q[cbase];  // the next entry is loaded one candidate ahead
       for (uint32_t k = 0; k < ncl; ++k) {
         const uint32_t q = qn;
         if (k + 1 < ncl) qn = P.cand_q[cbase + (size_t)(k + 1) * 32];
-        if (!passes(q)) continue;
+        float qf[D];
+        ldf<D>(P.curf, q, qf);
+        const uint32_t gq = P.node_grain[q];  // issued with the position, used after the prefilter
+        if (far(qf) || !allowed(q, gq)) continue;
         if (nc >= (int)P.max_cand) {
           set_status(P.status, PG_ECAPACITY);
           break;
@@ -331,7 +334,6 @@ __global__ void __launch_bounds__(128, BPS) k_force(const Dev P) {
         ++nc;
       }
     } else {
-      unsigned long long keys[MAX_CAND];
       int32_t cc[3] = {0, 0, 0};
       for (int c = 0; c < D; ++c) cc[c] = cell_coord(pf[c] + in.frame_off_f[c], in.inv_cell_f, in.dims[c]);
       const int z0 = (D == 3) ? max(cc[2] - 1, 0) : 0, z1 = (D == 3) ? min(cc[2] + 1, (int)in.dims[2] - 1) : 0;
@@ -341,13 +343,23 @@ __global__ void __launch_bounds__(128, BPS) k_force(const Dev P) {
         for (int y = y0; y <= y1; ++y) {
           const uint32_t row = in.table_off + ((uint32_t)z * in.dims[1] + (uint32_t)y) * in.dims[0];
           const uint32_t b0 = P.cell_start[row + x0], b1 = P.cell_start[row + x1 + 1];
-          for (uint32_t b = b0; b < b1; ++b) {
-            const uint32_t q = P.sorted[b];
-            if (q == d || !passes(q)) continue;
-            const uint32_t gq = P.node_grain[q];
-            const unsigned long long key =
-                ((unsigned long long)(gq == g ? 0u : 1u) << 63) | ((unsigned long long)gq << 32) | P.node_sub[q];
-            insert_cand<D>(keys, idx, nc, key, q, P);
+          for (uint32_t b = b0; b < b1; b += CELL_BATCH) {
+            uint32_t qs[CELL_BATCH];
+            float qf[CELL_BATCH][D];
+#pragma unroll
+            for (uint32_t k = 0; k < CELL_BATCH; ++k) qs[k] = b + k < b1 ? P.sorted[b + k] : d;
+#pragma unroll
+            for (uint32_t k = 0; k < CELL_BATCH; ++k) ldf<D>(P.curf, qs[k], qf[k]);
+#pragma unroll
+            for (uint32_t k = 0; k < CELL_BATCH; ++k) {
+              const uint32_t q = qs[k];
+              if (q == d || far(qf[k])) continue;
+              const uint32_t gq = P.node_grain[q];
+              if (!allowed(q, gq)) continue;
+              const unsigned long long key =
+                  ((unsigned long long)(gq == g ? 0u : 1u) << 63) | ((unsigned long long)gq << 32) | P.node_sub[q];
+              insert_cand<D>(keys, idx, nc, key, q, P);
+            }
           }
         }
     }
@@ -360,7 +372,7 @@ __global__ void __launch_bounds__(128, BPS) k_force(const Dev P) {
       } else {
         q = idx[ci];
       }
-      const uint32_t gqi = P.node_grain[q];
+      const uint32_t gqi = LIST ? P.node_grain[q] : (uint32_t)(keys[ci] >> 32) & 0x7fffffffu;
       const bool same = gqi == g;
       double xq[D], dir[D];
       ldv<D>(P.cur, q, xq);

@@ -777,20 +777,19 @@ __global__ void __launch_bounds__(128, BPS) k_force_mx(const Dev P) {
     float ph[D];
     ldf<D>(P.curf, d, ph);
     const float thr2 = in.pre_f * in.pre_f;
-    // does candidate q pass the FP32 prefilter, the contact rules and the grain-box test? (the box
-    // test of the grain asked about last is kept: a list is sorted by grain)
+    // is candidate q beyond the FP32 prefilter; is it within the contact rules and the grain-box test?
+    // (the box test of the grain asked about last is kept: a list is sorted by grain)
     uint32_t box_g = NONE;
     bool box_ok = false;
-    auto passes = [&](uint32_t q) {
-      float qf[D];
-      ldf<D>(P.curf, q, qf);
-      const uint32_t gq = P.node_grain[q];  // issued with the position, used after the prefilter
+    auto far = [&](const float (&qf)[D]) {
       float d2 = 0.f;
       for (int c = 0; c < D; ++c) {
         float dd = qf[c] - ph[c];
         d2 = fmaf(dd, dd, d2);
       }
-      if (d2 > thr2) return false;
+      return d2 > thr2;
+    };
+    auto allowed = [&](uint32_t q, uint32_t gq) {
       const bool same = (gq == g);
       if (same ? !selfc : !other) return false;
       if (P.nl_bdry_only && P.bdry_rank[q] == NONE) return false;
@@ -808,13 +807,17 @@ __global__ void __launch_bounds__(128, BPS) k_force_mx(const Dev P) {
     const size_t cbase = (size_t)chunk * P.cand_cap * 32 + lane;
     uint32_t hits = 0;
     uint32_t idx[LIST ? 1 : MAX_CAND];
+    unsigned long long keys[LIST ? 1 : MAX_CAND];
     int nc = 0;
     if constexpr (LIST) {
       uint32_t qn = P.cand_q[cbase];  // the next entry is loaded one candidate ahead
       for (uint32_t k = 0; k < ncl; ++k) {
         const uint32_t q = qn;
         if (k + 1 < ncl) qn = P.cand_q[cbase + (size_t)(k + 1) * 32];
-        if (!passes(q)) continue;
+        float qf[D];
+        ldf<D>(P.curf, q, qf);
+        const uint32_t gq = P.node_grain[q];  // issued with the position, used after the prefilter
+        if (far(qf) || !allowed(q, gq)) continue;
         if (nc >= (int)P.max_cand) {
           set_status(P.status, PG_ECAPACITY);
           break;
@@ -823,7 +826,6 @@ __global__ void __launch_bounds__(128, BPS) k_force_mx(const Dev P) {
         ++nc;
       }
     } else {
-      unsigned long long keys[MAX_CAND];
       int32_t cc[3] = {0, 0, 0};
       for (int c = 0; c < D; ++c) cc[c] = cell_coord(ph[c] + in.frame_off_f[c], in.inv_cell_f, in.dims[c]);
       const int z0 = (D == 3) ? max(cc[2] - 1, 0) : 0, z1 = (D == 3) ? min(cc[2] + 1, (int)in.dims[2] - 1) : 0;
@@ -833,13 +835,23 @@ __global__ void __launch_bounds__(128, BPS) k_force_mx(const Dev P) {
         for (int y = y0; y <= y1; ++y) {
           const uint32_t row = in.table_off + ((uint32_t)z * in.dims[1] + (uint32_t)y) * in.dims[0];
           const uint32_t b0 = P.cell_start[row + x0], b1 = P.cell_start[row + x1 + 1];
-          for (uint32_t b = b0; b < b1; ++b) {
-            const uint32_t q = P.sorted[b];
-            if (q == d || !passes(q)) continue;
-            const uint32_t gq = P.node_grain[q];
-            const unsigned long long key =
-                ((unsigned long long)(gq == g ? 0u : 1u) << 63) | ((unsigned long long)gq << 32) | P.node_sub[q];
-            insert_cand<D>(keys, idx, nc, key, q, P);
+          for (uint32_t b = b0; b < b1; b += CELL_BATCH) {
+            uint32_t qs[CELL_BATCH];
+            float qf[CELL_BATCH][D];
+#pragma unroll
+            for (uint32_t k = 0; k < CELL_BATCH; ++k) qs[k] = b + k < b1 ? P.sorted[b + k] : d;
+#pragma unroll
+            for (uint32_t k = 0; k < CELL_BATCH; ++k) ldf<D>(P.curf, qs[k], qf[k]);
+#pragma unroll
+            for (uint32_t k = 0; k < CELL_BATCH; ++k) {
+              const uint32_t q = qs[k];
+              if (q == d || far(qf[k])) continue;
+              const uint32_t gq = P.node_grain[q];
+              if (!allowed(q, gq)) continue;
+              const unsigned long long key =
+                  ((unsigned long long)(gq == g ? 0u : 1u) << 63) | ((unsigned long long)gq << 32) | P.node_sub[q];
+              insert_cand<D>(keys, idx, nc, key, q, P);
+            }
           }
         }
     }
@@ -861,7 +873,7 @@ __global__ void __launch_bounds__(128, BPS) k_force_mx(const Dev P) {
       } else {
         q = idx[ci];
       }
-      const uint32_t gqi = P.node_grain[q];
+      const uint32_t gqi = LIST ? P.node_grain[q] : (uint32_t)(keys[ci] >> 32) & 0x7fffffffu;
       ContactTerm<D> o;
       if (!contact_term<D, GC>(P, s, gqi, d, q, Partner<D>(P, q), o)) continue;
       apply(q, o);
@@ -1082,8 +1094,8 @@ __global__ void __launch_bounds__(128, BPS) k_force_mx(const Dev P) {
 // The force kernel's variants: mask recording (REC), per-grain contact parameters (GC), a node
 // layout other than the input order (PERM) and candidate lists or the grid search (LIST) are compiled
 // in only where used, so the plain kernel keeps its register budget; the plain kernel with lists also
-// for BPS = 5, 6 or 7 blocks of 128 threads per SM (96, 80 or 72 registers), see force_bps(), and each
-// with lists also for teams of warps (TEAM).
+// for BPS = 5, 6 or 7 blocks of 128 threads per SM (96, 80 or 72 registers), without lists for 5 or 6, see
+// force_bps(), and each with lists also for teams of warps (TEAM).
 template <int D>
 static const void* force_mx_ptr(bool rec, bool gc, bool perm, bool list, int bps, bool team) {
 #define PG_F(r, g, p, l, b) (const void*)k_force_mx<D, r, g, p, l, b, false>
@@ -1094,12 +1106,14 @@ static const void* force_mx_ptr(bool rec, bool gc, bool perm, bool list, int bps
 #undef PG_T
   static const void* const plain[2][3] = {{PG_F(0, 0, 0, 1, 5), PG_F(0, 0, 0, 1, 6), PG_F(0, 0, 0, 1, 7)},
                                           {PG_F(0, 0, 1, 1, 5), PG_F(0, 0, 1, 1, 6), PG_F(0, 0, 1, 1, 7)}};
+  static const void* const search[2] = {PG_F(0, 0, 0, 0, 6), PG_F(0, 0, 1, 0, 6)};
   static const void* const others[14] = {
-      PG_F(0, 0, 0, 0, 6), PG_F(0, 0, 1, 0, 6), PG_F(0, 1, 0, 0, 5), PG_F(0, 1, 0, 1, 5), PG_F(0, 1, 1, 0, 5),
+      PG_F(0, 0, 0, 0, 5), PG_F(0, 0, 1, 0, 5), PG_F(0, 1, 0, 0, 5), PG_F(0, 1, 0, 1, 5), PG_F(0, 1, 1, 0, 5),
       PG_F(0, 1, 1, 1, 5), PG_F(1, 0, 0, 0, 5), PG_F(1, 0, 0, 1, 5), PG_F(1, 0, 1, 0, 5), PG_F(1, 0, 1, 1, 5),
       PG_F(1, 1, 0, 0, 5), PG_F(1, 1, 0, 1, 5), PG_F(1, 1, 1, 0, 5), PG_F(1, 1, 1, 1, 5)};
 #undef PG_F
-  if (!rec && !gc) return list ? plain[perm ? 1 : 0][bps - 5] : others[perm ? 1 : 0];
+  if (!rec && !gc && list) return plain[perm ? 1 : 0][bps - 5];
+  if (!rec && !gc) return bps > 5 ? search[perm ? 1 : 0] : others[perm ? 1 : 0];
   return others[2 + (rec ? (gc ? 8 : 4) : 0) + (perm ? 2 : 0) + (list ? 1 : 0)];
 }
 template <int D>
