@@ -125,6 +125,11 @@ int run_steps(pg_handle* h, uint32_t n, uint64_t* launches) {
   return PG_OK;
 }
 
+cudaError_t write_device(pg_handle* h, void* dst, const void* src, size_t bytes) {
+  const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, h->stream);
+  return e != cudaSuccess ? e : cudaStreamSynchronize(h->stream);
+}
+
 // Force a rebuild of the contact candidate lists at the next step (after host writes of state).
 int request_list_rebuild(pg_handle* h) {
   if (!h->rebuild_pp[0]) return PG_OK;
@@ -1207,9 +1212,9 @@ int pg_set_field(pg_handle* h, int field, const double* in) {
     // keep the bond reference positions (xi = pos[j] - pos[i] at load time) unchanged
     double* x = nullptr;
     CU(cudaMalloc((void**)&x, (size_t)N * S * 8));
-    CU(cudaMemcpy(x, h->P.pos, (size_t)N * S * 8, cudaMemcpyDeviceToDevice));
     h->P.xpos = x;
     h->xpos_separate = true;
+    CU(cudaMemcpyAsync(x, h->P.pos, (size_t)N * S * 8, cudaMemcpyDeviceToDevice, h->stream));
     rc = build_graphs(h);
     if (rc) return rc;
   }
@@ -1224,8 +1229,8 @@ int pg_set_field(pg_handle* h, int field, const double* in) {
   std::vector<double> tmp((size_t)N * S, 0.0);
   for (uint32_t i = 0; i < N; ++i)
     for (uint32_t c = 0; c < D; ++c) tmp[(size_t)i * S + c] = in[(size_t)i * D + c];
-  CU(cudaMemcpy(dst, tmp.data(), tmp.size() * 8, cudaMemcpyHostToDevice));
-  if (field == PG_FIELD_DISP) CU(cudaMemset(h->P.clamp_pending, 0, N));
+  if (field == PG_FIELD_DISP) CU(cudaMemsetAsync(h->P.clamp_pending, 0, N, h->stream));
+  CU(write_device(h, dst, tmp.data(), tmp.size() * 8));
   rc = request_list_rebuild(h);
   if (rc) return rc;
   if (h->precision == PG_MIXED && field == PG_FIELD_ACC) {
@@ -1276,7 +1281,7 @@ int pg_set_bond_alive(pg_handle* h, const uint8_t* in) {
     for (uint32_t k = 0; k < h->node_deg[i]; ++k)
       if (in[h->bond_offset[h->orig(i)] + k]) words[h->chunk_word[c] + k] |= 1u << lane;
   }
-  if (!words.empty()) CU(cudaMemcpy(h->P.alive, words.data(), words.size() * 4, cudaMemcpyHostToDevice));
+  if (!words.empty()) CU(write_device(h, h->P.alive, words.data(), words.size() * 4));
   return PG_OK;
 }
 
@@ -1309,7 +1314,7 @@ int pg_set_wall(pg_handle* h, const double* geom) {
   const uint32_t NS = 2 * h->dim;
   for (uint32_t k = 0; k < h->P.I; ++k)
     for (uint32_t a = 0; a < NS; ++a) in[k].wall[a] = geom[(size_t)k * NS + a];
-  CU(cudaMemcpy(h->P.inst, in.data(), in.size() * sizeof(InstDev), cudaMemcpyHostToDevice));
+  CU(write_device(h, h->P.inst, in.data(), in.size() * sizeof(InstDev)));
   return PG_OK;
 }
 
@@ -1321,7 +1326,7 @@ int pg_set_grain_flags(pg_handle* h, uint32_t grain, int32_t movable, int32_t st
   CU(cudaMemcpy(&gd, h->P.grain + grain, sizeof(gd), cudaMemcpyDeviceToHost));
   if (movable >= 0) gd.flags = movable ? (gd.flags | GF_MOVABLE) : (gd.flags & ~GF_MOVABLE);
   if (stoppable >= 0) gd.flags = stoppable ? (gd.flags | GF_STOPPABLE) : (gd.flags & ~GF_STOPPABLE);
-  CU(cudaMemcpy(h->P.grain + grain, &gd, sizeof(gd), cudaMemcpyHostToDevice));
+  CU(write_device(h, h->P.grain + grain, &gd, sizeof(gd)));
   return request_list_rebuild(h);
 }
 
@@ -1351,8 +1356,7 @@ int pg_get_pair_log(pg_handle* h, uint32_t n, uint64_t* count, uint64_t* hash) {
 int pg_debug_grid_barrier(pg_handle* h, uint32_t arrivals) {
   if (!h) return fail(PG_EINVAL, "null handle");
   if (!h->P.gbar || !h->P.coop_blocks) return fail(PG_EINVAL, "no cooperative grid build on this handle");
-  CU(cudaStreamSynchronize(h->stream));
-  CU(cudaMemcpy(h->P.gbar, &arrivals, 4, cudaMemcpyHostToDevice));
+  CU(write_device(h, h->P.gbar, &arrivals, 4));
   return PG_OK;
 }
 

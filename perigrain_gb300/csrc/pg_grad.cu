@@ -336,7 +336,7 @@ int pg_set_grain_params(pg_handle* h, const double* cnot, const double* snot, co
     if (mu) g[k].mu = mu[k];
     set_grain_f(g[k]);
   }
-  CU(cudaMemcpy(h->P.grain, g.data(), g.size() * sizeof(GrainDev), cudaMemcpyHostToDevice));
+  CU(write_device(h, h->P.grain, g.data(), g.size() * sizeof(GrainDev)));
   if ((kn || zeta || mu) && !h->P.grain_contact) {
     h->P.grain_contact = 1;
     if (h->grad) h->grad->drop_graphs();
@@ -438,8 +438,8 @@ int pg_masks_record(pg_handle* h, uint32_t n_steps, pg_masks** out) {
     }
     if (st) return fail(st, std::string("device reported: ") + pg_status_string(st));
     m->n_ent = need;
-    CU(cudaMemcpy(m->end_alive, h->P.alive, (size_t)h->chunk_word[NC] * 4, cudaMemcpyDeviceToDevice));
-    CU(cudaMemcpy(m->break_step, h->P.break_step, (size_t)h->chunk_slot[NC] * 4, cudaMemcpyDeviceToDevice));
+    CU(cudaMemcpyAsync(m->end_alive, h->P.alive, (size_t)h->chunk_word[NC] * 4, cudaMemcpyDeviceToDevice, h->stream));
+    CU(cudaMemcpyAsync(m->break_step, h->P.break_step, (size_t)h->chunk_slot[NC] * 4, cudaMemcpyDeviceToDevice, h->stream));
     G->ready = false;
     *out = m.release();
     return PG_OK;

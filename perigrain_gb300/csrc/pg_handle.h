@@ -238,6 +238,10 @@ void enqueue_body(pg_handle* h, const pg::Dev& P, uint64_t* launches, bool rec);
 void enqueue_finalize(pg_handle* h, const pg::Dev& P, uint64_t* launches);
 // Run n steps from the handle's state: the graphs where they fit. Advances the parity, not next_t.
 int run_steps(pg_handle* h, uint32_t n, uint64_t* launches);
+// Host data to the device, complete when it returns. On the handle's own stream: a copy on the default
+// stream from pageable memory may return before the data has landed, and the handle's stream, a
+// non-blocking one, does not wait for that.
+cudaError_t write_device(pg_handle* h, void* dst, const void* src, size_t bytes);
 // CurrPos = pos + disp of the state at hand into its buffer (a restored state brings only disp).
 int refresh_currpos(pg_handle* h);
 int build_graphs(pg_handle* h);

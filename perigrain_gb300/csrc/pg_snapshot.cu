@@ -178,7 +178,7 @@ int pg_snapshot(pg_handle* h, const pg_snapshot_desc* d) {
   }
   if (want_alive && !s.bond_offset) {
     CU(cudaMalloc((void**)&s.bond_offset, (size_t)(N + 1) * 8));
-    CU(cudaMemcpy(s.bond_offset, h->bond_offset.data(), (size_t)(N + 1) * 8, cudaMemcpyHostToDevice));
+    CU(write_device(h, s.bond_offset, h->bond_offset.data(), (size_t)(N + 1) * 8));
   }
 
   SnapArgs a{};
