@@ -666,6 +666,14 @@ static __global__ void __launch_bounds__(256) k_chain(const Dev P) {
 // the contact rules could pair with d (same grain: self-contact; other grain: stoppable, or any in
 // the worm loop; boundary nodes only when nl_bdry_only), sorted by the reference's visit order.
 // The bounding-box prefilter is applied per step, not here. Also records the displacement.
+//
+// Bound by the latency of the chains' loads: the three chains of a row of cells are walked side by side, so
+// a round waits for one load where one chain after another waited for three. us a step with a build at
+// every other step, one chain / three at a time: two disks, 0.6 / 10 / 31 nodes a cell 13.4 / 25.8 / 46.7
+// and 12.8 / 22.6 / 40.0; 3D, 0.5 / 6.4 / 25 a cell 25.7 / 45.1 / 103 and 24.2 / 38.0 / 77.7; two disks
+// burst apart into cells of hundreds of nodes 114 / 55, in FP64 862 / 307 (444 with the cells' nodes
+// sorted and copied into a row). A layout of consecutive nodes for full cells in the same kernel was
+// faster still for these (168), but it slowed the chains of all others down by a quarter.
 template <int D>
 __device__ __forceinline__ void cand_build_node(const Dev& P, uint32_t d) {
   const uint32_t lane = d & 31, chunk = d >> 5;
@@ -695,19 +703,28 @@ __device__ __forceinline__ void cand_build_node(const Dev& P, uint32_t d) {
     for (int z = z0; z <= z1; ++z)
       for (int y = y0; y <= y1; ++y) {
         const uint32_t row = in.table_off + ((uint32_t)z * in.dims[1] + (uint32_t)y) * in.dims[0];
-        uint32_t first[3];  // the row's three chains, started together
-        for (int i = 0; i < 3; ++i) first[i] = x0 + i <= x1 ? P.cell_start[row + x0 + i] : NONE;
-        for (int i = 0; i < 3; ++i) {
-          uint32_t qn = first[i];
-          while (qn != NONE) {
-            const uint32_t q = qn;
-            qn = P.cell_rank[q];
-            float qf[D];
-            ldf<D>(P.curf, q, qf);
-            if (q == d) continue;
+        // the row's three chains side by side, so that a round waits for one load and not for three
+        uint32_t at[3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) at[i] = x0 + i <= x1 ? P.cell_start[row + x0 + i] : NONE;
+        while ((at[0] & at[1] & at[2]) != NONE) {
+          uint32_t next[3];
+          float qf[3][D];
+#pragma unroll
+          for (int i = 0; i < 3; ++i) {
+            next[i] = NONE;
+            if (at[i] == NONE) continue;
+            next[i] = P.cell_rank[at[i]];
+            ldf<D>(P.curf, at[i], qf[i]);
+          }
+#pragma unroll
+          for (int i = 0; i < 3; ++i) {
+            const uint32_t q = at[i];
+            at[i] = next[i];
+            if (q == NONE || q == d) continue;
             float d2 = 0.f;
             for (int c = 0; c < D; ++c) {
-              const float dd = qf[c] - pf[c];
+              const float dd = qf[i][c] - pf[c];
               d2 += dd * dd;
             }
             if (d2 > thr2) continue;

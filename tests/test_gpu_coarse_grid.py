@@ -48,3 +48,35 @@ def test_grid_search_reports_a_full_contact_list():
         with pytest.raises(Exception):
             sim.step(300)
             sim.synchronize()
+
+
+@pytest.mark.parametrize("skin", [0.25, 0.02])
+@pytest.mark.parametrize("far", [0.0, 2e-2, 2.0])
+@pytest.mark.parametrize("dim", [2, 3])
+def test_lists_from_coarse_cells(dim, far, skin):
+    s = _scene(dim, far)
+    kw = dict(dt=2e-8, enable_fracture=1)
+    r = O.OracleSim(s, **kw)
+    r.step(250)
+    for cells in (1, 0):
+        g = Simulation(s, record_pairs=True, contact_skin=skin, cells_per_node=cells, **kw)
+        g.step(250)
+        for f in FIELDS:
+            assert np.array_equal(g.field(f), r.field(f)), f
+        assert np.array_equal(g.break_step(), r.break_step())
+        assert np.array_equal(np.array(g.pair_log(250)), np.array(r.pair_log_all()))
+    sims = [Simulation(s, precision="mixed", contact_skin=k, cells_per_node=1, **kw) for k in (skin, 0.0)]
+    for sim in sims:
+        sim.step(250)
+    for f in FIELDS:
+        assert np.array_equal(sims[0].field(f), sims[1].field(f)), f
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_full_candidate_list_is_reported(precision):
+    s = setups.two_disk_collision(gap=-2e-4)
+    s.contact_radius = s.contact_radius * 6.0
+    sim = Simulation(s, dt=2e-8, precision=precision, self_contact=0)
+    with pytest.raises(Exception):
+        sim.step(2)
+        sim.synchronize()
