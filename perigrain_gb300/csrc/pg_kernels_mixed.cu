@@ -645,11 +645,10 @@ __global__ void __launch_bounds__(128, BPS) k_force_mx(const Dev P) {
   {
     // bond forces and bond breaking (particle2.h:102-232): two bonds per iteration, both
     // neighbour gathers issued before either is used
+    // (loaded for lanes without bonds in use too: those add 0 times a vector, which must be finite)
     float dh[D], dl[D], xh[D], xl[D];
-    if (mov) {
-      ld_hl<D>(P.dref, P.np, d, dh, dl);
-      ld_hl<D>(P.xref, P.np, d, xh, xl);
-    }
+    ld_hl<D>(P.dref, P.np, d, dh, dl);
+    ld_hl<D>(P.xref, P.np, d, xh, xl);
     if constexpr (REC) {
       if (mov && sub == 0 && P.rec_df) st_hl<D>(P.rec_df, P.np, d, dh, dl);
     }
