@@ -241,43 +241,93 @@ static int mixed_setup(pg_handle* h, const pg_setup_desc* s) {
 // Edge list of the FP64 path (Dev::edge_ij). Slot s = (i -> j, the m-th entry of row i naming j) is
 // paired with the m-th entry of row j naming i when there is one (the two compute the same bond); a
 // pair is listed once, at the lower node's slot, an unpaired slot by itself.
+// A block a chunk, lane = node, its warps taking the rows' entries in turn.
+// k_edge_rows: whether each row's entries ascend in the input's numbering, as a reference row does.
 // k_edge_pairs: each slot's partner (NONE: unpaired) to pair[s], EDGE_SKIP where the slot is not listed
-// (padding, or the partner's entry covers it),
-// and the chunk's number of entries to count[c]. One warp per 32-node chunk, lane = node.
-constexpr uint32_t EDGE_SKIP = NONE - 1u;
-__global__ void k_edge_pairs(const Dev P, uint32_t* pair, uint32_t* count) {
-  const uint32_t c = blockIdx.x, lane = threadIdx.x, i = c * 32 + lane;
-  const uint32_t deg = i < P.N ? P.node_deg[i] : 0u;
+// (padding, or the partner's entry covers it), and the chunk's number of entries to count[c]. A row that
+// ascends has no repeated entries and is searched by halves, any other entry by entry. Both kernels, us:
+// two disks (65k entries) 15, spheres in 3D (10.8M) 144; all rows entry by entry 34 and 1170. (With a warp
+// a chunk and entry by entry, 135 nodes alone took 50.)
+constexpr uint32_t EDGE_SKIP = NONE - 1u, EDGE_WARPS = 8;
+__global__ void __launch_bounds__(32 * EDGE_WARPS) k_edge_rows(const Dev P, uint32_t* ascends) {
+  __shared__ uint32_t bad;
+  const uint32_t c = blockIdx.x, lane = threadIdx.x & 31, i = c * 32 + lane;
+  const uint32_t deg = i < P.N ? P.node_deg[i] : 0u, row = P.chunk_slot[c] + lane;
+  if (threadIdx.x == 0) bad = 0;
+  __syncthreads();
+  bool ok = true;
+#pragma unroll 4
+  for (uint32_t k = 1 + (threadIdx.x >> 5); k < deg; k += EDGE_WARPS)
+    ok &= orig_of(P, P.bcol[row + 32u * (k - 1)]) < orig_of(P, P.bcol[row + 32u * k]);
+  const uint32_t wrong = __ballot_sync(0xffffffffu, !ok);
+  if (lane == 0 && wrong) atomicOr(&bad, wrong);
+  __syncthreads();
+  if (threadIdx.x < 32 && i < P.N) ascends[i] = (bad >> lane & 1u) ^ 1u;
+}
+__global__ void __launch_bounds__(32 * EDGE_WARPS)
+    k_edge_pairs(const Dev P, const uint32_t* ascends, uint32_t* pair, uint32_t* count) {
+  __shared__ uint32_t total;
+  const uint32_t c = blockIdx.x, lane = threadIdx.x & 31, i = c * 32 + lane;
+  const uint32_t deg = i < P.N ? P.node_deg[i] : 0u, oi = i < P.N ? orig_of(P, i) : 0u;
   const uint32_t row = P.chunk_slot[c] + lane, cd = P.chunk_deg[c];
+  const bool once = i < P.N && ascends[i];
+  if (threadIdx.x == 0) total = 0;
+  __syncthreads();
   uint32_t n = 0;
-  for (uint32_t k = 0; k < cd; ++k) {
+  for (uint32_t k = threadIdx.x >> 5; k < cd; k += EDGE_WARPS) {
     const uint32_t s = row + 32u * k;
     uint32_t other = EDGE_SKIP;
     if (k < deg) {
       const uint32_t j = P.bcol[s];
-      uint32_t m = 0;
-      for (uint32_t q = 0; q < k; ++q) m += P.bcol[row + 32u * q] == j ? 1u : 0u;
-      const uint32_t rj = P.chunk_slot[j >> 5] + (j & 31), dj = P.node_deg[j];
-      other = NONE;
-      for (uint32_t q = 0; q < dj && j != i; ++q)
-        if (P.bcol[rj + 32u * q] == i && m-- == 0) {
-          other = i < j ? rj + 32u * q : EDGE_SKIP;
-          break;
+      uint32_t m = 0;  // entries before this one that name j
+      if (!once)
+#pragma unroll 8
+        for (uint32_t q = 0; q < k; ++q) m += P.bcol[row + 32u * q] == j ? 1u : 0u;
+      const uint32_t rj = P.chunk_slot[j >> 5] + (j & 31), dj = j != i ? P.node_deg[j] : 0u;
+      uint32_t at = NONE;
+      if (ascends[j]) {
+        uint32_t lo = 0, hi = dj;
+        while (lo < hi) {
+          const uint32_t mid = (lo + hi) >> 1;
+          if (orig_of(P, P.bcol[rj + 32u * mid]) < oi) lo = mid + 1; else hi = mid;
         }
+        if (m == 0 && lo < dj && P.bcol[rj + 32u * lo] == i) at = rj + 32u * lo;
+      } else {
+        uint32_t seen = 0;
+#pragma unroll 8
+        for (uint32_t q = 0; q < dj; ++q) {
+          const bool back = P.bcol[rj + 32u * q] == i;
+          if (back && seen == m) at = rj + 32u * q;
+          seen += back ? 1u : 0u;
+        }
+      }
+      other = at == NONE || i < j ? at : EDGE_SKIP;
     }
     pair[s] = other;
     n += other != EDGE_SKIP ? 1u : 0u;
   }
   n = __reduce_add_sync(0xffffffffu, n);
-  if (lane == 0) count[c] = n;
+  if (lane == 0) atomicAdd(&total, n);
+  __syncthreads();
+  if (threadIdx.x == 0) count[c] = total;
 }
-// The chunk's entries, in slot order from first[c].
-__global__ void k_edge_fill(const Dev P, const uint32_t* pair, const uint32_t* first, uint2* ij, uint2* slot,
-                            double* xin) {
-  const uint32_t c = blockIdx.x, lane = threadIdx.x, i = c * 32 + lane;
+// The chunk's entries, in slot order from first[c]: each warp a run of the rows' entries.
+__global__ void __launch_bounds__(32 * EDGE_WARPS) k_edge_fill(const Dev P, const uint32_t* pair, const uint32_t* first,
+                                                               uint2* ij, uint2* slot, double* xin) {
+  __shared__ uint32_t run[EDGE_WARPS];
+  const uint32_t c = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5, i = c * 32 + lane;
   const uint32_t row = P.chunk_slot[c] + lane, cd = P.chunk_deg[c];
+  const uint32_t per = (cd + EDGE_WARPS - 1) / EDGE_WARPS, k0 = min(w * per, cd), k1 = min(k0 + per, cd);
+  uint32_t n = 0;
+#pragma unroll 4
+  for (uint32_t k = k0; k < k1; ++k) n += pair[row + 32u * k] != EDGE_SKIP ? 1u : 0u;
+  n = __reduce_add_sync(0xffffffffu, n);
+  if (lane == 0) run[w] = n;
+  __syncthreads();
   uint32_t at = first[c];
-  for (uint32_t k = 0; k < cd; ++k) {
+  for (uint32_t v = 0; v < w; ++v) at += run[v];
+#pragma unroll 4
+  for (uint32_t k = k0; k < k1; ++k) {
     const uint32_t s = row + 32u * k, other = pair[s];
     const uint32_t b = __ballot_sync(0xffffffffu, other != EDGE_SKIP);
     if (other != EDGE_SKIP) {
@@ -292,30 +342,28 @@ __global__ void k_edge_fill(const Dev P, const uint32_t* pair, const uint32_t* f
 
 static int edges_setup(pg_handle* h) {
   Dev& P = h->P;
-  const uint32_t NC = P.n_chunks, slots = h->chunk_slot[NC];
+  const uint32_t NC = P.n_chunks, slots = h->chunk_slot[NC], tiles = bond_scan_tiles(NC);
   P.n_edges = 0;
-  CU(h->dalloc(&P.addend, (size_t)slots * 2));
-  if (h->dim == 3) CU(h->dalloc(&P.addend_z, slots));
+  // the list's scratch is in the addends' place, which is cleared behind it
+  const size_t words = (size_t)slots * (h->dim == 3 ? 6 : 4), scratch = (size_t)slots + P.N + 2 * (size_t)NC + 2 + tiles;
+  CU(h->dalloc(&P.addend, (std::max(words, scratch) + 1) / 2));
+  if (h->dim == 3) P.addend_z = P.addend + (size_t)slots * 2;
   if (!slots) return PG_OK;
-  DevPool tmp;
-  uint32_t *pair = (uint32_t*)P.addend, *count = nullptr, *first = nullptr, *tile = nullptr, *done = nullptr;
-  CU(tmp.alloc(&count, NC));
-  CU(tmp.alloc(&first, NC + 1));
-  CU(tmp.alloc(&tile, bond_scan_tiles(NC)));
-  CU(tmp.alloc(&done, 1));
+  uint32_t *pair = (uint32_t*)P.addend, *count = pair + slots, *first = count + NC, *tile = first + NC + 1;
+  uint32_t *done = tile + tiles, *ascends = done + 1;
   CU(cudaMemset(done, 0, 4));
-  k_edge_pairs<<<NC, 32>>>(P, pair, count);
+  k_edge_rows<<<NC, 32 * EDGE_WARPS>>>(P, ascends);
+  CU(cudaGetLastError());
+  k_edge_pairs<<<NC, 32 * EDGE_WARPS>>>(P, ascends, pair, count);
   CU(cudaGetLastError());
   CU(scan_u32_dev(count, NC, first, tile, done, 0));
   CU(cudaMemcpy(&P.n_edges, first + NC, 4, cudaMemcpyDeviceToHost));
-  CU(h->dalloc(&P.edge_ij, P.n_edges));
-  CU(h->dalloc(&P.edge_slot, P.n_edges));
-  CU(h->dalloc(&P.edge_xin, P.n_edges));
-  k_edge_fill<<<NC, 32>>>(P, pair, first, P.edge_ij, P.edge_slot, P.edge_xin);
+  CU(h->dalloc(&P.edge_xin, (size_t)P.n_edges * 3));
+  P.edge_ij = (uint2*)(P.edge_xin + P.n_edges);
+  P.edge_slot = P.edge_ij + P.n_edges;
+  k_edge_fill<<<NC, 32 * EDGE_WARPS>>>(P, pair, first, P.edge_ij, P.edge_slot, P.edge_xin);
   CU(cudaGetLastError());
-  CU(cudaMemset(P.addend, 0, (size_t)slots * 16));
-  if (h->dim == 3) CU(cudaMemset(P.addend_z, 0, (size_t)slots * 8));
-  CU(cudaDeviceSynchronize());
+  CU(cudaMemset(P.addend, 0, words * 4));
   return PG_OK;
 }
 
@@ -700,10 +748,19 @@ static int create_impl(const pg_setup_desc* s, const pg_config* cfg_in, pg_handl
     }
   };
   double** vecs[] = {&P.pos, &P.disp, &h->cur_pp[0], &h->cur_pp[1], &h->vel_a, &h->vel_b, &P.acc, &P.force, &P.extf};
-  for (double** v : vecs) CU(h->dalloc(v, (size_t)N * S));
+  {
+    // one allocation for all of them (an allocation takes about as long as a small handle's copy)
+    const size_t V = ((size_t)N * S + 31) / 32 * 32, n_vec = sizeof vecs / sizeof vecs[0];
+    double* block = nullptr;
+    CU(h->dalloc(&block, (n_vec + 1) * V + N));
+    for (double** v : vecs) {
+      *v = block;
+      block += V;
+    }
+    for (int p = 0; p < 2; ++p) h->curf_pp[p] = (float*)block + (size_t)p * V;
+    P.vol = block + V;
+  }
   P.xpos = P.pos;
-  CU(h->dalloc(&P.vol, N));
-  for (int p = 0; p < 2; ++p) CU(h->dalloc(&h->curf_pp[p], (size_t)N * S));
   // in 2D the stride is the dimension: straight uploads; in 3D through the padded host buffer
   auto upload = [&](double* dst, const double* src) -> cudaError_t {
     if (S == D && !permuted) return cudaMemcpy(dst, src, (size_t)N * D * 8, cudaMemcpyHostToDevice);
@@ -717,11 +774,11 @@ static int create_impl(const pg_setup_desc* s, const pg_config* cfg_in, pg_handl
   CU(upload(P.acc, s->acc));
   CU(upload(P.extf, s->extforce));
   CU(cudaMemset(P.force, 0, (size_t)N * S * 8));
-  // CurrPos before the first step is pos + disp (the uploads ran on the default stream)
-  CU(cudaDeviceSynchronize());
-  rc = refresh_currpos(h.get());
-  if (rc) return rc;
-  CU(cudaStreamSynchronize(h->stream));
+  // CurrPos before the first step is pos + disp (on the default stream, as the uploads)
+  if (N) {
+    k_add_vec<<<(N * S + 255) / 256, 256>>>(P.pos, P.disp, h->cur(), N * S);
+    CU(cudaGetLastError());
+  }
   if (permuted) {
     std::vector<double> v(N);
     for (uint32_t i = 0; i < N; ++i) v[i] = s->vol[ord.perm[i]];
@@ -805,29 +862,23 @@ static int create_impl(const pg_setup_desc* s, const pg_config* cfg_in, pg_handl
     // the reference CSR goes up once; the SELL-32 slab, the alive words and xi_norm are built on
     // the device
     const uint64_t nb = s->bond_offset[N];
-    uint64_t* d_off = nullptr;
-    uint32_t* d_loc = nullptr;
-    uint32_t* d_gno = nullptr;
-    cudaError_t e = cudaMalloc((void**)&d_off, (size_t)(N + 1) * 8);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&d_loc, (size_t)std::max<uint64_t>(nb, 1) * 4);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&d_gno, (size_t)(G + 1) * 4);
+    void* block = nullptr;
+    cudaError_t e = cudaMalloc(&block, (size_t)(N + 2) * 8 + ((size_t)nb + G + 1) * 4);
+    uint64_t* d_off = (uint64_t*)block;
+    unsigned long long bad = ~0ull, *d_bad = (unsigned long long*)(d_off + N + 1);
+    uint32_t *d_loc = (uint32_t*)(d_bad + 1), *d_gno = d_loc + nb;
     if (e == cudaSuccess) e = cudaMemcpy(d_off, s->bond_offset, (size_t)(N + 1) * 8, cudaMemcpyHostToDevice);
     if (e == cudaSuccess && nb) e = cudaMemcpy(d_loc, s->bond_local, (size_t)nb * 4, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(d_gno, s->grain_node_offset, (size_t)(G + 1) * 4, cudaMemcpyHostToDevice);
     // bond rows checked before anything reads through them
-    unsigned long long bad = ~0ull, *d_bad = nullptr;
-    if (e == cudaSuccess) e = cudaMalloc((void**)&d_bad, 8);
     if (e == cudaSuccess) e = cudaMemcpy(d_bad, &bad, 8, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) {
       k_check_bonds<<<(N + 255) / 256, 256>>>(d_off, d_loc, d_gno, P.node_grain, N, nb, d_bad);
       e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaMemcpy(&bad, d_bad, 8, cudaMemcpyDeviceToHost);
-    if (d_bad) cudaFree(d_bad);
     if (e == cudaSuccess && bad != ~0ull) {
-      cudaFree(d_off);
-      cudaFree(d_loc);
-      cudaFree(d_gno);
+      cudaFree(block);
       const uint32_t node = (uint32_t)(bad & 0xffffffffu);
       if ((bad >> 32) == 0) return fail(PG_EINVAL, "bond_offset decreasing");
       return fail(PG_EINVAL, "bond of node " + std::to_string(node) + " points outside its grain");
@@ -839,9 +890,7 @@ static int create_impl(const pg_setup_desc* s, const pg_config* cfg_in, pg_handl
     }
     if (e == cudaSuccess) e = cudaMemset(P.break_step, 0, slots * 4);
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
-    cudaFree(d_off);
-    cudaFree(d_loc);
-    cudaFree(d_gno);
+    cudaFree(block);
     CU(e);
   }
   tr.mark("bond layout");
@@ -966,14 +1015,16 @@ static int create_impl(const pg_setup_desc* s, const pg_config* cfg_in, pg_handl
   // ---- grid buffers ----
   CU(h->dalloc(&P.cell_key, N));
   CU(h->dalloc(&P.cell_rank, N));
-  CU(h->dalloc(&P.sorted, N));
-  CU(h->dalloc(&P.cell_count, table_total));
   CU(h->dalloc(&P.cell_start, table_total + 1));
-  CU(cudaMemset(P.cell_count, 0, table_total * 4));
-  const uint32_t ntiles = (uint32_t)((table_total + 4095) / 4096);
-  CU(h->dalloc(&P.scan_tile_sum, ntiles));
-  CU(h->dalloc(&P.scan_done, 1));
-  CU(cudaMemset(P.scan_done, 0, 4));
+  if (!(cfg.contact_skin > 0)) {  // the counting sort of the grid search
+    CU(h->dalloc(&P.sorted, N));
+    CU(h->dalloc(&P.cell_count, table_total));
+    CU(cudaMemset(P.cell_count, 0, table_total * 4));
+    const uint32_t ntiles = (uint32_t)((table_total + 4095) / 4096);
+    CU(h->dalloc(&P.scan_tile_sum, ntiles));
+    CU(h->dalloc(&P.scan_done, 1));
+    CU(cudaMemset(P.scan_done, 0, 4));
+  }
   tr.mark("grains, grid");
 
   // ---- wall records, logs, control ----

@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 
 #include "pg_device.cuh"
@@ -21,15 +22,22 @@ inline cudaError_t ensure_local_bytes(size_t bytes) {
   if (e != cudaSuccess || cur >= bytes) return e;
   return cudaDeviceSetLimit(cudaLimitStackSize, (bytes + 255) / 256 * 256);
 }
-// The largest local frame (cudaFuncAttributes::localSizeBytes) among the kernels `fs`.
-inline cudaError_t max_local_bytes(const void* const* fs, int n, size_t* out) {
-  size_t m = 0;
+// The largest local frame (cudaFuncAttributes::localSizeBytes) among the kernels `fs`; asked for once
+// (*known, 0 before), as it is a constant of the compiled code and the 144 force kernels take a tenth of a
+// small handle's creation to ask.
+inline cudaError_t max_local_bytes(const void* const* fs, int n, std::atomic<size_t>* known, size_t* out) {
+  size_t m = known->load(std::memory_order_relaxed);
+  if (m) {
+    *out = m;
+    return cudaSuccess;
+  }
   for (int k = 0; k < n; ++k) {
     cudaFuncAttributes a;
     const cudaError_t e = cudaFuncGetAttributes(&a, fs[k]);
     if (e != cudaSuccess) return e;
     m = a.localSizeBytes > m ? a.localSizeBytes : m;
   }
+  known->store(m, std::memory_order_relaxed);
   *out = m;
   return cudaSuccess;
 }

@@ -1140,7 +1140,8 @@ cudaError_t kernels_mixed_init() {
     fs[n++] = force_mx_ptr<3>(k & 4, k & 2, k & 1, true, 5, true);
   }
   size_t need = 0;
-  e = max_local_bytes(fs, n, &need);
+  static std::atomic<size_t> known{0};
+  e = max_local_bytes(fs, n, &known, &need);
   return e == cudaSuccess ? ensure_local_bytes(need) : e;
 }
 
