@@ -20,6 +20,7 @@
 #include "pg_device.cuh"
 #include "pg_hilo.cuh"
 #include "pg_kernels_mixed.h"
+#include "pg_sqrt_float.cuh"
 
 namespace pg {
 
@@ -224,25 +225,6 @@ __device__ __forceinline__ float bond_term(const float (&dh)[D], const float (&d
   const float str = __fdividef(num * ixn, fmaf(yy, iyn, xx * ixn));
   *str_out = str;
   return use ? cv * str * iyn : 0.f;
-}
-
-// (float)sqrt(x), the FP64 square root rounded again, without it: c = sqrtf((float)x) is at most one
-// float off, and the exact remainder x - c c tells on which side of the halfway point between two
-// floats the root lies. Only within 2^-18 ulp of that point (where the second rounding could matter),
-// at a power of two and outside 1e-30..1e30 is the FP64 root itself taken. 300 cycles against 760: an
-// FP64 operation has a latency of 63 cycles here, and a square root chains ten.
-__device__ __forceinline__ float sqrt_to_float(double x) {
-  const float a = (float)x;
-  const float c = sqrtf(a);
-  const double cd = widen(c);
-  const float off = (float)fma(-cd, cd, x) * __fdividef(0.5f, c);  // sqrt(x) - c
-  const uint32_t cb = __float_as_uint(c);
-  const float up = __uint_as_float(cb + 1u) - c, h = 0.5f * up, ao = fabsf(off);
-  if (a > 1e-30f && a < 1e30f && (cb & 0x7fffffu) > 1u && (cb & 0x7fffffu) < 0x7ffffeu) {
-    if (ao < h * 0.999996f) return c;
-    if (ao > h * 1.000004f && ao < 1.4f * up) return __uint_as_float(off > 0.f ? cb + 1u : cb - 1u);
-  }
-  return (float)sqrt(x);
 }
 
 // What a contact reads of its partner q; loaded before anything is known of it, so that one latency
