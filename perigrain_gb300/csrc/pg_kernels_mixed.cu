@@ -882,13 +882,16 @@ __global__ void __launch_bounds__(128, BPS) k_force_mx(const Dev P) {
         const float dist = (float)(xc[dir] - in.wall[side]);
         if (!(fabsf(dist) <= R)) continue;
         wbits |= 1u << (4 * k);
-        const float dd = fabsf(dist);
+        // products and sums written out where the compiler may fuse either product or none: it chose
+        // differently for the variant of seven blocks an SM, whose wall forces were an ulp off the others'
+        const float dd = fabsf(dist), R2 = __fmul_rn(R, R), h2 = fmaf(-dd, dd, R2);
         float Area, I;
         if constexpr (D == 2) {
-          Area = 0.5f * (float)M_PI * R * R - R * R * asinf(dd / R) - sqrtf(fmaxf(R * R - dd * dd, 0.f)) * dd;
+          const float half = __fmul_rn(__fmul_rn(0.5f * (float)M_PI, R), R);
+          Area = fmaf(-sqrtf(fmaxf(h2, 0.f)), dd, fmaf(-R2, asinf(dd / R), half));
           I = 0.f;
         } else {
-          const float a = R - dd, b = R * R - dd * dd;
+          const float a = R - dd, b = h2;
           Area = ((float)M_PI / 3.f) * a * a * (2.f * R - dd);
           I = ((float)M_PI / 4.f) * b * b;
         }
@@ -919,13 +922,13 @@ __global__ void __launch_bounds__(128, BPS) k_force_mx(const Dev P) {
                 ff = -rv[tg] * rho / dtf;
                 wbits |= 4u << (4 * k);
               }
-              f[tg] += ff;
+              f[tg] = __fadd_rn(f[tg], ff);
               rec.a_t1 = vol_i * (double)ff;
               rec.has_fric = 1;
             }
           } else {
             const int t1 = (dir + 1) % 3, t2 = (dir + 2) % 3;
-            const float vn = sqrtf(rv[t1] * rv[t1] + rv[t2] * rv[t2]);
+            const float vn = sqrtf(fmaf(rv[t1], rv[t1], __fmul_rn(rv[t2], rv[t2])));
             if (vn > 0.f) {
               const float u1 = rv[t1] / vn, u2 = rv[t2] / vn;
               float sfr = -mu * fabsf(F);
@@ -934,8 +937,8 @@ __global__ void __launch_bounds__(128, BPS) k_force_mx(const Dev P) {
                 sfr = -vn / rho / dtf;
                 wbits |= 4u << (4 * k);
               }
-              f[t1] += sfr * u1;
-              f[t2] += sfr * u2;
+              f[t1] = __fadd_rn(f[t1], __fmul_rn(sfr, u1));
+              f[t2] = __fadd_rn(f[t2], __fmul_rn(sfr, u2));
               rec.a_t1 = vol_i * (double)(sfr * u1);
               rec.a_t2 = vol_i * (double)(sfr * u2);
               rec.has_fric = 1;
@@ -944,7 +947,7 @@ __global__ void __launch_bounds__(128, BPS) k_force_mx(const Dev P) {
         }
         if (P.allow_damping) {
           const float df = -(2.f * zeta * sqrtf(Kn * rho) * sqrtf(fabsf(Area))) * rv[dir];
-          f[dir] += df;
+          f[dir] = __fadd_rn(f[dir], df);
           rec.a_damp = vol_i * (double)df;
           rec.has_damp = 1;
         }
@@ -1014,8 +1017,8 @@ __global__ void __launch_bounds__(128, BPS) k_force_mx(const Dev P) {
       }
       const float orho = gr.one_over_rho_f, hdt = P.half_dt_f;
       for (int c = 0; c < D; ++c) {
-        a[c] = orho * f[c];
-        v[c] = vpd[c] + widen((ao[c] + a[c]) * hdt);  // FP64 accumulation of an FP32 increment
+        a[c] = __fmul_rn(orho, f[c]);
+        v[c] = vpd[c] + widen(__fmul_rn(__fadd_rn(ao[c], a[c]), hdt));  // FP64 accumulation of an FP32 increment
       }
       if ((D == 2) ? clamped_in : (P.clamped[d] != 0)) {
         for (int c = 0; c < D; ++c) {
