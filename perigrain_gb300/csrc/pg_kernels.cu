@@ -703,7 +703,7 @@ static void body_t(const Dev& P, const LaunchCfg& L, cudaStream_t s, uint64_t* l
   }
   if (e0) cudaEventRecord(e0, s);
   if (P.n_edges) {
-    launch_k(k_bonds<D>, cdiv(P.n_edges, 256), 256, 0, s, pdl, P);
+    launch_k(k_bonds<D>, (P.n_edges - 1u) / 256u + 1u, 256, 0, s, pdl, P);  // up to 2^32 - 1 entries
     *launches += 1;
   }
   const dim3 grid(cdiv(P.n_chunks * 32, L.force_block)), block(L.force_block);
