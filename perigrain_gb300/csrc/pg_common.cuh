@@ -794,8 +794,8 @@ __device__ __forceinline__ bool grid_barrier(const Dev& P, uint32_t* ok_smem) {
           ok = 0;
           set_status(P.status, PG_ETIMEOUT);
           // the arrival count now holds this launch's stale arrivals: later launches of this
-          // kernel must not use the barrier (an early release would let the scan read counts
-          // before every key is in and the scatter write outside the sorted list)
+          // kernel must not use the barrier (an early release would let nodes be chained into cells
+          // that others still empty)
           atomicExch(P.gbar + 2, 1u);
           break;
         }

@@ -146,7 +146,7 @@ PG_HD double hw_sqrt(double x) {
 // Division, square root and multiplication come twice: X_rn is the drop-in, which takes the hardware
 // operation outside the integer range; X_bits has no such branch and clears *ok there instead, so a
 // chain of them runs straight through and is redone once in hardware when any flag fell. (The +-1
-// corrections stay branches: as selects they took k_pack_maximin from 23.6 to 29.9 ms.)
+// corrections stay branches: as selects they took the packing ascent from 23.6 to 29.9 ms.)
 
 // A divisor prepared once for several quotients.
 struct Divisor {

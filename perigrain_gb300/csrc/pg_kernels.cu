@@ -1,15 +1,21 @@
 // GB300 (sm_103a) kernels of the PeriDEM time step, FP64 parity path.
 //
 // One step (reference src/particle/timeloop.h:608-879) is these launches on one stream:
-//   k_predict      position update (timeloop.h:661-669) + grid key + per-grain bounding box
-//   k_scan_reduce  \ exclusive scan of the per-bucket counts = cell-start table
+//   k_predict      position update (timeloop.h:661-669) + grid key or list-rebuild check + per-grain
+//                  bounding box
+//   k_grid_coop    candidate lists: grid refit, cell chains and lists on rebuild steps, or
+//   k_scan_reduce  \ the grid search: exclusive scan of the per-bucket counts = cell-start table
 //   k_scan_final   /
 //   k_scatter      nodes -> bucket order (counting sort, one digit spanning all buckets)
 //   k_bonds        bond force addends + break (particle2.h:102-232), one bond per thread
-//   k_force        sum of the bond forces, self/inter-grain contact (contact.h:668-812), wall (contact.h:900-964, :314-431, :16-41),
-//                  external force and torque (timeloop.h:774-824), velocity update
-//                  (timeloop.h:834-863) -- fused, one node per thread
+//   k_force        sum of the bond forces, self/inter-grain contact (contact.h:668-812), wall
+//                  (contact.h:900-964, :314-431, :16-41), external force and torque
+//                  (timeloop.h:774-824), velocity update (timeloop.h:834-863) -- fused, one node per
+//                  thread
 //   k_finalize     ordered wall-reaction sums, pair log, wall move (timeloop.h:866-878)
+// With lists the steps of one call run fused: k_force also makes the next step's position update and
+// k_grid_coop first ends the step before, so k_predict runs once ahead of the call's first step and
+// k_finalize once behind its last.
 //
 // This file is compiled with --fmad=false: every FP64 operation is the IEEE operation the
 // reference performs, in the reference's order, so the non-wall path is bit-exact.
@@ -133,8 +139,8 @@ __device__ __forceinline__ void ld_addend(const Dev& P, uint32_t s, double (&g)[
 //
 // Bound by the FP64 pipe (one warp instruction per 16 cycles and SM) beside the integer ALU: 15
 // FP64 instructions per bond in 2D, 21 in 3D, against twice 14 and twice 20 when each node
-// computed its own bonds. Collision ensemble (10.0M directed bonds): k_bonds 158 us + k_force 61 us
-// against 364 us fused; 3D spheres (10.8M): 245 + 116 against 804 us; two disks (65k): 4.8 + 8.0
+// computed its own bonds. Collision ensemble (10.0M directed bonds): k_bonds 158 us + k_force 73 us
+// (which also updates the next positions) against 364 us fused; 3D spheres (10.8M): 245 + 116 against 804 us; two disks (65k): 4.8 + 8.0
 // against 56 us, the work spread over 1,019 warps instead of 79. More of it on the integer pipe
 // (the extension en - xin, the scale and force products, the sum of the squares) was slower: the
 // ensemble step 250 us as it stands, 263 with the extension moved, 323 with all of them moved.
@@ -674,7 +680,8 @@ __global__ void __launch_bounds__(128, BPS) k_force(const Dev P) {
 // host-side launchers
 // ---------------------------------------------------------------------------------------------
 // The force kernel's variants: mask recording (REC), per-grain contact parameters (GC), candidate
-// lists or the grid search (LIST); the plain kernel with lists for 5 or 7 blocks of 128 threads per
+// lists or the grid search (LIST); the plain kernel with lists for 5 or 7 blocks (force_bps(): 6 takes
+// 7) of 128 threads per
 // SM (96 or 72 registers): the latency of its own chain counts where the chunks do not fill the GPU
 // (two disks: 20.5 us a step at 5 blocks, 21.1 at 7), occupancy where they do (3D spheres 366 and 359).
 template <int D>

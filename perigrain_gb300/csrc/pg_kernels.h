@@ -43,11 +43,13 @@ inline cudaError_t max_local_bytes(const void* const* fs, int n, std::atomic<siz
 }
 
 // Blocks of 128 threads per SM the force kernels are compiled for that suit a handle of n_chunks
-// warps: a warp holds its slot for its whole chunk, so the time goes as the number of rounds of
+// warps: a warp holds its slot for its whole chunk, so the time grows with the number of rounds of
 // resident warps times the warps that share an SM in each, rounds * bps; the smallest product wins,
-// the larger register budget on a tie. Mixed, us a step at 5 / 6 / 7 blocks: collision ensemble (80
-// warps an SM) 70 / 71 / 62, 3D spheres (26) 87 / 110 / 86, settling (24) 20.7 / 17.9 / 19.0, two
-// disks (1) 12.5 / 13.9 / 14.0.
+// the larger register budget on a tie. The product picks the fastest of those measured but is no model
+// of the times: an SM is not 1.4 times as fast with 7 blocks as with 5, and a last round is seldom full.
+// Mixed, us a step at 5 / 6 / 7 blocks (product): collision ensemble (80 warps an SM) 70 / 71 / 62
+// (25 / 24 / 21), 3D spheres (26) 87 / 110 / 86 (10 / 12 / 7), settling (24) 20.7 / 17.9 / 19.0
+// (10 / 6 / 7), two disks (1) 12.5 / 13.9 / 14.0 (5 / 6 / 7).
 inline int force_bps(uint32_t n_chunks, uint32_t sms) {
   int best = 5;
   uint64_t best_cost = ~0ull;
