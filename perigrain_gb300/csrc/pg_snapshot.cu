@@ -178,7 +178,9 @@ int pg_snapshot(pg_handle* h, const pg_snapshot_desc* d) {
   }
   if (want_alive && !s.bond_offset) {
     CU(cudaMalloc((void**)&s.bond_offset, (size_t)(N + 1) * 8));
-    CU(write_device(h, s.bond_offset, h->bond_offset.data(), (size_t)(N + 1) * 8));
+    // on the default stream and waited for there: the steps issued on the handle's stream run on
+    CU(cudaMemcpy(s.bond_offset, h->bond_offset.data(), (size_t)(N + 1) * 8, cudaMemcpyHostToDevice));
+    CU(cudaStreamSynchronize(0));
   }
 
   SnapArgs a{};
