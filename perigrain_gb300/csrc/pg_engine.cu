@@ -358,9 +358,10 @@ static int edges_setup(pg_handle* h) {
   CU(cudaGetLastError());
   CU(scan_u32_dev(count, NC, first, tile, done, 0));
   CU(cudaMemcpy(&P.n_edges, first + NC, 4, cudaMemcpyDeviceToHost));
-  CU(h->dalloc(&P.edge_xin, (size_t)P.n_edges * 3));
-  P.edge_ij = (uint2*)(P.edge_xin + P.n_edges);
-  P.edge_slot = P.edge_ij + P.n_edges;
+  const size_t E = ((size_t)P.n_edges + 31) / 32 * 32;  // each array on a 256-byte boundary
+  CU(h->dalloc(&P.edge_xin, E * 3));
+  P.edge_ij = (uint2*)(P.edge_xin + E);
+  P.edge_slot = P.edge_ij + E;
   k_edge_fill<<<NC, 32 * EDGE_WARPS>>>(P, pair, first, P.edge_ij, P.edge_slot, P.edge_xin);
   CU(cudaGetLastError());
   CU(cudaMemset(P.addend, 0, words * 4));
