@@ -116,6 +116,15 @@ __device__ __forceinline__ float dotf(const float (&a)[D], const float (&b)[D]) 
   return s;
 }
 
+// |v|^2 in FP64, fused, with the products' order written out so that every variant of the force kernel
+// takes the same contact decisions to the last bit.
+template <int D>
+__device__ __forceinline__ double sum_sq64(const double (&v)[D]) {
+  double s = fma(v[0], v[0], __dmul_rn(v[1], v[1]));
+  if constexpr (D == 3) s = fma(v[2], v[2], s);
+  return s;
+}
+
 // CurrPos of node d from its displacement, its FP32 images, and either the list-rebuild check or the
 // node's grid key.
 template <int D>
@@ -290,13 +299,12 @@ template <int D, bool GC>
 __device__ __forceinline__ bool contact_term(const Dev& P, const Side<D>& s, uint32_t gqi, uint32_t d, uint32_t q,
                                              const Partner<D>& pq, ContactTerm<D>& o) {
   const bool same = gqi == s.g;
-  // The contact decision |x_q - x_p| <= R_c' is made with the reference's FP64 arithmetic:
+  // The contact decision |x_q - x_p| <= R_c' is made in FP64 (the squares summed with fused products):
   // contact damping switches on at full strength at that boundary, so a decision flipped by
   // FP32 rounding would kick a node by metres per second.
   double dir64[D];
   for (int c = 0; c < D; ++c) dir64[c] = pq.x[c] - s.x[c];
-  double n2 = dir64[0] * dir64[0];
-  for (int c = 1; c < D; ++c) n2 = n2 + dir64[c] * dir64[c];
+  const double n2 = sum_sq64<D>(dir64);
   // |x_q - x_p| <= contact_rad as n2 <= contact_s_max, the same outcome without the square root
   if (!(n2 <= s.s_max)) return false;
   float Kn = s.Kn, zeta = s.zeta, mu = s.mu;
@@ -312,8 +320,7 @@ __device__ __forceinline__ bool contact_term(const Dev& P, const Side<D>& s, uin
     ldv<D>(P.pos, d, pp);
     ldv<D>(P.pos, q, ps);
     for (int c = 0; c < D; ++c) r[c] = pp[c] - ps[c];
-    double r2 = r[0] * r[0];
-    for (int c = 1; c < D; ++c) r2 = r2 + r[c] * r[c];
+    const double r2 = sum_sq64<D>(r);
     // |x_q - x_p| <= R_c' = min(ref, contact_rad), ref = sqrt(r2): the roots compare as n2 and r2 do
     // unless these are within a few units in the last place (1 + 2^-50: roots two such units apart)
     if (n2 > r2 * 1.0000000000000009) return false;
